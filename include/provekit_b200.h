@@ -787,9 +787,10 @@ int pkg_prover_load_bytes(const uint8_t *ptr, size_t len, pkg_prover **out);
 /* out[i] = op(a[i], b[i]) over n Fr (4 x u64 LE each, device, 16-byte
  * aligned), asynchronous on stream; results fully reduced (< p).
  *   PKG_FR_MUL_F64 / PKG_FR_SQR_F64: a*b*2^-256, a^2*2^-256 mod p on the FP64
- *     pipe (the routines of the NTT and Skyscraper kernels); inputs < 2p.
+ *     pipe; inputs < 2p.
  *   PKG_FR_FROM_MONT_F64: a*2^-256 mod p on the FP64 pipe; any 256-bit a.
- *   PKG_FR_MUL_INT / PKG_FR_SQR_INT: the same on the integer pipe; inputs < p.
+ *   PKG_FR_MUL_INT / PKG_FR_SQR_INT: the same on the integer pipe (the
+ *     routines of the library's kernels); inputs < 2p.
  *   PKG_FR_FROM_MONT_INT: the same on the integer pipe (REDC alone); any 256-bit a.
  * b is read only by the two products (may be NULL otherwise).  The reference's
  * scalar_mul/scalar_sqr return values in [0, 2^256 - 2p) with the same
@@ -853,8 +854,7 @@ int pkg_measure_imad_rate(double *instr_per_second);
 
 /* Sustained double-precision fma rate of this GPU (fma instructions per
  * second, one thread-instruction each), from eight independent chains per
- * thread on every SM.  Denominator of the FP64-pipe roofline: the Fr
- * products of the NTT butterflies and Skyscraper rounds run on that pipe.
+ * thread on every SM.
  * Synchronous.  No counterpart in the reference (a measurement helper). */
 int pkg_measure_dfma_rate(double *instr_per_second);
 

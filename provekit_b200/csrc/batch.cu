@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(512) batch_ntt_pass_kernel(const PassDesc* __r
       Fr tw = fr_load_ro(roots, (high << s) | (uint64_t)grp);
       int i0 = j0 * T + ll, i1 = j1 * T + ll;
       Fr x0 = sm_get(sm, E, i0), x1 = sm_get(sm, E, i1);
-      Fr m = fr_mul_f64(tw, x1);
+      Fr m = fr_mul(tw, x1);
       sm_put(sm, E, i0, fr_add(x0, m));
       sm_put(sm, E, i1, fr_sub(x0, m));
     }
@@ -233,7 +233,7 @@ __global__ void batch_sc_start_kernel(ScState* __restrict__ st, const JobDev* __
   s.sum_g = fr_add(dev_cubic(g0, fr_zero()), dev_cubic(g0, fr_one_mont()));
   t.absorb(s.sum_g);   // :541
   s.rho = t.squeeze();  // :543
-  s.saved = fr_mul_f64(s.rho, s.sum_g);
+  s.saved = fr_mul(s.rho, s.sum_g);
   s.tl = t.l;
   s.tr = t.r;
 }
@@ -256,7 +256,7 @@ __global__ void batch_eq_half_kernel(const RangeDesc* __restrict__ rd,
     Fr acc = fr_one_mont();
     for (int i = 0; i < nr; i++) {
       const Fr ri = st[d.job].r[r0 + i];
-      acc = fr_mul_f64(acc, ((x >> (nr - 1 - i)) & 1) ? ri : fr_sub(fr_one_mont(), ri));
+      acc = fr_mul(acc, ((x >> (nr - 1 - i)) & 1) ? ri : fr_sub(fr_one_mont(), ri));
     }
     fr_store(is_hi ? jb.eq_hi : jb.eq_lo, x, acc);
   }
@@ -270,7 +270,7 @@ __global__ void batch_eq_combine_kernel(const RangeDesc* __restrict__ rd,
     const RangeDesc d = rd[find_desc(begins, nd, o)];
     const JobDev& jb = jobs[d.job];
     const uint64_t x = o - d.begin;
-    fr_store(jb.eq, x, fr_mul_f64(fr_load_ro(jb.eq_hi, x >> jb.nlo),
+    fr_store(jb.eq, x, fr_mul(fr_load_ro(jb.eq_hi, x >> jb.nlo),
                               fr_load_ro(jb.eq_lo, x & ((uint64_t(1) << jb.nlo) - 1))));
   }
 }
@@ -340,11 +340,11 @@ __global__ void batch_sc_finish_round_kernel(ScState* __restrict__ st,
   Fr gp[4];
   dev_blinding_coeffs(&s.g[0][0], (int)s.m0, (int)round, s.alpha, gp);
   Fr cf[4];
-  cf[0] = fr_add(h[0], fr_mul_f64(s.rho, gp[0]));
+  cf[0] = fr_add(h[0], fr_mul(s.rho, gp[0]));
   Fr gem1 = fr_sub(fr_add(fr_sub(gp[0], gp[1]), gp[2]), gp[3]);
-  Fr cem1 = fr_add(h[1], fr_mul_f64(s.rho, gem1));
-  cf[2] = fr_mul_f64(fr_half_mont(), fr_sub(fr_sub(fr_sub(fr_add(s.saved, cem1), cf[0]), cf[0]), cf[0]));
-  cf[3] = fr_add(h[2], fr_mul_f64(s.rho, gp[3]));
+  Fr cem1 = fr_add(h[1], fr_mul(s.rho, gem1));
+  cf[2] = fr_mul(fr_half_mont(), fr_sub(fr_sub(fr_sub(fr_add(s.saved, cem1), cf[0]), cf[0]), cf[0]));
+  cf[3] = fr_add(h[2], fr_mul(s.rho, gp[3]));
   cf[1] = fr_sub(fr_sub(fr_sub(fr_sub(s.saved, cf[0]), cf[0]), cf[3]), cf[2]);
   DevTranscript t;
   t.l = s.tl;
@@ -369,8 +369,8 @@ __global__ void batch_sc_end_kernel(ScState* __restrict__ st, uint32_t njobs) {
   for (uint32_t i = 0; i < s.m0; i++) {
     Fr pw = fr_one_mont();
     for (int k = 0; k < 4; k++) {
-      acc = fr_add(acc, fr_mul_f64(pw, s.wb[i][k]));
-      pw = fr_mul_f64(pw, s.alpha[i]);
+      acc = fr_add(acc, fr_mul(pw, s.wb[i][k]));
+      pw = fr_mul(pw, s.alpha[i]);
     }
   }
   s.blinding_eval = acc;

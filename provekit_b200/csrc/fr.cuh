@@ -2,9 +2,8 @@
 //
 // An element is 8 x 32-bit little-endian limbs in registers; in memory it is
 // the arkworks layout (4 x u64 LE == 8 x u32 LE), 32 bytes, 32-byte aligned.
-// Multiplication is word-level CIOS Montgomery (Koc, Acar, Kaliski 1996) with
-// R = 2^256, written as explicit PTX carry chains (mad.lo.cc / madc.hi.cc) so
-// that every partial product is one IMAD-class instruction.  This replaces
+// Products are Montgomery products with R = 2^256 on the integer pipe, as
+// explicit PTX carry chains of 32x32 -> 64-bit multiply-adds.  This replaces
 // ark-ff's Fr multiply and bn254_multiplier::scalar_{mul,sqr}
 // (skyscraper/bn254-multiplier/src/scalar.rs:12-132); outputs are fully
 // reduced, as ark-ff stores them.
@@ -147,148 +146,329 @@ __device__ __forceinline__ Fr fr_sub(const Fr& a, const Fr& b) {
   return r;
 }
 
-// t[0..8] += a * b  (two carry chains: low halves into t0..t7 with the
-// carry into t8, high halves into t1..t8).  Requires the sum < 2^288.
-#define PK_ROW(T, A, B)                                                                          \
-  asm("mad.lo.cc.u32  %0, %9,  %17, %0;\n\t"                                                    \
-      "madc.lo.cc.u32 %1, %10, %17, %1;\n\t"                                                    \
-      "madc.lo.cc.u32 %2, %11, %17, %2;\n\t"                                                    \
-      "madc.lo.cc.u32 %3, %12, %17, %3;\n\t"                                                    \
-      "madc.lo.cc.u32 %4, %13, %17, %4;\n\t"                                                    \
-      "madc.lo.cc.u32 %5, %14, %17, %5;\n\t"                                                    \
-      "madc.lo.cc.u32 %6, %15, %17, %6;\n\t"                                                    \
-      "madc.lo.cc.u32 %7, %16, %17, %7;\n\t"                                                    \
-      "addc.u32       %8, %8, 0;"                                                                \
-      : "+r"(T[0]), "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]),      \
-        "+r"(T[7]), "+r"(T[8])                                                                   \
-      : "r"(A[0]), "r"(A[1]), "r"(A[2]), "r"(A[3]), "r"(A[4]), "r"(A[5]), "r"(A[6]), "r"(A[7]),  \
-        "r"(B));                                                                                 \
-  asm("mad.hi.cc.u32  %0, %8,  %16, %0;\n\t"                                                    \
-      "madc.hi.cc.u32 %1, %9,  %16, %1;\n\t"                                                    \
-      "madc.hi.cc.u32 %2, %10, %16, %2;\n\t"                                                    \
-      "madc.hi.cc.u32 %3, %11, %16, %3;\n\t"                                                    \
-      "madc.hi.cc.u32 %4, %12, %16, %4;\n\t"                                                    \
-      "madc.hi.cc.u32 %5, %13, %16, %5;\n\t"                                                    \
-      "madc.hi.cc.u32 %6, %14, %16, %6;\n\t"                                                    \
-      "madc.hi.u32    %7, %15, %16, %7;"                                                         \
-      : "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]), "+r"(T[7]),      \
-        "+r"(T[8])                                                                               \
-      : "r"(A[0]), "r"(A[1]), "r"(A[2]), "r"(A[3]), "r"(A[4]), "r"(A[5]), "r"(A[6]), "r"(A[7]),  \
-        "r"(B))
+// Products are rows of 32x32 -> 64-bit multiply-adds.  A row's partial
+// products y_j * b start at consecutive words, so they overlap; the even-index
+// ones (words 0-1, 2-3, ..) and the odd-index ones (words 1-2, 3-4, ..) each
+// tile their own 8-word accumulator without overlap.  Keeping two
+// accumulators -- E at words 0..7, O at words 1..8 of the current row -- makes
+// every row one carry chain per accumulator of lo/hi pairs, which compile to
+// one 64-bit multiply-add each instead of a low and a high one (B200 issues
+// 28 of either kind of 64-bit-wide multiply per SM and cycle, so the pairing
+// halves the work).  After a Montgomery row E[0] is 0: the frame moves up one
+// word, O becomes the even accumulator, E[2..7] the odd one, and E[1] is
+// carried into the next row's first sum.
 
-// t[0..8] += m * p, as PK_ROW with the modulus as immediates.
-#define PK_ROW_P(T, M)                                                                           \
-  asm("mad.lo.cc.u32  %0, %9,  %10, %0;\n\t"                                                    \
-      "madc.lo.cc.u32 %1, %9,  %11, %1;\n\t"                                                    \
-      "madc.lo.cc.u32 %2, %9,  %12, %2;\n\t"                                                    \
-      "madc.lo.cc.u32 %3, %9,  %13, %3;\n\t"                                                    \
-      "madc.lo.cc.u32 %4, %9,  %14, %4;\n\t"                                                    \
-      "madc.lo.cc.u32 %5, %9,  %15, %5;\n\t"                                                    \
-      "madc.lo.cc.u32 %6, %9,  %16, %6;\n\t"                                                    \
-      "madc.lo.cc.u32 %7, %9,  %17, %7;\n\t"                                                    \
-      "addc.u32       %8, %8, 0;"                                                                \
-      : "+r"(T[0]), "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]),      \
-        "+r"(T[7]), "+r"(T[8])                                                                   \
-      : "r"(M), "n"(PK_P0), "n"(PK_P1), "n"(PK_P2), "n"(PK_P3), "n"(PK_P4), "n"(PK_P5),          \
-        "n"(PK_P6), "n"(PK_P7));                                                                 \
-  asm("mad.hi.cc.u32  %0, %8,  %9,  %0;\n\t"                                                    \
-      "madc.hi.cc.u32 %1, %8,  %10, %1;\n\t"                                                    \
-      "madc.hi.cc.u32 %2, %8,  %11, %2;\n\t"                                                    \
-      "madc.hi.cc.u32 %3, %8,  %12, %3;\n\t"                                                    \
-      "madc.hi.cc.u32 %4, %8,  %13, %4;\n\t"                                                    \
-      "madc.hi.cc.u32 %5, %8,  %14, %5;\n\t"                                                    \
-      "madc.hi.cc.u32 %6, %8,  %15, %6;\n\t"                                                    \
-      "madc.hi.u32    %7, %8,  %16, %7;"                                                         \
-      : "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]), "+r"(T[7]),      \
-        "+r"(T[8])                                                                               \
-      : "r"(M), "n"(PK_P0), "n"(PK_P1), "n"(PK_P2), "n"(PK_P3), "n"(PK_P4), "n"(PK_P5),          \
-        "n"(PK_P6), "n"(PK_P7))
+// O[0..7] = (O[0..5] + y * b), with e0 += c first and its carry entering the chain.
+__device__ __forceinline__ void fr_odd_row(uint32_t& e0, uint32_t c, uint32_t* O, uint32_t y1,
+                                           uint32_t y3, uint32_t y5, uint32_t y7, uint32_t b) {
+  asm("add.cc.u32     %0, %0,  %9;\n\t"
+      "madc.lo.cc.u32 %1, %10, %14, %1;\n\t"
+      "madc.hi.cc.u32 %2, %10, %14, %2;\n\t"
+      "madc.lo.cc.u32 %3, %11, %14, %3;\n\t"
+      "madc.hi.cc.u32 %4, %11, %14, %4;\n\t"
+      "madc.lo.cc.u32 %5, %12, %14, %5;\n\t"
+      "madc.hi.cc.u32 %6, %12, %14, %6;\n\t"
+      "madc.lo.cc.u32 %7, %13, %14, 0;\n\t"
+      "madc.hi.u32    %8, %13, %14, 0;"
+      : "+r"(e0), "+r"(O[0]), "+r"(O[1]), "+r"(O[2]), "+r"(O[3]), "+r"(O[4]), "+r"(O[5]),
+        "=r"(O[6]), "=r"(O[7])
+      : "r"(c), "r"(y1), "r"(y3), "r"(y5), "r"(y7), "r"(b));
+}
 
-// Montgomery product a * b * 2^-256 mod p.  Inputs a, b < 2p; the CIOS
-// accumulator then stays below 3p at every word boundary and below 2^288
-// inside a word step, so 9 limbs suffice.  Output fully reduced (< p) when
-// a, b < p (one conditional subtraction; t < 2p), and < p after two
-// conditional subtractions for a, b < 2p (t < 3p).
-template <bool kTwoSub = false>
-__device__ __forceinline__ Fr fr_mul(const Fr& a, const Fr& b) {
-  uint32_t t[9];
+// E[0..7] += y * b, the carry into o7 (word 8).
+__device__ __forceinline__ void fr_even_row(uint32_t* E, uint32_t& o7, uint32_t y0, uint32_t y2,
+                                            uint32_t y4, uint32_t y6, uint32_t b) {
+  asm("mad.lo.cc.u32  %0, %9,  %13, %0;\n\t"
+      "madc.hi.cc.u32 %1, %9,  %13, %1;\n\t"
+      "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+      "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+      "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+      "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+      "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+      "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+      "addc.u32       %8, %8, 0;"
+      : "+r"(E[0]), "+r"(E[1]), "+r"(E[2]), "+r"(E[3]), "+r"(E[4]), "+r"(E[5]), "+r"(E[6]),
+        "+r"(E[7]), "+r"(o7)
+      : "r"(y0), "r"(y2), "r"(y4), "r"(y6), "r"(b));
+}
+
+// O[0..7] += y * b (the sum fits: the row's total is below 2^288).
+__device__ __forceinline__ void fr_odd_acc(uint32_t* O, uint32_t y1, uint32_t y3, uint32_t y5,
+                                           uint32_t y7, uint32_t b) {
+  asm("mad.lo.cc.u32  %0, %8,  %12, %0;\n\t"
+      "madc.hi.cc.u32 %1, %8,  %12, %1;\n\t"
+      "madc.lo.cc.u32 %2, %9,  %12, %2;\n\t"
+      "madc.hi.cc.u32 %3, %9,  %12, %3;\n\t"
+      "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+      "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+      "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+      "madc.hi.u32    %7, %11, %12, %7;"
+      : "+r"(O[0]), "+r"(O[1]), "+r"(O[2]), "+r"(O[3]), "+r"(O[4]), "+r"(O[5]), "+r"(O[6]),
+        "+r"(O[7])
+      : "r"(y1), "r"(y3), "r"(y5), "r"(y7), "r"(b));
+}
+
+// E, O = y * b (first row, nothing to accumulate).
+__device__ __forceinline__ void fr_first_row(uint32_t* E, uint32_t* O, const uint32_t* y,
+                                             uint32_t b) {
 #pragma unroll
-  for (int i = 0; i < 9; i++) t[i] = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    PK_ROW(t, a.v, b.v[i]);
-    uint32_t m = t[0] * PK_MU;
-    PK_ROW_P(t, m);
-    // t[0] is now 0: shift one word down.
-#pragma unroll
-    for (int j = 0; j < 8; j++) t[j] = t[j + 1];
-    t[8] = 0;
+  for (int i = 0; i < 4; i++) {
+    const uint64_t e = (uint64_t)y[2 * i] * b, o = (uint64_t)y[2 * i + 1] * b;
+    E[2 * i] = (uint32_t)e;
+    E[2 * i + 1] = (uint32_t)(e >> 32);
+    O[2 * i] = (uint32_t)o;
+    O[2 * i + 1] = (uint32_t)(o >> 32);
   }
-  Fr r;
+}
+
+// The frame one word up; returns the word carried into the next row (E[1]).
+__device__ __forceinline__ uint32_t fr_next_frame(uint32_t* E, uint32_t* O) {
+  const uint32_t c = E[1];
+  uint32_t t[6];
 #pragma unroll
-  for (int i = 0; i < 8; i++) r.v[i] = t[i];
-  r = fr_reduce_once(r);
-  if (kTwoSub) r = fr_reduce_once(r);
+  for (int i = 0; i < 6; i++) t[i] = E[i + 2];
+#pragma unroll
+  for (int i = 0; i < 8; i++) E[i] = O[i];
+#pragma unroll
+  for (int i = 0; i < 6; i++) O[i] = t[i];
+  return c;
+}
+
+// E at words 0..7 plus c at word 0 plus O[0..5] at words 1..6.
+__device__ __forceinline__ Fr fr_join(const uint32_t* E, const uint32_t* O, uint32_t c) {
+  Fr r;
+  asm("add.cc.u32  %0, %8,  %16;\n\t"
+      "addc.cc.u32 %1, %9,  %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, 0;"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+        "=r"(r.v[6]), "=r"(r.v[7])
+      : "r"(E[0]), "r"(E[1]), "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]),
+        "r"(c), "r"(O[0]), "r"(O[1]), "r"(O[2]), "r"(O[3]), "r"(O[4]), "r"(O[5]));
   return r;
 }
 
-// Montgomery square a^2 * 2^-256 mod p for a < p, as separated operand
-// scanning (SOS): the 28 cross products a_i a_j (i < j) once, doubled, plus
-// the 8 diagonal squares -- 36 word products instead of 64 -- then the
-// word-by-word Montgomery reduction.  Accumulation uses 64-bit
-// multiply-adds; the result is fully reduced.
+// a + b as 256-bit integers (the sum fits).
+__device__ __forceinline__ Fr fr_add_raw(const Fr& a, const uint32_t* b) {
+  Fr s;
+  asm("add.cc.u32  %0, %8,  %16;\n\t"
+      "addc.cc.u32 %1, %9,  %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(s.v[0]), "=r"(s.v[1]), "=r"(s.v[2]), "=r"(s.v[3]), "=r"(s.v[4]), "=r"(s.v[5]),
+        "=r"(s.v[6]), "=r"(s.v[7])
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]),
+        "r"(a.v[6]), "r"(a.v[7]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]),
+        "r"(b[5]), "r"(b[6]), "r"(b[7]));
+  return s;
+}
+
+// One Montgomery row on the frame: adds m p with m = -E[0] / p mod 2^32.
+__device__ __forceinline__ void fr_redc_row(uint32_t* E, uint32_t* O) {
+  const uint32_t m = E[0] * PK_MU;
+  fr_odd_acc(O, PK_P1, PK_P3, PK_P5, PK_P7, m);
+  fr_even_row(E, O[7], PK_P0, PK_P2, PK_P4, PK_P6, m);
+}
+
+// Montgomery product a * b * 2^-256 mod p for a, b < 2p: CIOS rows (Koc,
+// Acar, Kaliski 1996) over the two accumulators, 128 64-bit multiply-adds and
+// 8 low ones.  (a b + M p) / 2^256 < 4 p^2 / 2^256 + p < 1.8 p, so one
+// conditional subtraction reduces fully.  Measured on B200: 65.8 G products/s
+// (528 multiply cycles per warp of 565), against 44.8 G/s of the binary64
+// form (352 instructions) and 42.0 G/s of rows with separate low and high
+// chains.
+__device__ __forceinline__ Fr fr_mul(const Fr& a, const Fr& b) {
+  uint32_t E[8], O[8], c = 0;
+  fr_first_row(E, O, a.v, b.v[0]);
+  fr_redc_row(E, O);
+#pragma unroll
+  for (int i = 1; i < 8; i++) {
+    c = fr_next_frame(E, O);
+    fr_odd_row(E[0], c, O, a.v[1], a.v[3], a.v[5], a.v[7], b.v[i]);
+    fr_even_row(E, O[7], a.v[0], a.v[2], a.v[4], a.v[6], b.v[i]);
+    fr_redc_row(E, O);
+  }
+  c = fr_next_frame(E, O);
+  return fr_reduce_once(fr_join(E, O, c));
+}
+
+// (t + M p) / 2^256 for a 256-bit t: the Montgomery reduction alone, result
+// <= p (64 64-bit multiply-adds).
+__device__ __forceinline__ Fr fr_redc(const uint32_t* t) {
+  uint32_t E[8], O[8], c = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) E[i] = t[i];
+  {
+    const uint32_t P[8] = {PK_P0, PK_P1, PK_P2, PK_P3, PK_P4, PK_P5, PK_P6, PK_P7};
+    const uint32_t m = E[0] * PK_MU;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint64_t o = (uint64_t)P[2 * i + 1] * m;
+      O[2 * i] = (uint32_t)o;
+      O[2 * i + 1] = (uint32_t)(o >> 32);
+    }
+    fr_even_row(E, O[7], PK_P0, PK_P2, PK_P4, PK_P6, m);
+  }
+#pragma unroll
+  for (int i = 1; i < 8; i++) {
+    c = fr_next_frame(E, O);
+    const uint32_t m = (E[0] + c) * PK_MU;
+    fr_odd_row(E[0], c, O, PK_P1, PK_P3, PK_P5, PK_P7, m);
+    fr_even_row(E, O[7], PK_P0, PK_P2, PK_P4, PK_P6, m);
+  }
+  c = fr_next_frame(E, O);
+  return fr_join(E, O, c);
+}
+
+// Carry chains over n consecutive products a * y_j into X[0..2n).
+__device__ __forceinline__ void fr_chain1(uint32_t* X, uint32_t a, uint32_t y0) {
+  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
+      "madc.hi.u32   %1, %2, %3, %1;"
+      : "+r"(X[0]), "+r"(X[1])
+      : "r"(a), "r"(y0));
+}
+__device__ __forceinline__ void fr_chain1c(uint32_t* X, uint32_t a, uint32_t y0) {
+  asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+      "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+      "addc.u32       %2, 0, 0;"
+      : "+r"(X[0]), "+r"(X[1]), "=r"(X[2])
+      : "r"(a), "r"(y0));
+}
+__device__ __forceinline__ void fr_chain2(uint32_t* X, uint32_t a, uint32_t y0, uint32_t y1) {
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, %2;\n\t"
+      "madc.hi.u32    %3, %4, %6, %3;"
+      : "+r"(X[0]), "+r"(X[1]), "+r"(X[2]), "+r"(X[3])
+      : "r"(a), "r"(y0), "r"(y1));
+}
+__device__ __forceinline__ void fr_chain2c(uint32_t* X, uint32_t a, uint32_t y0, uint32_t y1) {
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;"
+      : "+r"(X[0]), "+r"(X[1]), "+r"(X[2]), "+r"(X[3]), "=r"(X[4])
+      : "r"(a), "r"(y0), "r"(y1));
+}
+__device__ __forceinline__ void fr_chain3(uint32_t* X, uint32_t a, uint32_t y0, uint32_t y1,
+                                          uint32_t y2) {
+  asm("mad.lo.cc.u32  %0, %6, %7, %0;\n\t"
+      "madc.hi.cc.u32 %1, %6, %7, %1;\n\t"
+      "madc.lo.cc.u32 %2, %6, %8, %2;\n\t"
+      "madc.hi.cc.u32 %3, %6, %8, %3;\n\t"
+      "madc.lo.cc.u32 %4, %6, %9, %4;\n\t"
+      "madc.hi.u32    %5, %6, %9, %5;"
+      : "+r"(X[0]), "+r"(X[1]), "+r"(X[2]), "+r"(X[3]), "+r"(X[4]), "+r"(X[5])
+      : "r"(a), "r"(y0), "r"(y1), "r"(y2));
+}
+__device__ __forceinline__ void fr_chain3c(uint32_t* X, uint32_t a, uint32_t y0, uint32_t y1,
+                                           uint32_t y2) {
+  asm("mad.lo.cc.u32  %0, %7, %8, %0;\n\t"
+      "madc.hi.cc.u32 %1, %7, %8, %1;\n\t"
+      "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
+      "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
+      "madc.lo.cc.u32 %4, %7, %10, %4;\n\t"
+      "madc.hi.cc.u32 %5, %7, %10, %5;\n\t"
+      "addc.u32       %6, 0, 0;"
+      : "+r"(X[0]), "+r"(X[1]), "+r"(X[2]), "+r"(X[3]), "+r"(X[4]), "+r"(X[5]), "=r"(X[6])
+      : "r"(a), "r"(y0), "r"(y1), "r"(y2));
+}
+
+// t[0..15] = a^2 for any 256-bit a: the 28 cross products a_i a_j (i < j)
+// once, those with i + j even in one accumulator and odd in the other (as in
+// a product row, each tiles its words), doubled, plus the 8 squares.
+__device__ __forceinline__ void fr_sqr_wide(const uint32_t* a, uint32_t* t) {
+  uint32_t o[15], e[14];
+#pragma unroll
+  for (int j = 1; j < 8; j++) {  // row 0
+    const uint64_t w = (uint64_t)a[0] * a[j];
+    uint32_t* x = (j & 1) ? o : e;
+    x[j] = (uint32_t)w;
+    x[j + 1] = (uint32_t)(w >> 32);
+  }
+  fr_chain3c(o + 3, a[1], a[2], a[4], a[6]);
+  e[8] = 0;
+  e[9] = 0;
+  fr_chain3(e + 4, a[1], a[3], a[5], a[7]);
+  o[10] = 0;
+  fr_chain3(o + 5, a[2], a[3], a[5], a[7]);
+  fr_chain2c(e + 6, a[2], a[4], a[6]);
+  fr_chain2c(o + 7, a[3], a[4], a[6]);
+  e[11] = 0;
+  fr_chain2(e + 8, a[3], a[5], a[7]);
+  o[12] = 0;
+  fr_chain2(o + 9, a[4], a[5], a[7]);
+  fr_chain1c(e + 10, a[4], a[6]);
+  fr_chain1c(o + 11, a[5], a[6]);
+  e[13] = 0;
+  fr_chain1(e + 12, a[5], a[7]);
+  o[14] = 0;
+  fr_chain1(o + 13, a[6], a[7]);
+  uint32_t s[15];  // e + o at words 1..14
+  s[1] = o[1];
+  asm("add.cc.u32  %0,  %13, %26;\n\t"
+      "addc.cc.u32 %1,  %14, %27;\n\t"
+      "addc.cc.u32 %2,  %15, %28;\n\t"
+      "addc.cc.u32 %3,  %16, %29;\n\t"
+      "addc.cc.u32 %4,  %17, %30;\n\t"
+      "addc.cc.u32 %5,  %18, %31;\n\t"
+      "addc.cc.u32 %6,  %19, %32;\n\t"
+      "addc.cc.u32 %7,  %20, %33;\n\t"
+      "addc.cc.u32 %8,  %21, %34;\n\t"
+      "addc.cc.u32 %9,  %22, %35;\n\t"
+      "addc.cc.u32 %10, %23, %36;\n\t"
+      "addc.cc.u32 %11, %24, %37;\n\t"
+      "addc.u32    %12, %25, 0;"
+      : "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(s[8]),
+        "=r"(s[9]), "=r"(s[10]), "=r"(s[11]), "=r"(s[12]), "=r"(s[13]), "=r"(s[14])
+      : "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]),
+        "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(e[2]), "r"(e[3]),
+        "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(e[8]), "r"(e[9]), "r"(e[10]),
+        "r"(e[11]), "r"(e[12]), "r"(e[13]));
+  t[0] = 0;
+  t[1] = s[1] << 1;
+#pragma unroll
+  for (int i = 2; i < 15; i++) t[i] = __funnelshift_l(s[i - 1], s[i], 1);
+  t[15] = s[14] >> 31;
+  asm("mad.lo.cc.u32  %0,  %16, %16, %0;\n\t"
+      "madc.hi.cc.u32 %1,  %16, %16, %1;\n\t"
+      "madc.lo.cc.u32 %2,  %17, %17, %2;\n\t"
+      "madc.hi.cc.u32 %3,  %17, %17, %3;\n\t"
+      "madc.lo.cc.u32 %4,  %18, %18, %4;\n\t"
+      "madc.hi.cc.u32 %5,  %18, %18, %5;\n\t"
+      "madc.lo.cc.u32 %6,  %19, %19, %6;\n\t"
+      "madc.hi.cc.u32 %7,  %19, %19, %7;\n\t"
+      "madc.lo.cc.u32 %8,  %20, %20, %8;\n\t"
+      "madc.hi.cc.u32 %9,  %20, %20, %9;\n\t"
+      "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
+      "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
+      "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
+      "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
+      "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
+      "madc.hi.u32    %15, %23, %23, %15;"
+      : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]),
+        "+r"(t[7]), "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]),
+        "+r"(t[14]), "+r"(t[15])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
+}
+
+// Montgomery square a^2 * 2^-256 mod p for a < 2p: 36 + 64 64-bit
+// multiply-adds.  The high half plus the reduced low half is below
+// 4 p^2 / 2^256 + p < 1.8 p.  Measured on B200: 78 G squares/s against 55 G/s
+// of the binary64 form (296 instructions) and 66 G/s of fr_mul(a, a).
 __device__ __forceinline__ Fr fr_sqr(const Fr& a) {
-  const uint32_t P[8] = {PK_P0, PK_P1, PK_P2, PK_P3, PK_P4, PK_P5, PK_P6, PK_P7};
-  uint32_t t[17];
-#pragma unroll
-  for (int i = 0; i < 17; i++) t[i] = 0;
-#pragma unroll
-  for (int i = 0; i < 7; i++) {
-    uint64_t c = 0;
-#pragma unroll
-    for (int j = i + 1; j < 8; j++) {
-      uint64_t s = (uint64_t)a.v[i] * a.v[j] + t[i + j] + c;
-      t[i + j] = (uint32_t)s;
-      c = s >> 32;
-    }
-    t[i + 8] = (uint32_t)c;
-  }
-#pragma unroll
-  for (int k = 15; k > 0; k--) t[k] = (t[k] << 1) | (t[k - 1] >> 31);
-  t[0] <<= 1;
-  uint64_t c = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    uint64_t sq = (uint64_t)a.v[i] * a.v[i];
-    uint64_t s = (uint64_t)t[2 * i] + (uint32_t)sq + c;
-    t[2 * i] = (uint32_t)s;
-    c = s >> 32;
-    s = (uint64_t)t[2 * i + 1] + (uint32_t)(sq >> 32) + c;
-    t[2 * i + 1] = (uint32_t)s;
-    c = s >> 32;
-  }
-  // reduction: t += m_i * p * 2^(32 i), i = 0..7 (a^2 < p^2 keeps t < 2^512 + p 2^256)
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint32_t m = t[i] * PK_MU;
-    uint64_t c2 = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      uint64_t s = (uint64_t)m * P[j] + t[i + j] + c2;
-      t[i + j] = (uint32_t)s;
-      c2 = s >> 32;
-    }
-#pragma unroll
-    for (int k = i + 8; k < 17; k++) {
-      uint64_t s = (uint64_t)t[k] + c2;
-      t[k] = (uint32_t)s;
-      c2 = s >> 32;
-    }
-  }
-  Fr r;
-#pragma unroll
-  for (int i = 0; i < 8; i++) r.v[i] = t[i + 8];
-  return fr_reduce_once(r);
+  uint32_t t[16];
+  fr_sqr_wide(a.v, t);
+  return fr_reduce_once(fr_add_raw(fr_redc(t), t + 8));
 }
 
 // canonical -> Montgomery: a * R^2 * R^-1
@@ -299,29 +479,10 @@ __device__ __forceinline__ Fr fr_to_mont(const Fr& a) {
   return fr_mul(a, r2);
 }
 
-// Montgomery -> canonical: a * 1 * R^-1
-// Montgomery -> canonical, a * 2^-256 mod p, for any 256-bit a: the
-// word-by-word Montgomery reduction alone (REDC, 8 x (1 + 16) multiply-adds
-// on the integer pipe, no product); t < 2^256 + p 2^256 keeps 9 words, the
-// result is < p + 1 before the one conditional subtraction.
-__device__ __forceinline__ Fr fr_from_mont(const Fr& a) {
-  uint32_t t[9];
-#pragma unroll
-  for (int i = 0; i < 8; i++) t[i] = a.v[i];
-  t[8] = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint32_t m = t[0] * PK_MU;
-    PK_ROW_P(t, m);
-#pragma unroll
-    for (int j = 0; j < 8; j++) t[j] = t[j + 1];
-    t[8] = 0;
-  }
-  Fr r;
-#pragma unroll
-  for (int i = 0; i < 8; i++) r.v[i] = t[i];
-  return fr_reduce_once(r);
-}
+// Montgomery -> canonical, a * 2^-256 mod p, for any 256-bit a: the reduction
+// alone.  Measured on B200: 121 G/s against 84 G/s with separate low and high
+// chains.
+__device__ __forceinline__ Fr fr_from_mont(const Fr& a) { return fr_reduce_once(fr_redc(a.v)); }
 
 __device__ __forceinline__ bool fr_eq(const Fr& a, const Fr& b) {
   uint32_t d = 0;

@@ -1,9 +1,9 @@
 // BN254 Fr Montgomery product and square on the FP64 (DFMA) pipe.
 //
-// B200 issues double-precision FMAs at the same rate as 32-bit integer
-// multiply-adds, and the two share that throughput (mixing them gains
-// nothing), so the form that is faster on its own wins; on B200 that is this
-// one (352 binary64 instructions per product, 296 per square).  These routines compute exactly the same integers as fr_mul / fr_sqr
+// The form of pkg_fr_mul_batch's FP64 operations.  The kernels multiply on the
+// integer pipe (fr.cuh): there a product is 128 64-bit multiply-adds of four
+// issue cycles each and here 352 binary64 instructions of two, on one shared
+// throughput (65.8 against 44.8 G products/s).  These routines compute exactly the same integers as fr_mul / fr_sqr
 // (a*b*2^-256 mod p, fully reduced), but do their products in binary64.  They follow the idea of Emmart, Zheng and Weems,
 // "Faster Modular Exponentiation Using Double Precision Floating Point
 // Arithmetic on the GPU" (ARITH 2018), with a digit size chosen so that no
@@ -120,23 +120,6 @@ __device__ __forceinline__ Fr fr_mul_f64(const Fr& a, const Fr& b) {
   for (int i = 0; i < 11; i++) {
 #pragma unroll
     for (int j = 0; j < 11; j++) T[j] = fma(A[i], B[j], T[j]);
-    if (i < 10) f64::step24(T);
-  }
-  return f64::tail16(T);
-}
-
-// fr_mul_f64 with the first operand already in digit form (A: the 11 digits
-// f64::digits produced, e.g. a twiddle converted once and shared).
-__device__ __forceinline__ Fr fr_mul_f64_digits(const double* A, const Fr& b) {
-  double B[11], T[11];
-  f64::digits(b, B);
-#pragma unroll
-  for (int j = 0; j < 11; j++) T[j] = 0.0;
-#pragma unroll
-  for (int i = 0; i < 11; i++) {
-    const double ai = A[i];
-#pragma unroll
-    for (int j = 0; j < 11; j++) T[j] = fma(ai, B[j], T[j]);
     if (i < 10) f64::step24(T);
   }
   return f64::tail16(T);

@@ -1,6 +1,6 @@
 // Element-wise Fr operations over device arrays on either multiply pipe:
-// the FP64-pipe routines (fr_f64.cuh) that the NTT and Skyscraper kernels use,
-// and the integer-pipe ones (fr.cuh).  A parity and microbenchmark surface
+// the integer-pipe routines (fr.cuh) that the library's kernels use, and the
+// FP64-pipe ones (fr_f64.cuh).  A parity and microbenchmark surface
 // for the field arithmetic itself (the reference's scalar_mul / scalar_sqr,
 // skyscraper/bn254-multiplier/src/scalar.rs:12-132, and ark-ff's
 // from_montgomery).

@@ -17,7 +17,6 @@
 #include <vector>
 
 #include "fr.cuh"
-#include "fr_f64.cuh"
 #include "fr_host.hpp"
 #include "ntt_internal.cuh"
 #include "host_stage.cuh"
@@ -169,10 +168,8 @@ __device__ __forceinline__ Fr source_load(const NttSource& s, uint64_t g) {
 }
 
 // kModeB selects mode B at compile time.  In mode A every line of the CTA
-// shares `high`, so stage s needs only the 2^s twiddles roots[(high << s) |
-// grp]; they are converted to FP64 digits once per CTA into shared memory
-// after the data tile (double-buffered across stages, 2 x 2^(K-1) x 11
-// doubles) instead of once per butterfly.
+// shares `high`, so stage s reads only the 2^s twiddles roots[(high << s) |
+// grp], which stay in L1.
 template <int K, bool kSrc, bool kModeB>
 __global__ void __launch_bounds__(512) ntt_pass_kernel(uint64_t* __restrict__ data,
                                                       const uint64_t* __restrict__ roots,
@@ -182,8 +179,6 @@ __global__ void __launch_bounds__(512) ntt_pass_kernel(uint64_t* __restrict__ da
   constexpr int R = 1 << K;
   constexpr bool mode_b = kModeB;
   const int E = R * T;
-  double* tw = reinterpret_cast<double*>(sm + 2 * E);
-  constexpr int kTw = (R / 2) * 11;
   const uint64_t l0 = (uint64_t)blockIdx.x * T;
   uint64_t high_a = 0, u0 = 0;
   if (!mode_b) {
@@ -215,7 +210,6 @@ __global__ void __launch_bounds__(512) ntt_pass_kernel(uint64_t* __restrict__ da
       sm[E + sidx] = in[1];  // high 16 bytes: plane 1
     }
   }
-  if (!kModeB && threadIdx.x == 0) f64::digits(fr_load_ro(roots, high_a), tw);  // stage 0
   __syncthreads();
   // ---- K radix-2 stages in shared memory ----
 #pragma unroll 1
@@ -237,27 +231,14 @@ __global__ void __launch_bounds__(512) ntt_pass_kernel(uint64_t* __restrict__ da
       bb = sm[E + i1];
       x1.v[0] = a.x; x1.v[1] = a.y; x1.v[2] = a.z; x1.v[3] = a.w;
       x1.v[4] = bb.x; x1.v[5] = bb.y; x1.v[6] = bb.z; x1.v[7] = bb.w;
-      Fr m;
-      if (kModeB) {
-        const uint64_t high = (l0 + ll) >> log_u;
-        m = fr_mul_f64(fr_load_ro(roots, (high << s) | (uint64_t)grp), x1);
-      } else {
-        m = fr_mul_f64_digits(tw + (s & 1) * kTw + 11 * grp, x1);
-      }
+      const uint64_t high = kModeB ? (l0 + ll) >> log_u : high_a;
+      const Fr m = fr_mul(x1, fr_load_ro(roots, (high << s) | (uint64_t)grp));
       Fr y0 = fr_add(x0, m);
       Fr y1 = fr_sub(x0, m);
       sm[i0] = make_uint4(y0.v[0], y0.v[1], y0.v[2], y0.v[3]);
       sm[E + i0] = make_uint4(y0.v[4], y0.v[5], y0.v[6], y0.v[7]);
       sm[i1] = make_uint4(y1.v[0], y1.v[1], y1.v[2], y1.v[3]);
       sm[E + i1] = make_uint4(y1.v[4], y1.v[5], y1.v[6], y1.v[7]);
-    }
-    // next stage's twiddles into the other buffer: no thread reads it before
-    // the barrier below, and its previous readers finished before the last one
-    if (!kModeB && s + 1 < K) {
-#pragma unroll 1
-      for (int g = threadIdx.x; g < (2 << s); g += blockDim.x)
-        f64::digits(fr_load_ro(roots, (high_a << (s + 1)) | (uint64_t)g),
-                    tw + ((s + 1) & 1) * kTw + 11 * g);
     }
     __syncthreads();
   }
@@ -336,7 +317,7 @@ int ntt_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end, const
     uint64_t E = (uint64_t(1) << K) * T;
     int threads = (int)std::min<uint64_t>((E / 2) >> PK_NTT_LOG_BPT, 512);
     if (threads < 32) threads = 32;
-    size_t smem = 32 * E + (mode_b ? 0 : sizeof(double) * 2 * 11 * (size_t(1) << (K - 1)));
+    size_t smem = 32 * E;
     uint64_t grid = num_lines / T;
     const bool from_src = src != nullptr && pi == 0;
     PassFn fn = pass_fn(K, from_src, mode_b != 0);

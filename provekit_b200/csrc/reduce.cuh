@@ -10,7 +10,6 @@
 #include <algorithm>
 
 #include "fr.cuh"
-#include "fr_f64.cuh"
 #include "pk_common.cuh"
 
 namespace pk {
@@ -89,7 +88,7 @@ __device__ __forceinline__ void block_finish(Fr (&v)[K], const RedOut& ro,
   if (threadIdx.x == 0) {
     if (scale)
 #pragma unroll
-      for (int k = 0; k < K; k++) v[k] = fr_mul_f64(v[k], *scale);
+      for (int k = 0; k < K; k++) v[k] = fr_mul(v[k], *scale);
 #pragma unroll
     for (int k = 0; k < K; k++) fr_store(ro.part, (size_t)blockIdx.x * K + k, v[k]);
     if (ro.ticket) {

@@ -8,7 +8,6 @@
 #include <vector>
 
 #include "fr.cuh"
-#include "fr_f64.cuh"
 #include "fr_host.hpp"
 #include "pk_common.cuh"
 
@@ -537,7 +536,7 @@ __device__ void chacha20_block_dev(uint32_t k0, uint32_t k1, uint64_t counter, u
 }
 
 // out[i] = lo + hi 2^253 mod p (Montgomery) from ChaCha20 block start + i,
-// as two products on the FP64 pipe: lo * R^2 and hi * (2^253 R^2), each
+// as two products: lo * R^2 and hi * (2^253 R^2), each
 // times R^-1 (lo, hi < 2^253 < p).
 __global__ void sample_indexed_kernel(uint32_t k0, uint32_t k1, uint64_t start, size_t n, Fr r2,
                                       Fr t253r2, uint64_t* __restrict__ out) {
@@ -553,7 +552,7 @@ __global__ void sample_indexed_kernel(uint32_t k0, uint32_t k1, uint64_t start, 
     }
     lo.v[7] &= 0x1fffffffu;
     hi.v[7] &= 0x1fffffffu;
-    fr_store(out, i, fr_add(fr_mul_f64(lo, r2), fr_mul_f64(hi, t253r2)));
+    fr_store(out, i, fr_add(fr_mul(lo, r2), fr_mul(hi, t253r2)));
   }
 }
 }  // namespace pk

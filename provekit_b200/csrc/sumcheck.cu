@@ -20,7 +20,6 @@
 #include <vector>
 
 #include "fr.cuh"
-#include "fr_f64.cuh"
 #include "fr_host.hpp"
 #include "fr_lazy.cuh"
 #include "pk_common.cuh"
@@ -57,7 +56,7 @@ __global__ void eq_small_kernel(const uint64_t* __restrict__ r, int nr, uint64_t
     for (int i = 0; i < nr; i++) {
       Fr ri = fr_load_ro(r, i);
       Fr f = ((x >> (nr - 1 - i)) & 1) ? ri : fr_sub(fr_one_mont(), ri);
-      acc = fr_mul_f64(acc, f);
+      acc = fr_mul(acc, f);
     }
     fr_store(out, x, acc);
   }
@@ -68,7 +67,7 @@ __global__ void eq_combine_kernel(const uint64_t* __restrict__ hi, const uint64_
                                   int nlo, size_t num_entries, uint64_t* __restrict__ out) {
   for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < num_entries;
        x += (size_t)gridDim.x * blockDim.x) {
-    fr_store(out, x, fr_mul_f64(fr_load_ro(hi, x >> nlo), fr_load_ro(lo, x & ((size_t(1) << nlo) - 1))));
+    fr_store(out, x, fr_mul(fr_load_ro(hi, x >> nlo), fr_load_ro(lo, x & ((size_t(1) << nlo) - 1))));
   }
 }
 
@@ -87,7 +86,7 @@ __global__ void spmv_csr_kernel(const uint64_t* __restrict__ row_ptr, const uint
         atomicOr(err, 1u);
         continue;
       }
-      acc = fr_add(acc, fr_mul_f64(fr_load_ro(vals, k), fr_load_ro(x, col)));
+      acc = fr_add(acc, fr_mul(fr_load_ro(vals, k), fr_load_ro(x, col)));
     }
     fr_store(y, row, acc);
   }
@@ -109,7 +108,7 @@ __global__ void spmv_products_kernel(const uint32_t* __restrict__ cols,
     if (col >= num_cols)
       atomicOr(err, 1u);
     else
-      v = fr_mul_f64(fr_load_ro(vals, k), fr_load_ro(x, col));
+      v = fr_mul(fr_load_ro(vals, k), fr_load_ro(x, col));
     fr_store(prod, k, v);
   }
 }
@@ -149,7 +148,7 @@ __global__ void witness_bounds_kernel(const uint64_t* __restrict__ rpa,
           atomicOr(err, 1u);
           continue;
         }
-        a = fr_add(a, fr_mul_f64(fr_load_ro(va, k), fr_load_ro(w, col)));
+        a = fr_add(a, fr_mul(fr_load_ro(va, k), fr_load_ro(w, col)));
       }
       for (uint64_t k = rpb[row]; k < rpb[row + 1]; k++) {
         const uint32_t col = cb[k];
@@ -157,9 +156,9 @@ __global__ void witness_bounds_kernel(const uint64_t* __restrict__ rpa,
           atomicOr(err, 1u);
           continue;
         }
-        b = fr_add(b, fr_mul_f64(fr_load_ro(vb, k), fr_load_ro(w, col)));
+        b = fr_add(b, fr_mul(fr_load_ro(vb, k), fr_load_ro(w, col)));
       }
-      c = fr_mul_f64(a, b);
+      c = fr_mul(a, b);
     }
     fr_store(ta, row, a);
     fr_store(tb, row, b);
@@ -171,7 +170,7 @@ __global__ void hadamard_pad_kernel(const uint64_t* __restrict__ a, const uint64
                                     size_t n, size_t padded, uint64_t* __restrict__ c) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < padded;
        i += (size_t)gridDim.x * blockDim.x)
-    fr_store(c, i, i < n ? fr_mul_f64(fr_load_ro(a, i), fr_load_ro(b, i)) : fr_zero());
+    fr_store(c, i, i < n ? fr_mul(fr_load_ro(a, i), fr_load_ro(b, i)) : fr_zero());
 }
 
 // The products are summed unreduced (fr_lazy.cuh) and reduced once per

@@ -20,7 +20,6 @@
 #include <vector>
 
 #include "fr.cuh"
-#include "fr_f64.cuh"
 #include "fr_host.hpp"
 #include "fr_lazy.cuh"
 #include "internal.cuh"
@@ -69,7 +68,7 @@ __global__ void whir_fold_coeffs_kernel(const uint64_t* __restrict__ c, size_t L
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < L;
        i += (size_t)gridDim.x * blockDim.x) {
     Fr acc = fr_load_ro(c, i);
-    for (int j = 1; j < m; j++) acc = fr_add(acc, fr_mul_f64(param_fr(W, j), fr_load_ro(c, j * L + i)));
+    for (int j = 1; j < m; j++) acc = fr_add(acc, fr_mul(param_fr(W, j), fr_load_ro(c, j * L + i)));
     fr_store(out, i, acc);
   }
 }
@@ -82,7 +81,7 @@ __global__ void whir_fold_rows_kernel(const uint64_t* __restrict__ rows, size_t 
        i += (size_t)gridDim.x * blockDim.x) {
     Fr acc = fr_load_ro(rows, i * m);
     for (int j = 1; j < m; j++)
-      acc = fr_add(acc, fr_mul_f64(param_fr(W, j), fr_load_ro(rows, i * m + j)));
+      acc = fr_add(acc, fr_mul(param_fr(W, j), fr_load_ro(rows, i * m + j)));
     fr_store(out, i, acc);
   }
 }
@@ -111,25 +110,25 @@ __global__ void __launch_bounds__(kRedThreads) poly_eval_kernel(
     const Fr y = param_fr(P, 0);
     const size_t end = n < c0 + C ? n : c0 + C;
     for (size_t k = (end - 1 - c0 - j) / kRedThreads + 1; k-- > 0;)
-      acc = fr_add(fr_mul_f64(acc, y), fr_load_ro(c, c0 + j + (size_t)kRedThreads * k));
+      acc = fr_add(fr_mul(acc, y), fr_load_ro(c, c0 + j + (size_t)kRedThreads * k));
   }
   Fr scale = fr_one_mont();
   if (j == 0)
     for (int b = 0; b < kEvalScaleBits; b++)
-      if ((blockIdx.x >> b) & 1) scale = fr_mul_f64(scale, param_fr(P, 1 + kEvalTreeLevels + b));
+      if ((blockIdx.x >> b) & 1) scale = fr_mul(scale, param_fr(P, 1 + kEvalTreeLevels + b));
   tree[j] = acc;
   __syncthreads();
 #pragma unroll 1
   for (int l = 0; l < kEvalTreeLevels; l++) {
     const unsigned half = kRedThreads >> (l + 1);
     Fr v;
-    if (j < half) v = fr_add(tree[2 * j], fr_mul_f64(param_fr(P, 1 + l), tree[2 * j + 1]));
+    if (j < half) v = fr_add(tree[2 * j], fr_mul(param_fr(P, 1 + l), tree[2 * j + 1]));
     __syncthreads();
     if (j < half) tree[j] = v;
     __syncthreads();
   }
   Fr out[1] = {fr_zero()};
-  if (j == 0) out[0] = fr_mul_f64(tree[0], scale);
+  if (j == 0) out[0] = fr_mul(tree[0], scale);
   block_finish<1>(out, ro);
 }
 
@@ -169,7 +168,7 @@ __global__ void gather_rows_kernel(const uint64_t* __restrict__ cw, size_t row_f
 // The round kernel's seven products go through one out-of-line call, and the
 // kernel is bounded to two CTAs per SM (128 registers): with them inlined the
 // folding kernel took 172 registers, one CTA of 256 threads per SM.
-static __device__ __noinline__ Fr whir_mul(const Fr a, const Fr b) { return fr_mul_f64(a, b); }
+static __device__ __noinline__ Fr whir_mul(const Fr a, const Fr b) { return fr_mul(a, b); }
 
 template <bool kFold>
 __global__ void __launch_bounds__(kRedThreads, 2) whir_round_kernel(
@@ -211,7 +210,7 @@ __global__ void eq_tables_kernel(const uint64_t* __restrict__ pts, size_t stride
     for (int i = 0; i < k; i++) {
       const Fr p = fr_load_ro(pts, j * stride + first + i);
       const bool bit = (x >> (k - 1 - i)) & 1;
-      acc = fr_mul_f64(acc, bit ? p : fr_sub(fr_one_mont(), p));
+      acc = fr_mul(acc, bit ? p : fr_sub(fr_one_mont(), p));
     }
     fr_store(tables, t, acc);
   }
@@ -227,7 +226,7 @@ __global__ void expand_points_kernel(const uint64_t* __restrict__ raw, size_t np
     Fr acc = fr_load_ro(raw, j);
     for (size_t i = 0; i < nv; i++) {
       fr_store(out, j * nv + nv - 1 - i, acc);
-      acc = fr_sqr_f64(acc);
+      acc = fr_sqr(acc);
     }
   }
 }
@@ -239,20 +238,18 @@ __global__ void eq_accumulate_kernel(uint64_t* __restrict__ w, size_t n, int nlo
   const size_t nlo_entries = size_t(1) << nlo;
   for (size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x; b < n;
        b += (size_t)gridDim.x * blockDim.x) {
-    // two independent products per step, one on the FP64 pipe and one on
-    // the integer pipe (the CIOS routine; the same integers), which issue
-    // side by side
+    // two independent products per step
     const size_t bh = b >> nlo, bl = b & (nlo_entries - 1);
     Fr acc = fr_load(w, b), acc2 = fr_zero();
     size_t j = 0;
     for (; j + 1 < npts; j += 2) {
-      acc = fr_add(acc, fr_mul_f64(fr_load_ro(hi, j * nhi_entries + bh),
+      acc = fr_add(acc, fr_mul(fr_load_ro(hi, j * nhi_entries + bh),
                                    fr_load_ro(lo, j * nlo_entries + bl)));
       acc2 = fr_add(acc2, fr_mul(fr_load_ro(hi, (j + 1) * nhi_entries + bh),
                                  fr_load_ro(lo, (j + 1) * nlo_entries + bl)));
     }
     if (j < npts)
-      acc = fr_add(acc, fr_mul_f64(fr_load_ro(hi, j * nhi_entries + bh),
+      acc = fr_add(acc, fr_mul(fr_load_ro(hi, j * nhi_entries + bh),
                                    fr_load_ro(lo, j * nlo_entries + bl)));
     fr_store(w, b, fr_add(acc, acc2));
   }

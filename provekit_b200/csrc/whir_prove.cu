@@ -25,7 +25,6 @@
 #include <vector>
 
 #include "fr.cuh"
-#include "fr_f64.cuh"
 #include "fr_host.hpp"
 #include "fr_lazy.cuh"
 #include "internal.cuh"
@@ -132,7 +131,7 @@ __global__ void combine_covectors_kernel(uint64_t* __restrict__ w, size_t n,
       Fr c;
 #pragma unroll
       for (int i = 0; i < 8; i++) c.v[i] = P.coef[a][i];
-      acc = fr_add(acc, fr_mul_f64(c, fr_load_ro(P.cov, (size_t)a * P.stride + b)));
+      acc = fr_add(acc, fr_mul(c, fr_load_ro(P.cov, (size_t)a * P.stride + b)));
     }
     fr_store(w, b, acc);
   }
@@ -193,8 +192,8 @@ __global__ void fold_tables_kernel(uint64_t* __restrict__ f, uint64_t* __restric
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < h;
        i += (size_t)gridDim.x * blockDim.x) {
     const Fr f0 = fr_load(f, i), w0 = fr_load(w, i);
-    fr_store(f, i, fr_add(f0, fr_mul_f64(r, fr_sub(fr_load(f, i + h), f0))));
-    fr_store(w, i, fr_add(w0, fr_mul_f64(r, fr_sub(fr_load(w, i + h), w0))));
+    fr_store(f, i, fr_add(f0, fr_mul(r, fr_sub(fr_load(f, i + h), f0))));
+    fr_store(w, i, fr_add(w0, fr_mul(r, fr_sub(fr_load(w, i + h), w0))));
   }
 }
 

@@ -1,6 +1,6 @@
 """Element-wise BN254 Fr arithmetic on device tensors (pkg_fr_mul_batch): the
-Montgomery product, square and Montgomery->canonical conversion on the FP64
-pipe (the routines inside the NTT and Skyscraper kernels) or the integer pipe.
+Montgomery product, square and Montgomery->canonical conversion on the integer
+pipe (the routines inside the library's kernels) or the FP64 pipe.
 Mirrors skyscraper/bn254-multiplier/src/scalar.rs:12-132 (scalar_mul,
 scalar_sqr) up to the residue (results here are fully reduced)."""
 import torch
