@@ -383,6 +383,21 @@ __device__ __forceinline__ void fr_chain3c(uint32_t* X, uint32_t a, uint32_t y0,
       : "r"(a), "r"(y0), "r"(y1), "r"(y2));
 }
 
+__device__ __forceinline__ void fr_chain4(uint32_t* X, uint32_t a, uint32_t y0, uint32_t y1,
+                                          uint32_t y2, uint32_t y3) {
+  asm("mad.lo.cc.u32  %0, %8, %9,  %0;\n\t"
+      "madc.hi.cc.u32 %1, %8, %9,  %1;\n\t"
+      "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
+      "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
+      "madc.lo.cc.u32 %4, %8, %11, %4;\n\t"
+      "madc.hi.cc.u32 %5, %8, %11, %5;\n\t"
+      "madc.lo.cc.u32 %6, %8, %12, %6;\n\t"
+      "madc.hi.u32    %7, %8, %12, %7;"
+      : "+r"(X[0]), "+r"(X[1]), "+r"(X[2]), "+r"(X[3]), "+r"(X[4]), "+r"(X[5]), "+r"(X[6]),
+        "+r"(X[7])
+      : "r"(a), "r"(y0), "r"(y1), "r"(y2), "r"(y3));
+}
+
 // t[0..15] = a^2 for any 256-bit a: the 28 cross products a_i a_j (i < j)
 // once, those with i + j even in one accumulator and odd in the other (as in
 // a product row, each tiles its words), doubled, plus the 8 squares.

@@ -8,10 +8,10 @@
 //   pkg_whir_commit               RS encode + Merkle tree of one polynomial
 //
 // One thread owns one compression chain (a leaf's left fold, or one node);
-// 32-byte chunks are read as two 128-bit vector loads.  Levels above
-// kSubtreeMax nodes take one launch each; below it one launch reduces
-// 256-node subtrees per CTA by eight levels, and one CTA finishes the top in
-// shared memory.
+// 32-byte chunks are read as two 128-bit vector loads.  Folds run 128 messages
+// at a time with their reductions on the tensor cores (sky_tc.cuh).  Levels
+// above kSubtreeMax nodes take one launch each; below it one launch reduces
+// 256-node subtrees per CTA by eight levels.
 #include <algorithm>
 #include <cstring>
 
@@ -22,10 +22,9 @@
 #include "pk_common.cuh"
 #include "rs_internal.cuh"
 #include "skyscraper.cuh"
+#include "sky_tc.cuh"
 
 namespace pk {
-
-constexpr int kTopNodes = 1024;  // nodes finished inside one CTA
 
 // CTAs of 128 threads per SM the leaf kernel is compiled for (its register
 // budget: 7 -> 72 registers).
@@ -58,20 +57,6 @@ __global__ void compress_many_kernel(const uint8_t* __restrict__ in, size_t n,
   }
 }
 
-// Left fold h = c(c(c(e0, e1), e2), ...) over `chunks` 32-byte chunks
-// (one compression call site keeps the register count low).
-__global__ void leaf_fold_kernel(const uint8_t* __restrict__ in, size_t size, size_t chunks,
-                                 size_t count, uint8_t* __restrict__ out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const uint8_t* msg = in + i * size;
-    Fr acc = load_raw(msg);
-#pragma unroll 1
-    for (size_t k = 1; k < chunks; k++) acc = sky_compress(acc, load_raw(msg + 32 * k));
-    store_raw(out + 32 * i, acc);
-  }
-}
-
 // Leaves straight from an Fr codeword: leaf i = row i (fr_per_leaf
 // consecutive Fr).  Canonical encoding converts each Montgomery element
 // (x*2^256 -> x) before hashing; Montgomery encoding hashes the raw limbs.
@@ -94,92 +79,107 @@ __global__ void __launch_bounds__(128, PK_LEAF_MIN_CTAS) leaf_fold_fr_kernel(con
   }
 }
 
-// One tree level: out[i] = compress(in[2i], in[2i+1]).
-__global__ void merkle_level_kernel(const uint8_t* __restrict__ in, size_t n_out,
-                                    uint8_t* __restrict__ out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n_out;
-       i += (size_t)gridDim.x * blockDim.x) {
-    store_raw(out + 32 * i, sky_compress(load_raw(in + 64 * i), load_raw(in + 64 * i + 32)));
+// ---- the same on the tensor cores (sky_tc.cuh) ---------------------------
+// A CTA takes tiles of skytc::kThreads messages; threads past the end work on
+// the last one and store nothing.
+struct ByteMessages {  // chunks of 32 bytes, hashed as they are
+  static constexpr bool kMont = false;
+  const uint8_t* in;
+  size_t size;
+  __device__ __forceinline__ Fr first(size_t i) const { return skytc::reduce_any(load_raw(in + i * size)); }
+  __device__ __forceinline__ Fr at(size_t i, size_t k) const { return load_raw(in + i * size + 32 * k); }
+};
+template <bool kCanonical>
+struct CodewordRows {  // rows of Fr, in canonical form or as their Montgomery limbs
+  static constexpr bool kMont = kCanonical;
+  const uint64_t* cw;
+  size_t fr_per_leaf;
+  __device__ __forceinline__ Fr first(size_t i) const {
+    const Fr x = fr_load_ro(cw, i * fr_per_leaf);
+    return kCanonical ? fr_from_mont(x) : skytc::reduce_any(x);
   }
+  __device__ __forceinline__ Fr at(size_t i, size_t k) const {
+    return fr_load_ro(cw, i * fr_per_leaf + k);
+  }
+};
+
+// Left fold of `chunks` >= 2 chunks of each message.
+template <class Messages>
+__global__ void __launch_bounds__(skytc::kThreads, skytc::kMinCtas)
+    fold_tc_kernel(const Messages msgs, size_t chunks, size_t count, uint8_t* __restrict__ out) {
+  __shared__ skytc::Shared sh;
+  skytc::Tile tile;
+  tile.open(sh);
+  for (size_t base = (size_t)blockIdx.x * skytc::kThreads; base < count;
+       base += (size_t)gridDim.x * skytc::kThreads) {
+    const size_t i = base + threadIdx.x, row = i < count ? i : count - 1;
+    Fr acc = msgs.first(row);
+#pragma unroll 1
+    for (size_t k = 1; k < chunks; k++)
+      acc = tile.compress<Messages::kMont>(acc, msgs.at(row, k));
+    if (i < count) store_raw(out + 32 * i, fr_reduce_once(acc));
+  }
+  tile.close(sh);
 }
 
-// The remaining levels from n (<= kTopNodes, power of two) nodes up to the
-// root, in one CTA: level digests live in shared memory and are also written
-// out to their slots in the layer array.
-__global__ void __launch_bounds__(512) merkle_top_kernel(const uint8_t* __restrict__ in,
-                                                         size_t n, uint8_t* __restrict__ out) {
-  __shared__ uint4 buf[2 * kTopNodes];
-  for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint4* q = reinterpret_cast<const uint4*>(in + 32 * i);
-    buf[2 * i] = q[0];
-    buf[2 * i + 1] = q[1];
-  }
-  __syncthreads();
-  size_t off = 0;
-  while (n > 1) {
-    const size_t half = n / 2;  // <= blockDim.x: one node per thread
-    Fr h;
-    if (threadIdx.x < half) {
-      const size_t i = threadIdx.x;
-      Fr l, r;
-      uint4 a = buf[4 * i], b = buf[4 * i + 1], c = buf[4 * i + 2], d = buf[4 * i + 3];
-      l.v[0] = a.x; l.v[1] = a.y; l.v[2] = a.z; l.v[3] = a.w;
-      l.v[4] = b.x; l.v[5] = b.y; l.v[6] = b.z; l.v[7] = b.w;
-      r.v[0] = c.x; r.v[1] = c.y; r.v[2] = c.z; r.v[3] = c.w;
-      r.v[4] = d.x; r.v[5] = d.y; r.v[6] = d.z; r.v[7] = d.w;
-      h = sky_compress(l, r);
-    }
-    __syncthreads();
-    if (threadIdx.x < half) {
-      const size_t i = threadIdx.x;
-      buf[2 * i] = make_uint4(h.v[0], h.v[1], h.v[2], h.v[3]);
-      buf[2 * i + 1] = make_uint4(h.v[4], h.v[5], h.v[6], h.v[7]);
-      store_raw(out + 32 * (off + i), h);
-    }
-    __syncthreads();
-    off += half;
-    n = half;
-  }
+// Folds of three or more chunks always run here: 6.2 us per compression of a
+// chain and 5 us to set up, against 8 and 2.5 in sky_compress.  A single
+// compression each (two chunks) pays from above 2^15 messages on: 2^14 take
+// 12.7 us here and 12.6 there, 2^16 20.9 and 24.8.
+constexpr size_t kTcMinPairs = (size_t(1) << 15) + 1;
+static bool tc_wanted(size_t count, size_t chunks) {
+  return chunks >= 3 || (chunks == 2 && count >= kTcMinPairs);
 }
 
-// The levels from kSubtreeMax nodes down: each CTA (one warp per SM
-// sub-partition) reduces kSubNodes consecutive nodes of the current level by
-// kSubLevels levels in shared memory and writes every level's digests to
-// their slots, so the latency-bound small levels cost one launch instead of
-// one each; the kSubNodes-fold fewer subroots go to merkle_top_kernel.
-constexpr int kSubThreads = 128;
-constexpr int kSubNodes = 2 * kSubThreads;
-constexpr int kSubLevels = 8;  // kSubNodes = 2^kSubLevels
-constexpr size_t kSubtreeMax = size_t(1) << 15;
-static_assert(kSubNodes == 1 << kSubLevels, "a CTA reduces its nodes to one subroot");
-static_assert(kSubtreeMax / kSubNodes <= (size_t)kTopNodes, "the subroots fit the top kernel");
+template <class Messages>
+static int fold_tc(const Messages& msgs, size_t chunks, size_t count, uint8_t* out,
+                   cudaStream_t s) {
+  const size_t tiles = (count + skytc::kThreads - 1) / skytc::kThreads;
+  const size_t cap = (size_t)sm_count() * skytc::kMinCtas;
+  fold_tc_kernel<Messages><<<(unsigned)std::min(tiles, cap), skytc::kThreads, 0, s>>>(
+      msgs, chunks, count, out);
+  PK_CHECK_LAUNCH("fold_tc_kernel");
+  return PKG_OK;
+}
 
-__global__ void __launch_bounds__(kSubThreads) merkle_subtree_kernel(uint8_t* __restrict__ lvl,
-                                                                     size_t n) {
+// All the levels above `nodes` (a power of two <= kSubNodes) consecutive nodes
+// of a level per CTA, in shared memory, each level's digests also written to
+// their slots: the small levels are latency-bound (one compression's latency
+// each, whatever their width), so they share one launch.  lvl: the level's
+// first node; n: its nodes, the slots of the next level following them.
+constexpr int kSubNodes = 2 * skytc::kThreads;
+// A level of 2^16 nodes ends in one launch fewer this way (115 -> 113 us for
+// the whole tree above it); from 2^17 on eight partly idle levels of that many
+// CTAs cost what the launches save (134 and 135 us).
+constexpr size_t kSubtreeMax = size_t(1) << 16;
+
+__global__ void __launch_bounds__(skytc::kThreads, 5)
+    merkle_subtree_kernel(uint8_t* __restrict__ lvl, size_t n, int nodes) {
+  __shared__ skytc::Shared sh;
   __shared__ uint4 buf[2 * kSubNodes];
-  const size_t c = blockIdx.x;  // this CTA's nodes: [c kSubNodes, (c + 1) kSubNodes)
-  for (int i = threadIdx.x; i < kSubNodes; i += blockDim.x) {
-    const uint4* q = reinterpret_cast<const uint4*>(lvl + 32 * (c * kSubNodes + i));
-    buf[2 * i] = q[0];
-    buf[2 * i + 1] = q[1];
-  }
+  skytc::Tile tile;
+  tile.open(sh);
+  const size_t c = blockIdx.x;  // this CTA's nodes: [c nodes, (c + 1) nodes)
+  for (int i = threadIdx.x; i < 2 * nodes; i += blockDim.x)
+    buf[i] = reinterpret_cast<const uint4*>(lvl + 32 * c * nodes)[i];
   __syncthreads();
   uint8_t* level = lvl;  // first node of the current level
   size_t level_n = n;
-  int cnt = kSubNodes;
 #pragma unroll 1
-  for (int l = 0; l < kSubLevels; l++) {
-    const int half = cnt / 2;
+  for (int half = nodes / 2; half > 0; half /= 2) {
     const int i = threadIdx.x;
     Fr h;
-    if (i < half) {
+    if ((int)tile.warp * 32 < half) {
+      const int j = i < half ? i : 0;
       Fr a, b;
-      const uint4 x0 = buf[4 * i], x1 = buf[4 * i + 1], y0 = buf[4 * i + 2], y1 = buf[4 * i + 3];
+      const uint4 x0 = buf[4 * j], x1 = buf[4 * j + 1], y0 = buf[4 * j + 2], y1 = buf[4 * j + 3];
       a.v[0] = x0.x; a.v[1] = x0.y; a.v[2] = x0.z; a.v[3] = x0.w;
       a.v[4] = x1.x; a.v[5] = x1.y; a.v[6] = x1.z; a.v[7] = x1.w;
       b.v[0] = y0.x; b.v[1] = y0.y; b.v[2] = y0.z; b.v[3] = y0.w;
       b.v[4] = y1.x; b.v[5] = y1.y; b.v[6] = y1.z; b.v[7] = y1.w;
-      h = sky_compress(a, b);
+      h = fr_reduce_once(tile.compress<false>(skytc::reduce_any(a), b));
+    } else {
+      tile.sit_out();
     }
     __syncthreads();
     uint8_t* next = level + 32 * level_n;
@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(kSubThreads) merkle_subtree_kernel(uint8_t* __
     __syncthreads();
     level = next;
     level_n /= 2;
-    cnt = half;
   }
+  tile.close(sh);
 }
 
 static int grid_for(size_t n, int threads) {
@@ -205,6 +205,7 @@ int compress_many_device(const uint8_t* in, size_t n, uint8_t* out, cudaStream_t
   if (n == 0) return PKG_OK;
   PK_REQUIRE(in && out, "null pointer");
   PK_REQUIRE(aligned16(in) && aligned16(out), "device buffers must be 16-byte aligned");
+  if (tc_wanted(n, 2)) return fold_tc(ByteMessages{in, 64}, 2, n, out, s);
   compress_many_kernel<<<grid_for(n, 128), 128, 0, s>>>(in, n, out);
   PK_CHECK_LAUNCH("compress_many_kernel");
   return PKG_OK;
@@ -222,34 +223,29 @@ int hash_many_device(size_t size, const uint8_t* in, size_t count, uint8_t* out,
     return PKG_OK;
   }
   if (size == 64) return compress_many_device(in, count, out, s);
-  leaf_fold_kernel<<<grid_for(count, 128), 128, 0, s>>>(in, size, size / 32, count, out);
-  PK_CHECK_LAUNCH("leaf_fold_kernel");
-  return PKG_OK;
+  return fold_tc(ByteMessages{in, size}, size / 32, count, out, s);
 }
 
 // Internal levels above the leaf digests already in layers[0..n) (n a power
 // of two): one launch per level while a level has more than kSubtreeMax
-// nodes, then the subtree kernel's kSubLevels levels, then the top.
+// nodes, then eight levels in subtrees of kSubNodes, until one node is left.
 int merkle_levels_device(uint8_t* layers, size_t n, cudaStream_t s) {
   uint8_t* cur = layers;
   while (n > kSubtreeMax) {
     uint8_t* next = cur + 32 * n;
-    merkle_level_kernel<<<grid_for(n / 2, 128), 128, 0, s>>>(cur, n / 2, next);
-    PK_CHECK_LAUNCH("merkle_level_kernel");
+    const int rc = compress_many_device(cur, n / 2, next, s);
+    if (rc) return rc;
     cur = next;
     n /= 2;
   }
-  if (n >= (size_t)kSubNodes * 2) {
-    merkle_subtree_kernel<<<(unsigned)(n / kSubNodes), kSubThreads, 0, s>>>(cur, n);
+  while (n > 1) {
+    const int nodes = (int)std::min<size_t>(n, kSubNodes);
+    merkle_subtree_kernel<<<(unsigned)(n / nodes), skytc::kThreads, 0, s>>>(cur, n, nodes);
     PK_CHECK_LAUNCH("merkle_subtree_kernel");
-    for (int l = 0; l < kSubLevels; l++) {
+    for (int k = nodes; k > 1; k /= 2) {
       cur += 32 * n;
       n /= 2;
     }
-  }
-  if (n > 1) {
-    merkle_top_kernel<<<1, 512, 0, s>>>(cur, n, cur + 32 * n);
-    PK_CHECK_LAUNCH("merkle_top_kernel");
   }
   return PKG_OK;
 }
@@ -262,6 +258,10 @@ int merkle_leaves_fr_device(const uint64_t* cw, size_t fr_per_leaf, size_t num_l
              "unknown leaf encoding %d", encoding);
   PK_REQUIRE(cw && layers, "null pointer");
   PK_REQUIRE(aligned16(cw) && aligned16(layers), "device buffers must be 16-byte aligned");
+  if (tc_wanted(num_leaves, fr_per_leaf))
+    return encoding == PKG_LEAF_CANONICAL
+               ? fold_tc(CodewordRows<true>{cw, fr_per_leaf}, fr_per_leaf, num_leaves, layers, s)
+               : fold_tc(CodewordRows<false>{cw, fr_per_leaf}, fr_per_leaf, num_leaves, layers, s);
   int g = grid_for(num_leaves, 128);
   if (encoding == PKG_LEAF_CANONICAL)
     leaf_fold_fr_kernel<true><<<g, 128, 0, s>>>(cw, fr_per_leaf, num_leaves, layers);
