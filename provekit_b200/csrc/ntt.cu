@@ -6,7 +6,7 @@
 // 2^t groups; group k pairs element i with i + half and multiplies the odd
 // element by roots[k] from the bit-reversed twiddle table
 // (init_roots_reverse_ordered, ntt/src/ntt.rs:275-306).  Stages are fused into
-// passes of K <= 10 stages: a pass owns independent 2^K-point sub-transforms
+// passes of K <= 8 stages: a pass owns independent 2^K-point sub-transforms
 // ("lines": fixed top t row bits and fixed low row bits), stages each line in
 // shared memory, and runs its K stages there, so global memory is read and
 // written once per pass instead of once per stage.  Exact modular arithmetic
@@ -21,27 +21,7 @@
 #include "ntt_internal.cuh"
 #include "host_stage.cuh"
 #include "pk_common.cuh"
-
-// Most stages per pass (a pass kernel exists for 1..9).  Eight: a 9-stage
-// pass stages 2 x 2^8 x 11 doubles of twiddle digits (45 KiB) besides its
-// 16 KiB tile, which holds it to 3 CTAs per SM; the whole proof's 18-stage
-// witness encode ran 0.39 ms faster per proof as three 6-stage passes than as
-// two 9-stage ones (18.65 vs 19.04 ms), and two 9-stage lines per CTA (512
-// threads, 2 CTAs per SM) gained nothing.
-#ifndef PK_NTT_KMAX
-#define PK_NTT_KMAX 8
-#endif
-// Butterflies per thread per stage, log2 (the CTA has E / 2^(1 + this)
-// threads, at least 32).  Two: 2^24 points in 5.01 ms against 5.14 ms with
-// one (a CTA of 256 elements' worth of 128 threads, each with two
-// independent products in flight per stage); four were slower (5.31 ms).
-#ifndef PK_NTT_LOG_BPT
-#define PK_NTT_LOG_BPT 1
-#endif
-// Elements per CTA, log2 (lines of 2^K elements: 2^(this - K) of them).
-#ifndef PK_NTT_LOG_ELEMS
-#define PK_NTT_LOG_ELEMS 9
-#endif
+#include "tc_reduce.cuh"
 
 namespace pk {
 
@@ -155,6 +135,14 @@ int roots_reserve(size_t order, const uint64_t** out) {
 // the CTA's lines cover a contiguous memory range.
 // Stage s of the pass (global stage t+s) pairs j0 = grp*2h + pos with
 // j0 + h (h = 2^(K-1-s)) and uses twiddle roots[(high << s) | grp].
+//
+// A CTA's 128 threads run a stage's butterflies 128 at a time, their products'
+// reductions on the tensor cores (tc_reduce.cuh): 72 64-bit multiply-adds per
+// product instead of 128.  Values stay below 5 p between stages and passes.
+// Bound by the multiplier and by latency between its phases: 2^24 points take
+// 2.89 ms (the multiplier 62 % busy, DRAM 13 %) against 3.56 ms with the whole
+// product on the integer pipe; with CTAs that stay for several tiles 3.30 ms,
+// since they do not finish together.
 // ---------------------------------------------------------------------------
 // Element g of the RS-encode layout (see NttSource).
 __device__ __forceinline__ Fr source_load(const NttSource& s, uint64_t g) {
@@ -167,39 +155,130 @@ __device__ __forceinline__ Fr source_load(const NttSource& s, uint64_t g) {
   return fr_zero();
 }
 
+__device__ __forceinline__ Fr tile_load(const uint4* sm, int E, int i) {
+  const uint4 a = sm[i], b = sm[E + i];
+  Fr x;
+  x.v[0] = a.x; x.v[1] = a.y; x.v[2] = a.z; x.v[3] = a.w;
+  x.v[4] = b.x; x.v[5] = b.y; x.v[6] = b.z; x.v[7] = b.w;
+  return x;
+}
+__device__ __forceinline__ void tile_store(uint4* sm, int E, int i, const Fr& x) {
+  sm[i] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
+  sm[E + i] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
+}
+// The product where the tensor cores' wait ran out (w < p, x < 5 p).
+static __device__ __noinline__ Fr product_alone(const Fr w, const Fr x) { return fr_mul(w, x); }
+
+// Index of tile element e in the data and in shared memory.
+template <bool kModeB>
+__device__ __forceinline__ void pass_index(int e, int K, int T, int log_t, int log_u, uint64_t U,
+                                           uint64_t l0, uint64_t high, uint64_t u0, uint64_t* g,
+                                           int* sidx) {
+  if (!kModeB) {
+    const int j = e >> log_t, ll = e & (T - 1);
+    *g = ((high << K) + j) * U + u0 + ll;
+    *sidx = e;
+  } else {
+    const int j = (e >> log_u) & ((1 << K) - 1);
+    const int hl = e >> (log_u + K);
+    const int u = e & ((1 << log_u) - 1);
+    *g = (((l0 >> log_u) << K) << log_u) + e;
+    *sidx = j * T + (hl << log_u) + u;
+  }
+}
+
+// x0, m -> x0 + m, x0 - m mod p, loosely: for x0 < 5 p and m < 1.1 p both
+// results are below 5 p (and 2^256).  2 p is taken from the sum when x0 is
+// above it, and added to the difference when it is not (x0 is compared by its
+// top word, so the border is up to 2^224 above 2 p).
+__device__ __forceinline__ void loose_butterfly(const Fr& x0, const Fr& m, Fr& y0, Fr& y1) {
+  asm("{\n\t"
+      ".reg .pred b;\n\t"
+      "setp.ge.u32 b, %23, 0x60c89ce6;\n\t"
+      "add.cc.u32  %0, %16, %24;\n\t"
+      "addc.cc.u32 %1, %17, %25;\n\t"
+      "addc.cc.u32 %2, %18, %26;\n\t"
+      "addc.cc.u32 %3, %19, %27;\n\t"
+      "addc.cc.u32 %4, %20, %28;\n\t"
+      "addc.cc.u32 %5, %21, %29;\n\t"
+      "addc.cc.u32 %6, %22, %30;\n\t"
+      "addc.u32    %7, %23, %31;\n\t"
+      "sub.cc.u32  %8,  %16, %24;\n\t"
+      "subc.cc.u32 %9,  %17, %25;\n\t"
+      "subc.cc.u32 %10, %18, %26;\n\t"
+      "subc.cc.u32 %11, %19, %27;\n\t"
+      "subc.cc.u32 %12, %20, %28;\n\t"
+      "subc.cc.u32 %13, %21, %29;\n\t"
+      "subc.cc.u32 %14, %22, %30;\n\t"
+      "subc.u32    %15, %23, %31;\n\t"
+      "@b sub.cc.u32  %0, %0, 0xe0000002;\n\t"
+      "@b subc.cc.u32 %1, %1, 0x87c3eb27;\n\t"
+      "@b subc.cc.u32 %2, %2, 0xf372e122;\n\t"
+      "@b subc.cc.u32 %3, %3, 0x5067d090;\n\t"
+      "@b subc.cc.u32 %4, %4, 0x0302b0ba;\n\t"
+      "@b subc.cc.u32 %5, %5, 0x70a08b6d;\n\t"
+      "@b subc.cc.u32 %6, %6, 0xc2634053;\n\t"
+      "@b subc.u32    %7, %7, 0x60c89ce5;\n\t"
+      "@!b add.cc.u32  %8,  %8,  0xe0000002;\n\t"
+      "@!b addc.cc.u32 %9,  %9,  0x87c3eb27;\n\t"
+      "@!b addc.cc.u32 %10, %10, 0xf372e122;\n\t"
+      "@!b addc.cc.u32 %11, %11, 0x5067d090;\n\t"
+      "@!b addc.cc.u32 %12, %12, 0x0302b0ba;\n\t"
+      "@!b addc.cc.u32 %13, %13, 0x70a08b6d;\n\t"
+      "@!b addc.cc.u32 %14, %14, 0xc2634053;\n\t"
+      "@!b addc.u32    %15, %15, 0x60c89ce5;\n\t"
+      "}"
+      : "=&r"(y0.v[0]), "=&r"(y0.v[1]), "=&r"(y0.v[2]), "=&r"(y0.v[3]), "=&r"(y0.v[4]),
+        "=&r"(y0.v[5]), "=&r"(y0.v[6]), "=&r"(y0.v[7]), "=&r"(y1.v[0]), "=&r"(y1.v[1]),
+        "=&r"(y1.v[2]), "=&r"(y1.v[3]), "=&r"(y1.v[4]), "=&r"(y1.v[5]), "=&r"(y1.v[6]),
+        "=&r"(y1.v[7])
+      : "r"(x0.v[0]), "r"(x0.v[1]), "r"(x0.v[2]), "r"(x0.v[3]), "r"(x0.v[4]), "r"(x0.v[5]),
+        "r"(x0.v[6]), "r"(x0.v[7]), "r"(m.v[0]), "r"(m.v[1]), "r"(m.v[2]), "r"(m.v[3]),
+        "r"(m.v[4]), "r"(m.v[5]), "r"(m.v[6]), "r"(m.v[7]));
+}
+
+// Most stages per pass: 8.  2^24 points take 2.89 ms as three 8-stage passes,
+// 3.06 as four of 6; 9 (tiles of one line) save a pass at 2^17 and 2^18 points
+// (40.5 against 43.2 us) but cost 5 % at 18 stages over 16 columns of 2^20.
+constexpr int kPassStages = 8;
+// Elements per CTA, log2: two batches of 128 butterflies a stage, or one below
+// 2^21 elements, where the batch's latency counts: 2^19 points 103 us with one
+// and 114 with two, 2^20 185 and 190, 2^22 744 and 699.  Four: 763.
+constexpr int kTileElems = 9, kSmallTileElems = 8;
+constexpr uint64_t kSmallBelow = uint64_t(1) << 21;
+
+struct PassShape {
+  uint64_t U;  // lines per `high`
+  int log_u, T, log_t, K;
+  bool first;      // stage 0 of the pass is stage 0 of the transform: every twiddle is 1
+  bool last;       // store fully reduced; other passes leave values below 5 p
+};
+
 // kModeB selects mode B at compile time.  In mode A every line of the CTA
 // shares `high`, so stage s reads only the 2^s twiddles roots[(high << s) |
 // grp], which stay in L1.
-template <int K, bool kSrc, bool kModeB>
-__global__ void __launch_bounds__(512) ntt_pass_kernel(uint64_t* __restrict__ data,
-                                                      const uint64_t* __restrict__ roots,
-                                                      uint64_t U, int log_u, int T, int log_t,
-                                                      int mode_b_unused, const NttSource src) {
+template <bool kSrc, bool kModeB>
+__global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
+    ntt_pass_kernel(uint64_t* __restrict__ data, const uint64_t* __restrict__ roots,
+                    const PassShape shape, const NttSource src) {
   extern __shared__ uint4 sm[];
-  constexpr int R = 1 << K;
-  constexpr bool mode_b = kModeB;
-  const int E = R * T;
+  __shared__ tc::ProductShared sh;
+  const int K = shape.K, T = shape.T, log_t = shape.log_t, log_u = shape.log_u;
+  const int E = T << K, half = E >> 1;
+  const uint64_t U = shape.U;
+  tc::ProductTile tile;
+  tile.open(sh, tc::kProductImage);
   const uint64_t l0 = (uint64_t)blockIdx.x * T;
   uint64_t high_a = 0, u0 = 0;
-  if (!mode_b) {
+  if (!kModeB) {
     high_a = l0 / U;
     u0 = l0 - high_a * U;
   }
   // ---- load ----
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    if (!mode_b) {
-      int j = e >> log_t, ll = e & (T - 1);
-      g = (high_a * R + j) * U + u0 + ll;
-      sidx = j * T + ll;
-    } else {
-      int j = (e >> log_u) & (R - 1);
-      int hl = e >> (log_u + K);
-      int u = e & ((1 << log_u) - 1);
-      g = (l0 >> log_u) * R * U + e;
-      sidx = j * T + (hl << log_u) + u;
-    }
+    pass_index<kModeB>(e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     if (kSrc) {
       const Fr v = source_load(src, g);
       sm[sidx] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
@@ -215,119 +294,97 @@ __global__ void __launch_bounds__(512) ntt_pass_kernel(uint64_t* __restrict__ da
 #pragma unroll 1
   for (int s = 0; s < K; s++) {
     const int log_h = K - 1 - s;
-    for (int b = threadIdx.x; b < (E >> 1); b += blockDim.x) {
-      int ll = b & (T - 1);
-      int p = b >> log_t;
-      int grp = p >> log_h;
-      int pos = p & ((1 << log_h) - 1);
-      int j0 = (grp << (log_h + 1)) + pos;
-      int j1 = j0 + (1 << log_h);
-      int i0 = j0 * T + ll, i1 = j1 * T + ll;
-      Fr x0, x1;
-      uint4 a = sm[i0], bb = sm[E + i0];
-      x0.v[0] = a.x; x0.v[1] = a.y; x0.v[2] = a.z; x0.v[3] = a.w;
-      x0.v[4] = bb.x; x0.v[5] = bb.y; x0.v[6] = bb.z; x0.v[7] = bb.w;
-      a = sm[i1];
-      bb = sm[E + i1];
-      x1.v[0] = a.x; x1.v[1] = a.y; x1.v[2] = a.z; x1.v[3] = a.w;
-      x1.v[4] = bb.x; x1.v[5] = bb.y; x1.v[6] = bb.z; x1.v[7] = bb.w;
-      const uint64_t high = kModeB ? (l0 + ll) >> log_u : high_a;
-      const Fr m = fr_mul(x1, fr_load_ro(roots, (high << s) | (uint64_t)grp));
-      Fr y0 = fr_add(x0, m);
-      Fr y1 = fr_sub(x0, m);
-      sm[i0] = make_uint4(y0.v[0], y0.v[1], y0.v[2], y0.v[3]);
-      sm[E + i0] = make_uint4(y0.v[4], y0.v[5], y0.v[6], y0.v[7]);
-      sm[i1] = make_uint4(y1.v[0], y1.v[1], y1.v[2], y1.v[3]);
-      sm[E + i1] = make_uint4(y1.v[4], y1.v[5], y1.v[6], y1.v[7]);
+#pragma unroll 1
+    for (int b0 = 0; b0 < half; b0 += tc::kThreads) {
+      const int b = b0 + (int)threadIdx.x;
+      const bool live = b < half;
+      const int bb = live ? b : 0;  // others repeat butterfly 0 and store nothing
+      const int ll = bb & (T - 1);
+      const int pp = bb >> log_t;
+      const int grp = pp >> log_h;
+      const int j0 = (grp << (log_h + 1)) + (pp & ((1 << log_h) - 1));
+      const int i0 = j0 * T + ll, i1 = i0 + (T << log_h);
+      const Fr x1 = tile_load(sm, E, i1);
+      Fr m;
+      if (shape.first && s == 0) {
+        m = fr_reduce_once(x1);
+      } else {
+        const uint64_t high = kModeB ? (l0 + ll) >> log_u : high_a;
+        const Fr w = fr_load_ro(roots, (high << s) | (uint64_t)grp);
+        uint32_t S[9];
+        tile.start(w, x1);
+        tile.finish(S);
+        if (tile.alone)
+          m = product_alone(w, x1);
+        else
+          m = tc::quotient_step(S);
+        __syncwarp();
+      }
+      const Fr x0 = tile_load(sm, E, i0);
+      Fr y0, y1;
+      loose_butterfly(x0, m, y0, y1);
+      if (live) {
+        tile_store(sm, E, i0, y0);
+        tile_store(sm, E, i1, y1);
+      }
     }
     __syncthreads();
   }
   // ---- store ----
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    if (!mode_b) {
-      int j = e >> log_t, ll = e & (T - 1);
-      g = (high_a * R + j) * U + u0 + ll;
-      sidx = j * T + ll;
-    } else {
-      int j = (e >> log_u) & (R - 1);
-      int hl = e >> (log_u + K);
-      int u = e & ((1 << log_u) - 1);
-      g = (l0 >> log_u) * R * U + e;
-      sidx = j * T + (hl << log_u) + u;
-    }
-    uint4* dst = reinterpret_cast<uint4*>(data + 4 * g);
-    dst[0] = sm[sidx];
-    dst[1] = sm[E + sidx];
+    pass_index<kModeB>(e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    Fr v = tile_load(sm, E, sidx);
+    if (shape.last) v = fr_reduce_once(tc::reduce_any(v));
+    fr_store(data, g, v);
   }
-}
-
-typedef void (*PassFn)(uint64_t*, const uint64_t*, uint64_t, int, int, int, int, const NttSource);
-template <bool kSrc, bool kModeB>
-static PassFn pass_fn_t(int k) {
-  switch (k) {
-    case 1: return ntt_pass_kernel<1, kSrc, kModeB>;
-    case 2: return ntt_pass_kernel<2, kSrc, kModeB>;
-    case 3: return ntt_pass_kernel<3, kSrc, kModeB>;
-    case 4: return ntt_pass_kernel<4, kSrc, kModeB>;
-    case 5: return ntt_pass_kernel<5, kSrc, kModeB>;
-    case 6: return ntt_pass_kernel<6, kSrc, kModeB>;
-    case 7: return ntt_pass_kernel<7, kSrc, kModeB>;
-    case 8: return ntt_pass_kernel<8, kSrc, kModeB>;
-    default: return ntt_pass_kernel<9, kSrc, kModeB>;
-  }
-}
-static PassFn pass_fn(int k, bool src, bool mode_b) {
-  if (src) return mode_b ? pass_fn_t<true, true>(k) : pass_fn_t<true, false>(k);
-  return mode_b ? pass_fn_t<false, true>(k) : pass_fn_t<false, false>(k);
+  tile.close();
 }
 
 static inline uint64_t pow2_part(uint64_t x) { return x & (~x + 1); }
 
-// Run global stages [t_begin, t_end) of an N-point transform over M columns.
+// Run global stages [t_begin, t_end) of an N-point transform over M columns;
+// t_end is the last stage.
 int ntt_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end, const uint64_t* roots,
                cudaStream_t stream, const NttSource* src) {
-  const int S = log2_exact(N);
-  (void)S;
-  const int kmax = PK_NTT_KMAX;
-  int total = t_end - t_begin;
+  const int total = t_end - t_begin;
   if (total <= 0) return PKG_OK;
-  int npasses = (total + kmax - 1) / kmax;
+  const int npasses = (total + kPassStages - 1) / kPassStages;
+  const int log_elems = N * M < kSmallBelow ? kSmallTileElems : kTileElems;
   int t = t_begin;
   for (int pi = 0; pi < npasses; pi++) {
-    int K = (total - (t - t_begin) + (npasses - pi) - 1) / (npasses - pi);
-    int B = log2_exact(N) - t - K;
-    uint64_t U = (uint64_t(1) << B) * M;
-    uint64_t num_lines = (uint64_t(1) << t) * U;
-    // aim for 2^PK_NTT_LOG_ELEMS elements per CTA
-    int log_tgt = K >= PK_NTT_LOG_ELEMS ? 0 : PK_NTT_LOG_ELEMS - K;
-    uint64_t T = uint64_t(1) << log_tgt;
+    const int K = (total - (t - t_begin) + (npasses - pi) - 1) / (npasses - pi);
+    const int B = log2_exact(N) - t - K;
+    const uint64_t U = (uint64_t(1) << B) * M;
+    const uint64_t num_lines = (uint64_t(1) << t) * U;
+    uint64_t T = uint64_t(1) << (K >= log_elems ? 0 : log_elems - K);
     if (T > num_lines) T = pow2_part(num_lines);
-    int mode_b = 0;
-    int log_u = 0;
-    if (is_pow2(U) && U < T) {
-      mode_b = 1;
-      log_u = log2_exact(U);
-    } else {
-      uint64_t pu = pow2_part(U);
-      if (T > pu) T = pu;
-    }
-    int log_t = log2_exact(T);
-    uint64_t E = (uint64_t(1) << K) * T;
-    int threads = (int)std::min<uint64_t>((E / 2) >> PK_NTT_LOG_BPT, 512);
-    if (threads < 32) threads = 32;
-    size_t smem = 32 * E;
-    uint64_t grid = num_lines / T;
-    const bool from_src = src != nullptr && pi == 0;
-    PassFn fn = pass_fn(K, from_src, mode_b != 0);
-    if (smem > 48 * 1024) {
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    }
+    const bool mode_b = is_pow2(U) && U < T;
+    if (!mode_b) T = std::min(T, pow2_part(U));
+    PassShape shape;
+    shape.U = U;
+    shape.log_u = mode_b ? log2_exact(U) : 0;
+    shape.T = (int)T;
+    shape.log_t = log2_exact(T);
+    shape.K = K;
+    shape.first = t == 0;
+    shape.last = pi == npasses - 1;
+    const size_t smem = 32 * (T << K);
+    const unsigned grid = (unsigned)(num_lines / T);
     NttSource s;
     memset(&s, 0, sizeof s);
-    if (from_src) s = *src;
-    fn<<<(unsigned)grid, threads, smem, stream>>>(data, roots, U, log_u, (int)T, log_t, mode_b, s);
+    if (src && pi == 0) {
+      s = *src;
+      if (mode_b)
+        ntt_pass_kernel<true, true><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
+      else
+        ntt_pass_kernel<true, false><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
+    } else if (mode_b) {
+      ntt_pass_kernel<false, true><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
+    } else {
+      ntt_pass_kernel<false, false><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
+    }
     PK_CHECK_LAUNCH("ntt_pass_kernel");
     t += K;
   }
