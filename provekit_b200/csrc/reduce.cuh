@@ -1,49 +1,90 @@
 // reduce.cuh -- block-wide sums of field elements and the grid-size helpers
 // shared by the reduction kernels (sumcheck, dot products, WHIR rounds).
 //
-// Each thread accumulates a grid-stride slice; warps combine with
-// __shfl_down_sync (8 limbs per element, field additions), warps combine
-// through shared memory, and one partial per CTA goes to a small scratch
-// array that a single-CTA kernel sums.  Field addition is exact, so the
-// result does not depend on the reduction order.
+// Each thread accumulates a grid-stride slice, a CTA adds its threads' sums,
+// and one partial per CTA goes to a small scratch array that a single CTA
+// sums.  Field addition is exact, so the result does not depend on the
+// reduction order.
 #pragma once
 #include <algorithm>
 
 #include "fr.cuh"
+#include "fr_sum.cuh"
 #include "pk_common.cuh"
 
 namespace pk {
 
 constexpr int kRedThreads = 256;
 
-__device__ __forceinline__ Fr shfl_down(const Fr& x, int off) {
-  Fr r;
-#pragma unroll
-  for (int i = 0; i < 8; i++) r.v[i] = __shfl_down_sync(0xffffffffu, x.v[i], off);
-  return r;
-}
+constexpr int kSumLimbs = 11;  // 24-bit limbs of an element
 
-// Block-wide sum of K field elements per thread; thread 0 gets the result.
+// Block-wide sum of K field elements per thread (at most 256 threads); thread
+// 0 gets the result, fully reduced.  Elements are added as integers, limb by
+// limb: 256 limbs of 24 bits fit 32 bits, so a warp adds each limb with one
+// redux, one warp adds the warps' sums, and the total is reduced once.  Bound
+// by latency: modular additions down a shuffle tree took 5 + 5 dependent
+// levels of 8 shuffles and a 16-step carry chain each.
 template <int K>
 __device__ __forceinline__ void block_sum(Fr (&v)[K]) {
-  __shared__ Fr warp_sums[kRedThreads / 32][K];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = fr_add(v[k], shfl_down(v[k], off));
+  __shared__ uint32_t limbs[kRedThreads / 32][K * kSumLimbs];
+  __shared__ uint32_t total[K * kSumLimbs];
+  __shared__ Fr sums[K];
+  constexpr uint32_t M = 0xffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
 #pragma unroll
-    for (int k = 0; k < K; k++) warp_sums[warp][k] = v[k];
+  for (int k = 0; k < K; k++) {
+    const uint32_t* x = v[k].v;
+    const uint32_t d[kSumLimbs] = {x[0] & M,
+                                   __funnelshift_r(x[0], x[1], 24) & M,
+                                   __funnelshift_r(x[1], x[2], 16) & M,
+                                   x[2] >> 8,
+                                   x[3] & M,
+                                   __funnelshift_r(x[3], x[4], 24) & M,
+                                   __funnelshift_r(x[4], x[5], 16) & M,
+                                   x[5] >> 8,
+                                   x[6] & M,
+                                   __funnelshift_r(x[6], x[7], 24) & M,
+                                   x[7] >> 16};
+#pragma unroll
+    for (int i = 0; i < kSumLimbs; i++) {
+      const uint32_t sum = __reduce_add_sync(0xffffffffu, d[i]);
+      if (lane == 0) limbs[warp][k * kSumLimbs + i] = sum;
+    }
+  }
   __syncthreads();
   if (warp == 0) {
     const int nw = blockDim.x >> 5;
+    for (int i = lane; i < K * kSumLimbs; i += 32) {
+      uint32_t sum = 0;
+      for (int w = 0; w < nw; w++) sum += limbs[w][i];
+      total[i] = sum;
+    }
+    __syncwarp();
+    if (lane < K) {
+      uint32_t d[kSumLimbs + 1], S[9];
+      uint64_t carry = 0;
 #pragma unroll
-    for (int k = 0; k < K; k++) v[k] = lane < nw ? warp_sums[lane][k] : fr_zero();
+      for (int i = 0; i < kSumLimbs; i++) {
+        carry += total[lane * kSumLimbs + i];
+        d[i] = (uint32_t)carry & M;
+        carry >>= 24;
+      }
+      d[kSumLimbs] = (uint32_t)carry;
+      S[0] = d[0] | (d[1] << 24);
+      S[1] = (d[1] >> 8) | (d[2] << 16);
+      S[2] = (d[2] >> 16) | (d[3] << 8);
+      S[3] = d[4] | (d[5] << 24);
+      S[4] = (d[5] >> 8) | (d[6] << 16);
+      S[5] = (d[6] >> 16) | (d[7] << 8);
+      S[6] = d[8] | (d[9] << 24);
+      S[7] = (d[9] >> 8) | (d[10] << 16);
+      S[8] = (d[10] >> 16) | (d[11] << 8);
+      sums[lane] = fr_reduce_once(tc::quotient_step(S));
+    }
+    __syncwarp();
+    if (lane == 0)
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-      for (int k = 0; k < K; k++) v[k] = fr_add(v[k], shfl_down(v[k], off));
+      for (int k = 0; k < K; k++) v[k] = sums[k];
   }
 }
 
@@ -85,31 +126,36 @@ __device__ __forceinline__ void block_finish(Fr (&v)[K], const RedOut& ro,
                                              const Fr* scale = nullptr) {
   __shared__ bool last;
   block_sum<K>(v);
+  const bool alone = ro.ticket && gridDim.x == 1;  // this CTA's sum is the sum
   if (threadIdx.x == 0) {
     if (scale)
 #pragma unroll
       for (int k = 0; k < K; k++) v[k] = fr_mul(v[k], *scale);
+    if (!alone) {
 #pragma unroll
-    for (int k = 0; k < K; k++) fr_store(ro.part, (size_t)blockIdx.x * K + k, v[k]);
-    if (ro.ticket) {
-      __threadfence();
-      last = atomicAdd(ro.ticket, 1u) == gridDim.x - 1;
+      for (int k = 0; k < K; k++) fr_store(ro.part, (size_t)blockIdx.x * K + k, v[k]);
+      if (ro.ticket) {
+        __threadfence();
+        last = atomicAdd(ro.ticket, 1u) == gridDim.x - 1;
+      }
     }
   }
   if (!ro.ticket) return;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
+  if (!alone) {
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
 #pragma unroll
-  for (int k = 0; k < K; k++) v[k] = fr_zero();
-  for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x)
+    for (int k = 0; k < K; k++) v[k] = fr_zero();
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x)
 #pragma unroll
-    for (int k = 0; k < K; k++) v[k] = fr_add(v[k], fr_load_cg(ro.part, (size_t)i * K + k));
-  block_sum<K>(v);
+      for (int k = 0; k < K; k++) v[k] = fr_add(v[k], fr_load_cg(ro.part, (size_t)i * K + k));
+    block_sum<K>(v);
+  }
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < K; k++) fr_store(ro.out, k, v[k]);
-    *ro.ticket = 0u;
+    if (!alone) *ro.ticket = 0u;
     if (ro.seq) {
       volatile unsigned* word = *reinterpret_cast<unsigned* const*>(ro.ticket + 2);
       __threadfence_system();  // the sums before the completion word
