@@ -55,50 +55,6 @@ struct Shared {
   uint32_t tmem;
 };
 
-// a^2 = sum E[i] 2^(32 i) + sum O[i] 2^(32 i) (E: words 0..15, O: words 1..14)
-// for a < 2^255.  Cross products take a doubled right operand: the words of
-// 2a, with f where the row's first word must not bring in the bit below it.
-// Every chain ends on a pair that no earlier one wrote, so no carry is left.
-__device__ __forceinline__ void square_words(const uint32_t* a, uint32_t* E, uint32_t* O) {
-  uint32_t f[8], g[8];
-#pragma unroll
-  for (int j = 1; j < 8; j++) {
-    f[j] = a[j] << 1;
-    g[j] = __funnelshift_l(a[j - 1], a[j], 1);
-  }
-  PK_NEW_PAIR(O, 1, a[0], f[1]);
-  PK_NEW_PAIR(O, 3, a[0], g[3]);
-  PK_NEW_PAIR(O, 5, a[0], g[5]);
-  PK_NEW_PAIR(O, 7, a[0], g[7]);
-  PK_CHAIN4(O, 3, a[1], f[2], a[1], g[4], a[1], g[6], a[2], g[7]);
-  PK_CHAIN4(O, 5, a[2], f[3], a[2], g[5], a[3], g[6], a[4], g[7]);
-  PK_CHAIN4(O, 7, a[3], f[4], a[4], f[5], a[5], f[6], a[6], f[7]);
-  PK_NEW_PAIR(E, 2, a[0], g[2]);
-  PK_NEW_PAIR(E, 4, a[0], g[4]);
-  PK_NEW_PAIR(E, 6, a[0], g[6]);
-  PK_CHAIN3(E, 4, a[1], g[3], a[1], g[5], a[1], g[7]);
-  PK_CHAIN3(E, 6, a[2], g[4], a[2], g[6], a[3], g[7]);
-  PK_CHAIN3(E, 8, a[3], g[5], a[4], g[6], a[5], g[7]);
-  PK_NEW_PAIR(E, 0, a[0], a[0]);
-  asm("mad.lo.cc.u32  %0,  %14, %14, %0;\n\t"
-      "madc.hi.cc.u32 %1,  %14, %14, %1;\n\t"
-      "madc.lo.cc.u32 %2,  %15, %15, %2;\n\t"
-      "madc.hi.cc.u32 %3,  %15, %15, %3;\n\t"
-      "madc.lo.cc.u32 %4,  %16, %16, %4;\n\t"
-      "madc.hi.cc.u32 %5,  %16, %16, %5;\n\t"
-      "madc.lo.cc.u32 %6,  %17, %17, %6;\n\t"
-      "madc.hi.cc.u32 %7,  %17, %17, %7;\n\t"
-      "madc.lo.cc.u32 %8,  %18, %18, %8;\n\t"
-      "madc.hi.cc.u32 %9,  %18, %18, %9;\n\t"
-      "madc.lo.cc.u32 %10, %19, %19, %10;\n\t"
-      "madc.hi.cc.u32 %11, %19, %19, %11;\n\t"
-      "madc.lo.cc.u32 %12, %20, %20, 0;\n\t"
-      "madc.hi.u32    %13, %20, %20, 0;"
-      : "+r"(E[2]), "+r"(E[3]), "+r"(E[4]), "+r"(E[5]), "+r"(E[6]), "+r"(E[7]), "+r"(E[8]),
-        "+r"(E[9]), "+r"(E[10]), "+r"(E[11]), "+r"(E[12]), "+r"(E[13]), "=r"(E[14]), "=r"(E[15])
-      : "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
-}
-
 // t = E + O (words 0..15; the sum fits)
 __device__ __forceinline__ void merge_words(const uint32_t* E, const uint32_t* O, uint32_t* t) {
   t[0] = E[0];

@@ -16,8 +16,8 @@
 // against constants for its own offsets, and so does anything else that has a
 // weight, carries and additive constants among them.  A and D live in tensor
 // memory: thread i writes its bytes to lane i (tcgen05.st) and reads its 32
-// columns back (tcgen05.ld); shared memory holds only the constants.  64
-// columns of tensor memory per CTA:
+// columns back (tcgen05.ld); shared memory holds only the constants.  Columns
+// of tensor memory with one product:
 //     0..31   D
 //     32..47  even accumulator E, words 0..15   (K blocks 0 and 1)
 //     48..61  odd accumulator O, words 1..14    (K blocks 2 and 3)
@@ -32,7 +32,6 @@ namespace tc {
 constexpr int kThreads = 128;      // one MMA tile: 128 elements
 constexpr int kMaxCtas = 8;        // CTAs per SM: 8 x 64 of the 512 columns
 constexpr int kBlockBytes = 1024;  // a K block: 32 columns x 32 bytes
-constexpr uint32_t kColumns = 64;
 
 constexpr uint64_t kP64[4] = {0x43e1f593f0000001ULL, 0x2833e84879b97091ULL, 0xb85045b68181585dULL,
                               0x30644e72e131a029ULL};
@@ -162,6 +161,15 @@ __device__ __forceinline__ void tmem_st16(uint32_t t, const uint32_t* v) {
       "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t t, uint32_t* c) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]),
+        "=r"(c[7])
+      : "r"(t)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t t, uint32_t* c) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
@@ -221,7 +229,8 @@ __device__ __forceinline__ bool elect_lane() {
 
 // The CTA's tensor memory, constants and barrier.  All kThreads threads call
 // every member, together.
-struct Tile {
+template <uint32_t kColumns>
+struct TileOf {
   uint32_t cols;   // the CTA's columns of tensor memory
   uint32_t tmem;   // this warp's lanes of them
   uint32_t warp;
@@ -300,19 +309,76 @@ struct Tile {
           : "memory");
     }
   }
-  // D (+)= A's K block kblock x block of the constants
-  __device__ __forceinline__ void block(int kblock, int image_block) const {
-    mma(cols, cols + 32 + 8 * kblock, image, image_block, kblock > 0);
+  // D at column d (+)= A's K block at column a x block of the constants
+  __device__ __forceinline__ void block(uint32_t d, uint32_t a, int image_block,
+                                        bool accumulate) const {
+    mma(cols + d, cols + a, image, image_block, accumulate);
   }
-  // D's columns; meaningless where the thread is alone.
-  __device__ __forceinline__ void finish(uint32_t* c) {
+  // The MMAs of start() are done, or the thread is alone from here on.
+  __device__ __forceinline__ void join() {
     if (!alone && !wait(phase)) alone = true;
     phase ^= 1;
     __syncwarp();
     tmem_after_sync();
+  }
+};
+
+// 64 columns: D and one product.
+struct Tile : TileOf<64> {
+  // D (+)= A's K block kblock x block of the constants
+  __device__ __forceinline__ void block(int kblock, int image_block) const {
+    TileOf<64>::block(0, 32 + 8 * kblock, image_block, kblock > 0);
+  }
+  // D's columns; meaningless where the thread is alone.
+  __device__ __forceinline__ void finish(uint32_t* c) {
+    join();
     tmem_ld32(tmem, c);  // warp-wide: also where a thread is alone
   }
 };
+
+// a^2 = sum E[i] 2^(32 i) + sum O[i] 2^(32 i) (E: words 0..15, O: words 1..14)
+// for a < 2^255.  Cross products take a doubled right operand: the words of
+// 2a, with f where the row's first word must not bring in the bit below it.
+// Every chain ends on a pair that no earlier one wrote, so no carry is left.
+__device__ __forceinline__ void square_words(const uint32_t* a, uint32_t* E, uint32_t* O) {
+  uint32_t f[8], g[8];
+#pragma unroll
+  for (int j = 1; j < 8; j++) {
+    f[j] = a[j] << 1;
+    g[j] = __funnelshift_l(a[j - 1], a[j], 1);
+  }
+  PK_NEW_PAIR(O, 1, a[0], f[1]);
+  PK_NEW_PAIR(O, 3, a[0], g[3]);
+  PK_NEW_PAIR(O, 5, a[0], g[5]);
+  PK_NEW_PAIR(O, 7, a[0], g[7]);
+  PK_CHAIN4(O, 3, a[1], f[2], a[1], g[4], a[1], g[6], a[2], g[7]);
+  PK_CHAIN4(O, 5, a[2], f[3], a[2], g[5], a[3], g[6], a[4], g[7]);
+  PK_CHAIN4(O, 7, a[3], f[4], a[4], f[5], a[5], f[6], a[6], f[7]);
+  PK_NEW_PAIR(E, 2, a[0], g[2]);
+  PK_NEW_PAIR(E, 4, a[0], g[4]);
+  PK_NEW_PAIR(E, 6, a[0], g[6]);
+  PK_CHAIN3(E, 4, a[1], g[3], a[1], g[5], a[1], g[7]);
+  PK_CHAIN3(E, 6, a[2], g[4], a[2], g[6], a[3], g[7]);
+  PK_CHAIN3(E, 8, a[3], g[5], a[4], g[6], a[5], g[7]);
+  PK_NEW_PAIR(E, 0, a[0], a[0]);
+  asm("mad.lo.cc.u32  %0,  %14, %14, %0;\n\t"
+      "madc.hi.cc.u32 %1,  %14, %14, %1;\n\t"
+      "madc.lo.cc.u32 %2,  %15, %15, %2;\n\t"
+      "madc.hi.cc.u32 %3,  %15, %15, %3;\n\t"
+      "madc.lo.cc.u32 %4,  %16, %16, %4;\n\t"
+      "madc.hi.cc.u32 %5,  %16, %16, %5;\n\t"
+      "madc.lo.cc.u32 %6,  %17, %17, %6;\n\t"
+      "madc.hi.cc.u32 %7,  %17, %17, %7;\n\t"
+      "madc.lo.cc.u32 %8,  %18, %18, %8;\n\t"
+      "madc.hi.cc.u32 %9,  %18, %18, %9;\n\t"
+      "madc.lo.cc.u32 %10, %19, %19, %10;\n\t"
+      "madc.hi.cc.u32 %11, %19, %19, %11;\n\t"
+      "madc.lo.cc.u32 %12, %20, %20, 0;\n\t"
+      "madc.hi.u32    %13, %20, %20, 0;"
+      : "+r"(E[2]), "+r"(E[3]), "+r"(E[4]), "+r"(E[5]), "+r"(E[6]), "+r"(E[7]), "+r"(E[8]),
+        "+r"(E[9]), "+r"(E[10]), "+r"(E[11]), "+r"(E[12]), "+r"(E[13]), "=r"(E[14]), "=r"(E[15])
+      : "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
+}
 
 // a b = sum E[i] 2^(32 i) + sum O[i] 2^(32 i) + sum C[i] 2^(32 (9 + i)) for any
 // 256-bit a, b; E: words 0..15, O: words 1..14, C: seven carries, one a byte.
@@ -360,6 +426,25 @@ constexpr Image<kProductBlocks> make_product_image() {
 }
 static __device__ const Image<kProductBlocks> kProductImage = make_product_image();
 
+// The words of a square or a product to tensor memory, at the columns of A.
+__device__ __forceinline__ void put_square(uint32_t A, const Fr& x) {
+  uint32_t E[16], O[16];
+  square_words(x.v, E, O);
+  tmem_st8(A + 16, O + 1);
+  tmem_st4(A + 24, O + 9);
+  tmem_st2(A + 28, O + 13);
+  tmem_st16(A, E);
+}
+__device__ __forceinline__ void put_product(uint32_t A, const Fr& a, const Fr& b) {
+  uint32_t E[16], O[16], t[8];
+  product_words(a.v, b.v, E, O, t + 6);
+#pragma unroll
+  for (int i = 0; i < 6; i++) t[i] = O[9 + i];
+  tmem_st8(A + 16, O + 1);
+  tmem_st16(A, E);
+  tmem_st8(A + 24, t);
+}
+
 struct ProductShared {
   alignas(128) uint4 image[kProductBlocks * kBlockBytes / 16];
   alignas(8) uint64_t mbar;
@@ -371,13 +456,7 @@ struct ProductShared {
 // S = a b 2^-256 mod p; a < p, b < 2^256.
 struct ProductTile : Tile {
   __device__ __forceinline__ void start(const Fr& a, const Fr& b) {
-    uint32_t E[16], O[16], t[8];
-    product_words(a.v, b.v, E, O, t + 6);
-#pragma unroll
-    for (int i = 0; i < 6; i++) t[i] = O[9 + i];
-    tmem_st8(tmem + 48, O + 1);
-    tmem_st16(tmem + 32, E);
-    tmem_st8(tmem + 56, t);
+    put_product(tmem + 32, a, b);
     Tile::start([&] {
       block(0, 0);
       block(1, 1);
