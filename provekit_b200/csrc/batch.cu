@@ -23,7 +23,9 @@
 #include "fr.cuh"
 #include "fr_host.hpp"
 #include "ntt_internal.cuh"
+#include "ntt_tile.cuh"
 #include "pk_common.cuh"
+#include "sky_tc.cuh"
 #include "skyscraper.cuh"
 #include "sumcheck_device.cuh"
 
@@ -39,13 +41,14 @@ struct PassDesc {  // one job's share of one grouped NTT pass
   uint64_t* data;
   uint64_t U;
   uint64_t cta_begin;
-  uint32_t log_u, K, T, log_t, mode_b, pad;
+  uint32_t log_u, K, T, log_t, mode_b;
+  uint32_t first, last;  // the pass with the transform's stage 0, with its last stage
   // Where a job's first pass reads its input: 0 = data itself, 1 = src (the
   // coefficients, same indices), 2 = src through the RS-encode layout of
   // kMsgs messages of src_n / kMsgs (the transpose and 4-coset replication).
   const uint64_t* src;
   uint64_t src_n;
-  uint32_t src_kind, pad2;
+  uint32_t src_kind;
 };
 
 struct RangeDesc {  // job j owns [begin, begin + count) of a grouped launch
@@ -83,50 +86,30 @@ __device__ __forceinline__ uint32_t find_desc(const uint64_t* begins, uint32_t n
   return lo;
 }
 
-// Shared memory as two planes of 16-byte halves (see ntt_pass_kernel).
-__device__ __forceinline__ Fr sm_get(const uint4* sm, int E, int i) {
-  uint4 a = sm[i], b = sm[E + i];
-  Fr x;
-  x.v[0] = a.x; x.v[1] = a.y; x.v[2] = a.z; x.v[3] = a.w;
-  x.v[4] = b.x; x.v[5] = b.y; x.v[6] = b.z; x.v[7] = b.w;
-  return x;
-}
-__device__ __forceinline__ void sm_put(uint4* sm, int E, int i, const Fr& x) {
-  sm[i] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-  sm[E + i] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
-}
-
-// ---- grouped NTT pass: the ntt_pass_kernel index scheme with run-time K ----
-__global__ void __launch_bounds__(512) batch_ntt_pass_kernel(const PassDesc* __restrict__ descs,
-                                                            const uint64_t* __restrict__ begins,
-                                                            uint32_t ndesc,
-                                                            const uint64_t* __restrict__ roots) {
+// ---- grouped NTT pass: ntt_pass_kernel with every job's own shape ---------
+__global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
+    batch_ntt_pass_kernel(const PassDesc* __restrict__ descs, const uint64_t* __restrict__ begins,
+                          uint32_t ndesc, const uint64_t* __restrict__ roots) {
   extern __shared__ uint4 sm[];
-  const PassDesc d = descs[find_desc(begins, ndesc, blockIdx.x)];
-  const int K = (int)d.K, R = 1 << K, T = (int)d.T, log_t = (int)d.log_t, log_u = (int)d.log_u;
-  const int E = R * T;
+  __shared__ tc::ProductShared sh;
+  tc::ProductTile tile;
+  tile.open(sh, tc::kProductImage);
+  const PassDesc& d = descs[find_desc(begins, ndesc, blockIdx.x)];
+  const int K = (int)d.K, T = (int)d.T, log_t = (int)d.log_t, log_u = (int)d.log_u;
+  const int E = T << K;
+  const bool mode_b = d.mode_b != 0;
   const uint64_t U = d.U;
   const uint64_t l0 = (uint64_t)(blockIdx.x - d.cta_begin) * T;
   uint64_t high_a = 0, u0 = 0;
-  if (!d.mode_b) {
+  if (!mode_b) {
     high_a = l0 / U;
     u0 = l0 - high_a * U;
   }
   uint64_t* data = d.data;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    if (!d.mode_b) {
-      int j = e >> log_t, ll = e & (T - 1);
-      g = (high_a * R + j) * U + u0 + ll;
-      sidx = j * T + ll;
-    } else {
-      int j = (e >> log_u) & (R - 1);
-      int hl = e >> (log_u + K);
-      int u = e & ((1 << log_u) - 1);
-      g = (l0 >> log_u) * R * U + e;
-      sidx = j * T + (hl << log_u) + u;
-    }
+    pass_index(mode_b, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     const uint4* in;
     if (d.src_kind == 0) {
       in = reinterpret_cast<const uint4*>(data + 4 * g);
@@ -140,43 +123,17 @@ __global__ void __launch_bounds__(512) batch_ntt_pass_kernel(const PassDesc* __r
     sm[E + sidx] = in[1];  // high 16 bytes: plane 1
   }
   __syncthreads();
-  for (int s = 0; s < K; s++) {
-    const int log_h = K - 1 - s;
-    for (int b = threadIdx.x; b < (E >> 1); b += blockDim.x) {
-      int ll = b & (T - 1);
-      int p = b >> log_t;
-      int grp = p >> log_h;
-      int pos = p & ((1 << log_h) - 1);
-      int j0 = (grp << (log_h + 1)) + pos;
-      int j1 = j0 + (1 << log_h);
-      uint64_t high = d.mode_b ? ((l0 + ll) >> log_u) : high_a;
-      Fr tw = fr_load_ro(roots, (high << s) | (uint64_t)grp);
-      int i0 = j0 * T + ll, i1 = j1 * T + ll;
-      Fr x0 = sm_get(sm, E, i0), x1 = sm_get(sm, E, i1);
-      Fr m = fr_mul(tw, x1);
-      sm_put(sm, E, i0, fr_add(x0, m));
-      sm_put(sm, E, i1, fr_sub(x0, m));
-    }
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  tile_stages(tile, sm, mode_b, K, T, log_t, log_u, l0, high_a, d.first != 0, roots);
+  const bool last = d.last != 0;
+  for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    if (!d.mode_b) {
-      int j = e >> log_t, ll = e & (T - 1);
-      g = (high_a * R + j) * U + u0 + ll;
-      sidx = j * T + ll;
-    } else {
-      int j = (e >> log_u) & (R - 1);
-      int hl = e >> (log_u + K);
-      int u = e & ((1 << log_u) - 1);
-      g = (l0 >> log_u) * R * U + e;
-      sidx = j * T + (hl << log_u) + u;
-    }
-    uint4* dst = reinterpret_cast<uint4*>(data + 4 * g);
-    dst[0] = sm[sidx];
-    dst[1] = sm[E + sidx];
+    pass_index(mode_b, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    Fr v = tile_load(sm, E, sidx);
+    if (last) v = fr_reduce_once(tc::reduce_any(v));
+    fr_store(data, g, v);
   }
+  tile.close();
 }
 
 // ---- grouped element-wise phases ------------------------------------------
@@ -191,19 +148,24 @@ __global__ void batch_copy_kernel(const RangeDesc* __restrict__ rd, const uint64
   }
 }
 
-// Merkle leaves: leaf i = codeword row i (8 Fr), canonical encoding.
-__global__ void batch_leaves_kernel(const RangeDesc* __restrict__ rd,
-                                    const uint64_t* __restrict__ begins, uint32_t nd,
-                                    uint64_t total) {
-  for (uint64_t o = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; o < total;
-       o += (uint64_t)gridDim.x * blockDim.x) {
-    const RangeDesc d = rd[find_desc(begins, nd, o)];
-    const uint64_t i = o - d.begin;
-    Fr acc = fr_from_mont(fr_load_ro(d.in, i * kMsgs));
+// Merkle leaves: leaf i = codeword row i (8 Fr), canonical encoding; one tile
+// of 128 leaves per CTA (see fold_tc_kernel).
+__global__ void __launch_bounds__(skytc::kThreads, skytc::kMinCtas)
+    batch_leaves_kernel(const RangeDesc* __restrict__ rd, const uint64_t* __restrict__ begins,
+                        uint32_t nd, uint64_t total) {
+  __shared__ skytc::Shared sh;
+  skytc::SkyTile tile;
+  tile.open(sh);
+  const uint64_t o = (uint64_t)blockIdx.x * skytc::kThreads + threadIdx.x;
+  const uint64_t at = o < total ? o : total - 1;
+  const RangeDesc& d = rd[find_desc(begins, nd, at)];
+  const uint64_t* row = d.in + 4 * kMsgs * (at - d.begin);
+  Fr acc = fr_from_mont(fr_load_ro(row, 0));
 #pragma unroll 1
-    for (int k = 1; k < kMsgs; k++) acc = sky_compress(acc, fr_from_mont(fr_load_ro(d.in, i * kMsgs + k)));
-    fr_store(reinterpret_cast<uint64_t*>(d.out), i, acc);
-  }
+  for (int k = 1; k < kMsgs; k++) acc = tile.compress<true>(acc, fr_load_ro(row, k));
+  if (o < total)
+    fr_store(reinterpret_cast<uint64_t*>(d.out), at - d.begin, fr_reduce_once(acc));
+  tile.close();
 }
 
 // One tree level for every job that still has one: out[i] = compress(in[2i], in[2i+1]).
@@ -217,25 +179,107 @@ __global__ void batch_level_kernel(const RangeDesc* __restrict__ rd,
     fr_store(reinterpret_cast<uint64_t*>(d.out), i, sky_compress(l, r));
   }
 }
+// The same in tiles, for levels wide enough to pay for them.
+__global__ void __launch_bounds__(skytc::kThreads, skytc::kMinCtas)
+    batch_level_tc_kernel(const RangeDesc* __restrict__ rd, const uint64_t* __restrict__ begins,
+                          uint32_t nd, uint64_t total) {
+  __shared__ skytc::Shared sh;
+  skytc::SkyTile tile;
+  tile.open(sh);
+  const uint64_t o = (uint64_t)blockIdx.x * skytc::kThreads + threadIdx.x;
+  const uint64_t at = o < total ? o : total - 1;
+  const RangeDesc& d = rd[find_desc(begins, nd, at)];
+  const uint64_t i = at - d.begin;
+  const Fr h = tile.compress<false>(fr_load_ro(d.in, 2 * i), fr_load_ro(d.in, 2 * i + 1));
+  if (o < total) fr_store(reinterpret_cast<uint64_t*>(d.out), i, fr_reduce_once(h));
+  tile.close();
+}
 
 // ---- device sumcheck ------------------------------------------------------
+// The transcript kernels take four jobs per CTA: a warp each for the round's
+// arithmetic, whose sums and products run across its lanes, then all four
+// transcripts in one tile (sky_tc.cuh) in the first warp, a lane each.  One
+// thread per job took 122 us a round: 5 permutations of 8 us and up to 30
+// cubics one after the other.
+constexpr int kScJobs = 4;
+
+struct ScShared {
+  skytc::Shared tile;
+  Fr scratch[kScJobs][6];
+  Fr cf[kScJobs][4];    // a round polynomial, or in [0] a value to absorb
+  Fr can[kScJobs][4];   // the same in canonical form
+};
+
+// Job of this thread in the tile phase (lanes past the CTA's jobs repeat them;
+// only those with live() store).
+struct ScLane {
+  uint32_t job;
+  bool live;
+};
+__device__ __forceinline__ ScLane sc_lane(uint32_t njobs) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t j = blockIdx.x * kScJobs + (lane & (kScJobs - 1));
+  return {j < njobs ? j : njobs - 1, lane < kScJobs && j < njobs};
+}
+
+// l += x (x canonical), then the permutation: a transcript absorbing x
+__device__ __forceinline__ void sc_absorb(skytc::SkyTile& tile, Fr& l, Fr& r, const Fr& x) {
+  l = fr_add_raw(l, x.v);
+  tile.permute(l, r);
+}
+
 // Start: transcript init, r challenges, eq half tables, sum_g, rho.
-__global__ void batch_sc_start_kernel(ScState* __restrict__ st, const JobDev* __restrict__ jobs,
-                                      uint32_t njobs) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njobs) return;
-  ScState& s = st[j];
-  DevTranscript t;
-  t.init(s.domain);
-  for (uint32_t i = 0; i < s.m0; i++) s.r[i] = t.squeeze();  // whir_r1cs.rs:529
-  Fr g0[4];
-  dev_blinding_coeffs(&s.g[0][0], (int)s.m0, 0, s.alpha, g0);
-  s.sum_g = fr_add(dev_cubic(g0, fr_zero()), dev_cubic(g0, fr_one_mont()));
-  t.absorb(s.sum_g);   // :541
-  s.rho = t.squeeze();  // :543
-  s.saved = fr_mul(s.rho, s.sum_g);
-  s.tl = t.l;
-  s.tr = t.r;
+__global__ void __launch_bounds__(skytc::kThreads)
+    batch_sc_start_kernel(ScState* __restrict__ st, uint32_t njobs) {
+  __shared__ ScShared sh;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t j = blockIdx.x * kScJobs + warp;
+  skytc::SkyTile tile;
+  tile.open(sh.tile);
+  if (j < njobs) {
+    ScState& s = st[j];
+    Fr g0[4];
+    warp_blinding_coeffs(&s.g[0][0], (int)s.m0, 0, s.alpha, (int)lane, sh.scratch[warp], g0);
+    const Fr sum_g = fr_add(fr_add(fr_add(g0[0], g0[0]), g0[1]), fr_add(g0[2], g0[3]));
+    if (lane == 0) {
+      s.sum_g = sum_g;
+      sh.cf[warp][0] = sum_g;
+      sh.can[warp][0] = fr_from_mont(sum_g);
+    }
+  }
+  uint32_t most = 0;
+  for (uint32_t k = 0; k < kScJobs; k++)
+    if (blockIdx.x * kScJobs + k < njobs) most = max(most, st[blockIdx.x * kScJobs + k].m0);
+  __syncthreads();
+  if (tile.warp == 0) {
+    const ScLane me = sc_lane(njobs);
+    ScState& s = st[me.job];
+    const uint32_t q = lane & (kScJobs - 1), m0 = s.m0;
+    Fr l = s.domain, r = fr_zero();
+    tile.permute(l, r);
+    for (uint32_t i = 0; i < most; i++) {
+      Fr nl = l, nr = r;
+      tile.permute(nl, nr);
+      if (i < m0) {
+        l = nl;
+        r = nr;
+        if (me.live) s.r[i] = fr_to_mont(fr_reduce_once(l));  // whir_r1cs.rs:529
+      }
+      __syncwarp();
+    }
+    sc_absorb(tile, l, r, sh.can[q][0]);  // :541
+    tile.permute(l, r);
+    if (me.live) {
+      s.rho = fr_to_mont(fr_reduce_once(l));  // :543
+      s.saved = fr_mul(s.rho, sh.cf[q][0]);
+      s.tl = fr_reduce_once(l);
+      s.tr = fr_reduce_once(r);
+    }
+    __syncwarp();
+  } else {
+    for (uint32_t i = 0; i < most + 3; i++) tile.sit_out();
+  }
+  tile.close();
 }
 
 // eq half tables: hi over r[0..nhi), lo over r[nhi..m0) (same split as
@@ -325,61 +369,106 @@ __global__ void __launch_bounds__(kScThreads) batch_sc_round_kernel(
 // Round bookkeeping for every job still running: sum the CTA partials, build
 // the round polynomial with the blinding terms (whir_r1cs.rs:567-609), absorb
 // it and squeeze alpha.
-__global__ void batch_sc_finish_round_kernel(ScState* __restrict__ st,
-                                             const JobDev* __restrict__ jobs, uint32_t njobs,
-                                             uint32_t round, const uint32_t* __restrict__ nctas) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njobs) return;
-  ScState& s = st[j];
-  if (round >= s.m0) return;
-  const JobDev& jb = jobs[j];
-  Fr h[3] = {fr_zero(), fr_zero(), fr_zero()};
-  for (uint32_t c = 0; c < nctas[j]; c++)
+__global__ void __launch_bounds__(skytc::kThreads)
+    batch_sc_finish_round_kernel(ScState* __restrict__ st, const JobDev* __restrict__ jobs,
+                                 uint32_t njobs, uint32_t round,
+                                 const uint32_t* __restrict__ nctas) {
+  __shared__ ScShared sh;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t j = blockIdx.x * kScJobs + warp;
+  bool any = false;
+  for (uint32_t k = 0; k < kScJobs; k++)
+    if (blockIdx.x * kScJobs + k < njobs) any |= round < st[blockIdx.x * kScJobs + k].m0;
+  if (!any) return;
+  skytc::SkyTile tile;
+  tile.open(sh.tile);
+  if (j < njobs && round < st[j].m0) {
+    ScState& s = st[j];
+    const JobDev& jb = jobs[j];
+    Fr h[3] = {fr_zero(), fr_zero(), fr_zero()};
+    for (uint32_t c = lane; c < nctas[j]; c += 32)
 #pragma unroll
-    for (int k = 0; k < 3; k++) h[k] = fr_add(h[k], fr_load(jb.part, (uint64_t)c * 3 + k));
-  Fr gp[4];
-  dev_blinding_coeffs(&s.g[0][0], (int)s.m0, (int)round, s.alpha, gp);
-  Fr cf[4];
-  cf[0] = fr_add(h[0], fr_mul(s.rho, gp[0]));
-  Fr gem1 = fr_sub(fr_add(fr_sub(gp[0], gp[1]), gp[2]), gp[3]);
-  Fr cem1 = fr_add(h[1], fr_mul(s.rho, gem1));
-  cf[2] = fr_mul(fr_half_mont(), fr_sub(fr_sub(fr_sub(fr_add(s.saved, cem1), cf[0]), cf[0]), cf[0]));
-  cf[3] = fr_add(h[2], fr_mul(s.rho, gp[3]));
-  cf[1] = fr_sub(fr_sub(fr_sub(fr_sub(s.saved, cf[0]), cf[0]), cf[3]), cf[2]);
-  DevTranscript t;
-  t.l = s.tl;
-  t.r = s.tr;
-#pragma unroll 1
-  for (int k = 0; k < 4; k++) {
-    s.coeffs[round][k] = cf[k];
-    t.absorb(cf[k]);
+      for (int k = 0; k < 3; k++) h[k] = fr_add(h[k], fr_load(jb.part, (uint64_t)c * 3 + k));
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; k++) h[k] = warp_sum(h[k]);
+    Fr gp[4];
+    warp_blinding_coeffs(&s.g[0][0], (int)s.m0, (int)round, s.alpha, (int)lane, sh.scratch[warp],
+                         gp);
+    const Fr gem1 = fr_sub(fr_add(fr_sub(gp[0], gp[1]), gp[2]), gp[3]);
+    // rho times the blinding polynomial at 0, at -1 and its leading term
+    if (lane < 3) sh.scratch[warp][lane] = fr_mul(s.rho, lane == 0 ? gp[0] : (lane == 1 ? gem1 : gp[3]));
+    __syncwarp();
+    Fr cf[4];
+    const Fr saved = s.saved, cem1 = fr_add(h[1], sh.scratch[warp][1]);
+    cf[0] = fr_add(h[0], sh.scratch[warp][0]);
+    cf[2] = fr_mul(fr_half_mont(), fr_sub(fr_sub(fr_sub(fr_add(saved, cem1), cf[0]), cf[0]), cf[0]));
+    cf[3] = fr_add(h[2], sh.scratch[warp][2]);
+    cf[1] = fr_sub(fr_sub(fr_sub(fr_sub(saved, cf[0]), cf[0]), cf[3]), cf[2]);
+    if (lane < 4) {
+      const Fr c = lane == 0 ? cf[0] : (lane == 1 ? cf[1] : (lane == 2 ? cf[2] : cf[3]));
+      s.coeffs[round][lane] = c;
+      sh.cf[warp][lane] = c;
+      sh.can[warp][lane] = fr_from_mont(c);
+    }
   }
-  s.alpha[round] = t.squeeze();
-  s.saved = dev_cubic(cf, s.alpha[round]);
-  s.tl = t.l;
-  s.tr = t.r;
+  __syncthreads();
+  if (tile.warp == 0) {
+    const ScLane me = sc_lane(njobs);
+    ScState& s = st[me.job];
+    const uint32_t q = lane & (kScJobs - 1);
+    Fr l = s.tl, r = s.tr;
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) sc_absorb(tile, l, r, sh.can[q][k]);
+    tile.permute(l, r);
+    if (me.live && round < s.m0) {
+      const Fr alpha = fr_to_mont(fr_reduce_once(l));
+      s.alpha[round] = alpha;
+      s.saved = dev_cubic(sh.cf[q], alpha);
+      s.tl = fr_reduce_once(l);
+      s.tr = fr_reduce_once(r);
+    }
+    __syncwarp();
+  } else {
+    for (int k = 0; k < 5; k++) tile.sit_out();
+  }
+  tile.close();
 }
 
 // blinding_eval = <expand_powers::<4>(alpha), w1[offset..]> (whir_r1cs.rs:613-618), absorbed.
-__global__ void batch_sc_end_kernel(ScState* __restrict__ st, uint32_t njobs) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njobs) return;
-  ScState& s = st[j];
-  Fr acc = fr_zero();
-  for (uint32_t i = 0; i < s.m0; i++) {
-    Fr pw = fr_one_mont();
-    for (int k = 0; k < 4; k++) {
-      acc = fr_add(acc, fr_mul(pw, s.wb[i][k]));
-      pw = fr_mul(pw, s.alpha[i]);
+__global__ void __launch_bounds__(skytc::kThreads)
+    batch_sc_end_kernel(ScState* __restrict__ st, uint32_t njobs) {
+  __shared__ ScShared sh;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t j = blockIdx.x * kScJobs + warp;
+  skytc::SkyTile tile;
+  tile.open(sh.tile);
+  if (j < njobs) {
+    ScState& s = st[j];
+    Fr acc = fr_zero();
+    if (lane < s.m0) acc = dev_cubic(s.wb[lane], s.alpha[lane]);
+    __syncwarp();
+    acc = warp_sum(acc);
+    if (lane == 0) {
+      s.blinding_eval = acc;
+      sh.can[warp][0] = fr_from_mont(acc);
     }
   }
-  s.blinding_eval = acc;
-  DevTranscript t;
-  t.l = s.tl;
-  t.r = s.tr;
-  t.absorb(acc);
-  s.tl = t.l;
-  s.tr = t.r;
+  __syncthreads();
+  if (tile.warp == 0) {
+    const ScLane me = sc_lane(njobs);
+    ScState& s = st[me.job];
+    Fr l = s.tl, r = s.tr;
+    sc_absorb(tile, l, r, sh.can[lane & (kScJobs - 1)][0]);
+    if (me.live) {
+      s.tl = fr_reduce_once(l);
+      s.tr = fr_reduce_once(r);
+    }
+    __syncwarp();
+  } else {
+    tile.sit_out();
+  }
+  tile.close();
 }
 
 // ---------------------------------------------------------------------------
@@ -395,7 +484,6 @@ struct Grouped {  // one grouped launch: descriptor arrays on the device
 struct PassLaunch {
   uint32_t n = 0;
   uint64_t ctas = 0;
-  int threads = 32;
   size_t smem = 0;
   PassDesc* d_desc = nullptr;
   uint64_t* d_begin = nullptr;
@@ -416,18 +504,16 @@ struct pkg_batch {
   uint8_t* tables = nullptr;     // descriptor tables (rebuilt by plan())
   size_t tables_bytes = 0;
   const uint64_t* roots = nullptr;
-  // the autotuner's choice on a mix of 256 jobs of 2^10..2^22 points as the default plan:
-  // radix 2^10, 1024 elements per CTA, 4 butterflies per thread per stage
-  // (492.6 ms per batch, against 503 ms with radix 2^8, 256 elements and one
-  // butterfly per thread)
-  int kmax = 10, log_elems = 10;
-  int log_bpt = 2;  // log2 butterflies per thread per stage (CTA size E / 2^(1 + log_bpt))
+  int kmax = 8, log_elems = 9;
+  int log_bpt = 2;  // kept and reported; the passes' CTAs have 128 threads
   // plan
   std::vector<pk::PassLaunch> passes;
   pk::Grouped leaves, eq_half, eq_comb, copy_sc;
   std::vector<pk::Grouped> levels, rounds;
   std::vector<uint64_t> round_ctas;
   uint32_t max_m0 = 0;
+  cudaStream_t side = nullptr;  // the sumchecks' stream
+  cudaEvent_t forked = nullptr, joined = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -468,11 +554,11 @@ static void plan_passes(size_t N, size_t M, int t_begin, int t_end, int kmax, in
     d.T = (uint32_t)T;
     d.log_t = (uint32_t)log2_exact(T);
     d.mode_b = mode_b;
-    d.pad = 0;
+    d.first = t == 0;
+    d.last = pi == np - 1;
     d.src = pi == 0 ? src : nullptr;
     d.src_n = src_n;
     d.src_kind = pi == 0 ? src_kind : 0;
-    d.pad2 = 0;
     if ((int)out.size() <= pi) out.resize(pi + 1);
     out[pi].push_back(d);
     t += K;
@@ -579,8 +665,6 @@ static int batch_plan(pkg_batch* b) {
       maxe = std::max<uint64_t>(maxe, (uint64_t(1) << p[i].K) * p[i].T);
     }
     pl.ctas = acc;
-    pl.threads =
-        (int)std::max<uint64_t>(32, std::min<uint64_t>((maxe / 2) >> b->log_bpt, 512));
     pl.smem = 32 * maxe;
     pl.d_desc = reinterpret_cast<PassDesc*>(cur);
     cur += align256(sizeof(PassDesc) * p.size());
@@ -609,36 +693,33 @@ static int ew_blocks(uint64_t total) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(g, (uint64_t)sm_count() * 32));
 }
 
-// Enqueue the whole batch on s.
-static int batch_enqueue(pkg_batch* b, cudaStream_t s) {
-  const uint32_t nj = (uint32_t)b->jobs.size();
-  PK_CUDA(cudaMemcpyAsync(b->d_state, b->d_state_init, sizeof(ScState) * nj,
-                          cudaMemcpyDeviceToDevice, s));
-  for (auto& p : b->passes) {
-    if (p.smem > 48 * 1024)
-      PK_CUDA(cudaFuncSetAttribute(batch_ntt_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)p.smem));
-    batch_ntt_pass_kernel<<<(unsigned)p.ctas, p.threads, p.smem, s>>>(p.d_desc, p.d_begin, p.n,
-                                                                     b->roots);
-    PK_CHECK_LAUNCH("batch_ntt_pass_kernel");
-  }
-  batch_leaves_kernel<<<(int)std::max<uint64_t>(1, std::min<uint64_t>((b->leaves.total + 127) / 128,
-                                                                     (uint64_t)sm_count() * 64)),
-                        128, 0, s>>>(b->leaves.d_desc, b->leaves.d_begin, b->leaves.n,
-                                     b->leaves.total);
+static unsigned tiles_of(uint64_t n) { return (unsigned)((n + 127) / 128); }
+
+// Leaves and tree levels of every job.
+static int enqueue_trees(pkg_batch* b, cudaStream_t s) {
+  batch_leaves_kernel<<<tiles_of(b->leaves.total), skytc::kThreads, 0, s>>>(
+      b->leaves.d_desc, b->leaves.d_begin, b->leaves.n, b->leaves.total);
   PK_CHECK_LAUNCH("batch_leaves_kernel");
   for (auto& l : b->levels) {
-    batch_level_kernel<<<(int)std::max<uint64_t>(1, std::min<uint64_t>((l.total + 127) / 128,
-                                                                      (uint64_t)sm_count() * 64)),
-                         128, 0, s>>>(l.d_desc, l.d_begin, l.n, l.total);
-    PK_CHECK_LAUNCH("batch_level_kernel");
+    if (l.total > (uint64_t(1) << 15)) {  // the line between the two forms of skyscraper.cu
+      batch_level_tc_kernel<<<tiles_of(l.total), skytc::kThreads, 0, s>>>(l.d_desc, l.d_begin, l.n,
+                                                                         l.total);
+      PK_CHECK_LAUNCH("batch_level_tc_kernel");
+    } else {
+      batch_level_kernel<<<tiles_of(l.total), 128, 0, s>>>(l.d_desc, l.d_begin, l.n, l.total);
+      PK_CHECK_LAUNCH("batch_level_kernel");
+    }
   }
-  // sumcheck
+  return PKG_OK;
+}
+
+static int enqueue_sumchecks(pkg_batch* b, cudaStream_t s) {
+  const uint32_t nj = (uint32_t)b->jobs.size();
   batch_copy_kernel<<<ew_blocks(b->copy_sc.total), 256, 0, s>>>(b->copy_sc.d_desc, b->copy_sc.d_begin,
                                                                 b->copy_sc.n, b->copy_sc.total);
   PK_CHECK_LAUNCH("batch_copy_kernel");
-  const int jb_blocks = (int)((nj + 63) / 64);
-  batch_sc_start_kernel<<<jb_blocks, 64, 0, s>>>(b->d_state, b->d_jobs, nj);
+  const unsigned jb_blocks = (nj + kScJobs - 1) / kScJobs;
+  batch_sc_start_kernel<<<jb_blocks, skytc::kThreads, 0, s>>>(b->d_state, nj);
   PK_CHECK_LAUNCH("batch_sc_start_kernel");
   batch_eq_half_kernel<<<ew_blocks(b->eq_half.total), 256, 0, s>>>(
       b->eq_half.d_desc, b->eq_half.d_begin, b->eq_half.n, b->eq_half.total, b->d_state, b->d_jobs);
@@ -655,13 +736,39 @@ static int batch_enqueue(pkg_batch* b, cudaStream_t s) {
       batch_sc_round_kernel<true><<<(unsigned)g.total, kScThreads, 0, s>>>(
           g.d_desc, g.d_begin, g.n, b->d_jobs, b->d_state, r);
     PK_CHECK_LAUNCH("batch_sc_round_kernel");
-    batch_sc_finish_round_kernel<<<jb_blocks, 64, 0, s>>>(b->d_state, b->d_jobs, nj, r,
+    batch_sc_finish_round_kernel<<<jb_blocks, skytc::kThreads, 0, s>>>(b->d_state, b->d_jobs, nj, r,
                                                           b->d_nctas + (size_t)r * nj);
     PK_CHECK_LAUNCH("batch_sc_finish_round_kernel");
   }
-  batch_sc_end_kernel<<<jb_blocks, 64, 0, s>>>(b->d_state, nj);
+  batch_sc_end_kernel<<<jb_blocks, skytc::kThreads, 0, s>>>(b->d_state, nj);
   PK_CHECK_LAUNCH("batch_sc_end_kernel");
   return PKG_OK;
+}
+
+// Enqueue the whole batch on s.
+static int batch_enqueue(pkg_batch* b, cudaStream_t s) {
+  const uint32_t nj = (uint32_t)b->jobs.size();
+  PK_CUDA(cudaMemcpyAsync(b->d_state, b->d_state_init, sizeof(ScState) * nj,
+                          cudaMemcpyDeviceToDevice, s));
+  for (auto& p : b->passes) {
+    if (p.smem > 32 * 1024)  // beside the tile's own shared memory
+      PK_CUDA(cudaFuncSetAttribute(batch_ntt_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)p.smem));
+    batch_ntt_pass_kernel<<<(unsigned)p.ctas, tc::kThreads, p.smem, s>>>(p.d_desc, p.d_begin, p.n,
+                                                                     b->roots);
+    PK_CHECK_LAUNCH("batch_ntt_pass_kernel");
+  }
+  // The trees and the sumchecks both need only the transforms: the sumcheck
+  // rounds, whose transcripts leave the GPU nearly idle, run beside the trees
+  // on the batch's own stream, with priority, since they are the longer chain.
+  PK_CUDA(cudaEventRecord(b->forked, s));
+  PK_CUDA(cudaStreamWaitEvent(b->side, b->forked, 0));
+  int rc = enqueue_sumchecks(b, b->side);
+  const int rc2 = rc ? rc : enqueue_trees(b, s);
+  // joined also after a failed launch, so that a capture can end
+  PK_CUDA(cudaEventRecord(b->joined, b->side));
+  PK_CUDA(cudaStreamWaitEvent(s, b->joined, 0));
+  return rc2;
 }
 
 static void drop_graph(pkg_batch* b) {
@@ -804,6 +911,15 @@ extern "C" int pkg_batch_create(const uint32_t* log_sizes, size_t njobs, uint64_
     pkg_batch_destroy(b);
     return cuda_status(e, "pkg_batch_create tables");
   }
+  int low = 0, high = 0;
+  e = cudaDeviceGetStreamPriorityRange(&low, &high);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->side, cudaStreamNonBlocking, high);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->joined, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    pkg_batch_destroy(b);
+    return cuda_status(e, "pkg_batch_create stream");
+  }
   int rc = roots_reserve(max_order, &b->roots);
   if (!rc) rc = batch_replan(b);
   if (rc) {
@@ -823,6 +939,9 @@ extern "C" void pkg_batch_destroy(pkg_batch* b) {
   cudaFree(b->d_state_init);
   cudaFree(b->d_nctas);
   cudaFree(b->tables);
+  if (b->forked) cudaEventDestroy(b->forked);
+  if (b->joined) cudaEventDestroy(b->joined);
+  if (b->side) cudaStreamDestroy(b->side);
   delete b;
 }
 
@@ -924,32 +1043,27 @@ extern "C" int pkg_batch_tune(pkg_batch* b, pkg_stream_t stream, int* best_kmax,
   PK_CUDA(cudaEventCreate(&e0));
   PK_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
-  int bk = b->kmax, be = b->log_elems, bb = b->log_bpt;
+  int bk = b->kmax, be = b->log_elems;
   for (int k = 4; k <= 11; k++) {
     for (int le = std::max(k, 8); le <= 11; le++) {
-      for (int lb = 0; lb <= 2; lb++) {
-        b->log_bpt = lb;
-        int rc = pkg_batch_set_params(b, k, le);
-        if (rc) return rc;
-        if ((rc = batch_enqueue(b, s))) return rc;  // warm-up
-        PK_CUDA(cudaEventRecord(e0, s));
-        if ((rc = batch_enqueue(b, s))) return rc;
-        PK_CUDA(cudaEventRecord(e1, s));
-        PK_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best) {
-          best = ms;
-          bk = k;
-          be = le;
-          bb = lb;
-        }
+      int rc = pkg_batch_set_params(b, k, le);
+      if (rc) return rc;
+      if ((rc = batch_enqueue(b, s))) return rc;  // warm-up
+      PK_CUDA(cudaEventRecord(e0, s));
+      if ((rc = batch_enqueue(b, s))) return rc;
+      PK_CUDA(cudaEventRecord(e1, s));
+      PK_CUDA(cudaEventSynchronize(e1));
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      if (ms < best) {
+        best = ms;
+        bk = k;
+        be = le;
       }
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  b->log_bpt = bb;
   int rc = pkg_batch_set_params(b, bk, be);
   if (rc) return rc;
   if (best_kmax) *best_kmax = bk;

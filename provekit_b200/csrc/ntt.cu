@@ -19,6 +19,7 @@
 #include "fr.cuh"
 #include "fr_host.hpp"
 #include "ntt_internal.cuh"
+#include "ntt_tile.cuh"
 #include "host_stage.cuh"
 #include "pk_common.cuh"
 #include "tc_reduce.cuh"
@@ -155,88 +156,6 @@ __device__ __forceinline__ Fr source_load(const NttSource& s, uint64_t g) {
   return fr_zero();
 }
 
-__device__ __forceinline__ Fr tile_load(const uint4* sm, int E, int i) {
-  const uint4 a = sm[i], b = sm[E + i];
-  Fr x;
-  x.v[0] = a.x; x.v[1] = a.y; x.v[2] = a.z; x.v[3] = a.w;
-  x.v[4] = b.x; x.v[5] = b.y; x.v[6] = b.z; x.v[7] = b.w;
-  return x;
-}
-__device__ __forceinline__ void tile_store(uint4* sm, int E, int i, const Fr& x) {
-  sm[i] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-  sm[E + i] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
-}
-// The product where the tensor cores' wait ran out (w < p, x < 5 p).
-static __device__ __noinline__ Fr product_alone(const Fr w, const Fr x) { return fr_mul(w, x); }
-
-// Index of tile element e in the data and in shared memory.
-template <bool kModeB>
-__device__ __forceinline__ void pass_index(int e, int K, int T, int log_t, int log_u, uint64_t U,
-                                           uint64_t l0, uint64_t high, uint64_t u0, uint64_t* g,
-                                           int* sidx) {
-  if (!kModeB) {
-    const int j = e >> log_t, ll = e & (T - 1);
-    *g = ((high << K) + j) * U + u0 + ll;
-    *sidx = e;
-  } else {
-    const int j = (e >> log_u) & ((1 << K) - 1);
-    const int hl = e >> (log_u + K);
-    const int u = e & ((1 << log_u) - 1);
-    *g = (((l0 >> log_u) << K) << log_u) + e;
-    *sidx = j * T + (hl << log_u) + u;
-  }
-}
-
-// x0, m -> x0 + m, x0 - m mod p, loosely: for x0 < 5 p and m < 1.1 p both
-// results are below 5 p (and 2^256).  2 p is taken from the sum when x0 is
-// above it, and added to the difference when it is not (x0 is compared by its
-// top word, so the border is up to 2^224 above 2 p).
-__device__ __forceinline__ void loose_butterfly(const Fr& x0, const Fr& m, Fr& y0, Fr& y1) {
-  asm("{\n\t"
-      ".reg .pred b;\n\t"
-      "setp.ge.u32 b, %23, 0x60c89ce6;\n\t"
-      "add.cc.u32  %0, %16, %24;\n\t"
-      "addc.cc.u32 %1, %17, %25;\n\t"
-      "addc.cc.u32 %2, %18, %26;\n\t"
-      "addc.cc.u32 %3, %19, %27;\n\t"
-      "addc.cc.u32 %4, %20, %28;\n\t"
-      "addc.cc.u32 %5, %21, %29;\n\t"
-      "addc.cc.u32 %6, %22, %30;\n\t"
-      "addc.u32    %7, %23, %31;\n\t"
-      "sub.cc.u32  %8,  %16, %24;\n\t"
-      "subc.cc.u32 %9,  %17, %25;\n\t"
-      "subc.cc.u32 %10, %18, %26;\n\t"
-      "subc.cc.u32 %11, %19, %27;\n\t"
-      "subc.cc.u32 %12, %20, %28;\n\t"
-      "subc.cc.u32 %13, %21, %29;\n\t"
-      "subc.cc.u32 %14, %22, %30;\n\t"
-      "subc.u32    %15, %23, %31;\n\t"
-      "@b sub.cc.u32  %0, %0, 0xe0000002;\n\t"
-      "@b subc.cc.u32 %1, %1, 0x87c3eb27;\n\t"
-      "@b subc.cc.u32 %2, %2, 0xf372e122;\n\t"
-      "@b subc.cc.u32 %3, %3, 0x5067d090;\n\t"
-      "@b subc.cc.u32 %4, %4, 0x0302b0ba;\n\t"
-      "@b subc.cc.u32 %5, %5, 0x70a08b6d;\n\t"
-      "@b subc.cc.u32 %6, %6, 0xc2634053;\n\t"
-      "@b subc.u32    %7, %7, 0x60c89ce5;\n\t"
-      "@!b add.cc.u32  %8,  %8,  0xe0000002;\n\t"
-      "@!b addc.cc.u32 %9,  %9,  0x87c3eb27;\n\t"
-      "@!b addc.cc.u32 %10, %10, 0xf372e122;\n\t"
-      "@!b addc.cc.u32 %11, %11, 0x5067d090;\n\t"
-      "@!b addc.cc.u32 %12, %12, 0x0302b0ba;\n\t"
-      "@!b addc.cc.u32 %13, %13, 0x70a08b6d;\n\t"
-      "@!b addc.cc.u32 %14, %14, 0xc2634053;\n\t"
-      "@!b addc.u32    %15, %15, 0x60c89ce5;\n\t"
-      "}"
-      : "=&r"(y0.v[0]), "=&r"(y0.v[1]), "=&r"(y0.v[2]), "=&r"(y0.v[3]), "=&r"(y0.v[4]),
-        "=&r"(y0.v[5]), "=&r"(y0.v[6]), "=&r"(y0.v[7]), "=&r"(y1.v[0]), "=&r"(y1.v[1]),
-        "=&r"(y1.v[2]), "=&r"(y1.v[3]), "=&r"(y1.v[4]), "=&r"(y1.v[5]), "=&r"(y1.v[6]),
-        "=&r"(y1.v[7])
-      : "r"(x0.v[0]), "r"(x0.v[1]), "r"(x0.v[2]), "r"(x0.v[3]), "r"(x0.v[4]), "r"(x0.v[5]),
-        "r"(x0.v[6]), "r"(x0.v[7]), "r"(m.v[0]), "r"(m.v[1]), "r"(m.v[2]), "r"(m.v[3]),
-        "r"(m.v[4]), "r"(m.v[5]), "r"(m.v[6]), "r"(m.v[7]));
-}
-
 // Most stages per pass: 8.  2^24 points take 2.89 ms as three 8-stage passes,
 // 3.06 as four of 6; 9 (tiles of one line) save a pass at 2^17 and 2^18 points
 // (40.5 against 43.2 us) but cost 5 % at 18 stages over 16 columns of 2^20.
@@ -264,7 +183,7 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
   extern __shared__ uint4 sm[];
   __shared__ tc::ProductShared sh;
   const int K = shape.K, T = shape.T, log_t = shape.log_t, log_u = shape.log_u;
-  const int E = T << K, half = E >> 1;
+  const int E = T << K;
   const uint64_t U = shape.U;
   tc::ProductTile tile;
   tile.open(sh, tc::kProductImage);
@@ -278,7 +197,7 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    pass_index<kModeB>(e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    pass_index(kModeB, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     if (kSrc) {
       const Fr v = source_load(src, g);
       sm[sidx] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
@@ -290,51 +209,12 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
     }
   }
   __syncthreads();
-  // ---- K radix-2 stages in shared memory ----
-#pragma unroll 1
-  for (int s = 0; s < K; s++) {
-    const int log_h = K - 1 - s;
-#pragma unroll 1
-    for (int b0 = 0; b0 < half; b0 += tc::kThreads) {
-      const int b = b0 + (int)threadIdx.x;
-      const bool live = b < half;
-      const int bb = live ? b : 0;  // others repeat butterfly 0 and store nothing
-      const int ll = bb & (T - 1);
-      const int pp = bb >> log_t;
-      const int grp = pp >> log_h;
-      const int j0 = (grp << (log_h + 1)) + (pp & ((1 << log_h) - 1));
-      const int i0 = j0 * T + ll, i1 = i0 + (T << log_h);
-      const Fr x1 = tile_load(sm, E, i1);
-      Fr m;
-      if (shape.first && s == 0) {
-        m = fr_reduce_once(x1);
-      } else {
-        const uint64_t high = kModeB ? (l0 + ll) >> log_u : high_a;
-        const Fr w = fr_load_ro(roots, (high << s) | (uint64_t)grp);
-        uint32_t S[9];
-        tile.start(w, x1);
-        tile.finish(S);
-        if (tile.alone)
-          m = product_alone(w, x1);
-        else
-          m = tc::quotient_step(S);
-        __syncwarp();
-      }
-      const Fr x0 = tile_load(sm, E, i0);
-      Fr y0, y1;
-      loose_butterfly(x0, m, y0, y1);
-      if (live) {
-        tile_store(sm, E, i0, y0);
-        tile_store(sm, E, i1, y1);
-      }
-    }
-    __syncthreads();
-  }
+  tile_stages(tile, sm, kModeB, K, T, log_t, log_u, l0, high_a, shape.first, roots);
   // ---- store ----
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    pass_index<kModeB>(e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    pass_index(kModeB, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     Fr v = tile_load(sm, E, sidx);
     if (shape.last) v = fr_reduce_once(tc::reduce_any(v));
     fr_store(data, g, v);

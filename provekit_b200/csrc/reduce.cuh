@@ -16,40 +16,77 @@ namespace pk {
 
 constexpr int kRedThreads = 256;
 
+// Sums of field elements as integers, limb by limb: 256 limbs of 24 bits fit
+// 32 bits, so a warp adds each limb with one redux and a total is reduced
+// once.  (Modular additions down a shuffle tree were 5 dependent levels of 8
+// shuffles and a 16-step carry chain each.)
 constexpr int kSumLimbs = 11;  // 24-bit limbs of an element
 
+// This warp's sum of x, limb by limb, in every lane.
+__device__ __forceinline__ void warp_limbs(const Fr& v, uint32_t* sum) {
+  constexpr uint32_t M = 0xffffffu;
+  const uint32_t* x = v.v;
+  const uint32_t d[kSumLimbs] = {x[0] & M,
+                                 __funnelshift_r(x[0], x[1], 24) & M,
+                                 __funnelshift_r(x[1], x[2], 16) & M,
+                                 x[2] >> 8,
+                                 x[3] & M,
+                                 __funnelshift_r(x[3], x[4], 24) & M,
+                                 __funnelshift_r(x[4], x[5], 16) & M,
+                                 x[5] >> 8,
+                                 x[6] & M,
+                                 __funnelshift_r(x[6], x[7], 24) & M,
+                                 x[7] >> 16};
+#pragma unroll
+  for (int i = 0; i < kSumLimbs; i++) sum[i] = __reduce_add_sync(0xffffffffu, d[i]);
+}
+
+// sum limbs[i] 2^(24 i) mod p, fully reduced, of at most 256 elements
+__device__ __forceinline__ Fr limbs_reduce(const uint32_t* limbs) {
+  constexpr uint32_t M = 0xffffffu;
+  uint32_t d[kSumLimbs + 1], S[9];
+  uint64_t carry = 0;
+#pragma unroll
+  for (int i = 0; i < kSumLimbs; i++) {
+    carry += limbs[i];
+    d[i] = (uint32_t)carry & M;
+    carry >>= 24;
+  }
+  d[kSumLimbs] = (uint32_t)carry;
+  S[0] = d[0] | (d[1] << 24);
+  S[1] = (d[1] >> 8) | (d[2] << 16);
+  S[2] = (d[2] >> 16) | (d[3] << 8);
+  S[3] = d[4] | (d[5] << 24);
+  S[4] = (d[5] >> 8) | (d[6] << 16);
+  S[5] = (d[6] >> 16) | (d[7] << 8);
+  S[6] = d[8] | (d[9] << 24);
+  S[7] = (d[9] >> 8) | (d[10] << 16);
+  S[8] = (d[10] >> 16) | (d[11] << 8);
+  return fr_reduce_once(tc::quotient_step(S));
+}
+
+// This warp's sum of x in every lane.
+__device__ __forceinline__ Fr warp_sum(const Fr& x) {
+  uint32_t limbs[kSumLimbs];
+  warp_limbs(x, limbs);
+  return limbs_reduce(limbs);
+}
+
 // Block-wide sum of K field elements per thread (at most 256 threads); thread
-// 0 gets the result, fully reduced.  Elements are added as integers, limb by
-// limb: 256 limbs of 24 bits fit 32 bits, so a warp adds each limb with one
-// redux, one warp adds the warps' sums, and the total is reduced once.  Bound
-// by latency: modular additions down a shuffle tree took 5 + 5 dependent
-// levels of 8 shuffles and a 16-step carry chain each.
+// 0 gets the result, fully reduced: the warps' limbs are added by one warp.
 template <int K>
 __device__ __forceinline__ void block_sum(Fr (&v)[K]) {
   __shared__ uint32_t limbs[kRedThreads / 32][K * kSumLimbs];
   __shared__ uint32_t total[K * kSumLimbs];
   __shared__ Fr sums[K];
-  constexpr uint32_t M = 0xffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < K; k++) {
-    const uint32_t* x = v[k].v;
-    const uint32_t d[kSumLimbs] = {x[0] & M,
-                                   __funnelshift_r(x[0], x[1], 24) & M,
-                                   __funnelshift_r(x[1], x[2], 16) & M,
-                                   x[2] >> 8,
-                                   x[3] & M,
-                                   __funnelshift_r(x[3], x[4], 24) & M,
-                                   __funnelshift_r(x[4], x[5], 16) & M,
-                                   x[5] >> 8,
-                                   x[6] & M,
-                                   __funnelshift_r(x[6], x[7], 24) & M,
-                                   x[7] >> 16};
+    uint32_t sum[kSumLimbs];
+    warp_limbs(v[k], sum);
+    if (lane == 0)
 #pragma unroll
-    for (int i = 0; i < kSumLimbs; i++) {
-      const uint32_t sum = __reduce_add_sync(0xffffffffu, d[i]);
-      if (lane == 0) limbs[warp][k * kSumLimbs + i] = sum;
-    }
+      for (int i = 0; i < kSumLimbs; i++) limbs[warp][k * kSumLimbs + i] = sum[i];
   }
   __syncthreads();
   if (warp == 0) {
@@ -60,27 +97,7 @@ __device__ __forceinline__ void block_sum(Fr (&v)[K]) {
       total[i] = sum;
     }
     __syncwarp();
-    if (lane < K) {
-      uint32_t d[kSumLimbs + 1], S[9];
-      uint64_t carry = 0;
-#pragma unroll
-      for (int i = 0; i < kSumLimbs; i++) {
-        carry += total[lane * kSumLimbs + i];
-        d[i] = (uint32_t)carry & M;
-        carry >>= 24;
-      }
-      d[kSumLimbs] = (uint32_t)carry;
-      S[0] = d[0] | (d[1] << 24);
-      S[1] = (d[1] >> 8) | (d[2] << 16);
-      S[2] = (d[2] >> 16) | (d[3] << 8);
-      S[3] = d[4] | (d[5] << 24);
-      S[4] = (d[5] >> 8) | (d[6] << 16);
-      S[5] = (d[6] >> 16) | (d[7] << 8);
-      S[6] = d[8] | (d[9] << 24);
-      S[7] = (d[9] >> 8) | (d[10] << 16);
-      S[8] = (d[10] >> 16) | (d[11] << 8);
-      sums[lane] = fr_reduce_once(tc::quotient_step(S));
-    }
+    if (lane < K) sums[lane] = limbs_reduce(total + lane * kSumLimbs);
     __syncwarp();
     if (lane == 0)
 #pragma unroll

@@ -179,11 +179,26 @@ struct SkyTile : Tile {
     return quotient_step(S);
   }
 
-  // In place of compress in a warp that has nothing to compress while others of
+  // In place of compress or permute in a warp that has nothing to compress while others of
   // the CTA do.
   __device__ __forceinline__ void sit_out() {
 #pragma unroll 1
     for (int i = 0; i < kSquares; i++) cta_sync();  // kSquares completions: phase as it was
+  }
+
+  // The permutation without the feed-forward (skyscraper/core/src/reference.rs:49-60),
+  // l < 2.2 p and r < 1.1 p to both below 1.1 p.
+  __device__ __forceinline__ void permute(Fr& l, Fr& r) {
+#pragma unroll 1
+    for (int k = 0; k < 18; k += 2) {
+      if (k == 6 || k == 10) {
+        r = bar_round(l, r, k);
+        l = bar_round(r, l, k + 1);
+      } else {
+        r = square_round<false>(l, r, k, false);
+        l = square_round<false>(r, l, k + 1, false);
+      }
+    }
   }
 
   // Skyscraper compress(l, r) in [0, 1.1 p) for l < 1.1 p and r < 2^256

@@ -1,44 +1,12 @@
 // sumcheck_device.cuh -- device-side pieces of the Spartan zk-sumcheck used by
-// the batched form: the transcript stand-in (same definition as the host's
-// pkg_transcript_*), compute_blinding_coefficients_for_round
-// (provekit/prover/src/whir_r1cs.rs:427-492) and the cubic evaluation
-// (provekit/common/src/utils/sumcheck.rs:156-158), one thread per job.
+// the batched form: compute_blinding_coefficients_for_round
+// (provekit/prover/src/whir_r1cs.rs:427-492) by one warp and the cubic
+// evaluation (provekit/common/src/utils/sumcheck.rs:156-158).
 #pragma once
 #include "fr.cuh"
-#include "skyscraper.cuh"
+#include "reduce.cuh"
 
 namespace pk {
-
-// reference::permute (skyscraper/core/src/reference.rs:49-60) on canonical
-// values: 18 rounds, square (Montgomery square of a canonical value = l^2 *
-// SIGMA_INV) or bar, plus the round constant.
-__device__ __forceinline__ void sky_permute(Fr& l, Fr& r) {
-#pragma unroll 1
-  for (int k = 0; k < 18; k++) {
-    const bool is_bar = (k == 6 || k == 7 || k == 10 || k == 11);
-    Fr f = is_bar ? sky_bar(l) : fr_sqr(l);
-    Fr nl = fr_add(fr_add(r, f), sky_rc(k));
-    r = l;
-    l = nl;
-  }
-}
-
-struct DevTranscript {
-  Fr l, r;  // canonical
-  __device__ void init(const Fr& domain_canonical) {
-    l = domain_canonical;
-    r = fr_zero();
-    sky_permute(l, r);
-  }
-  __device__ void absorb(const Fr& x_mont) {
-    l = fr_add(l, fr_from_mont(x_mont));
-    sky_permute(l, r);
-  }
-  __device__ Fr squeeze() {
-    sky_permute(l, r);
-    return fr_to_mont(l);
-  }
-};
 
 __device__ __forceinline__ Fr dev_cubic(const Fr* c, const Fr& x) {
   Fr acc = fr_mul(x, c[3]);
@@ -76,34 +44,38 @@ __device__ __forceinline__ Fr fr_half_mont() {
   return h;
 }
 
-// compute_blinding_coefficients_for_round (whir_r1cs.rs:427-492); g: n x 4,
-// alphas: at least compute_for entries.
-__device__ __forceinline__ void dev_blinding_coeffs(const Fr* g, int n, int compute_for,
-                                                    const Fr* alphas, Fr out[4]) {
-  bool all_fixed = false;
-  int cf = compute_for;
-  if (cf == n) {
-    all_fixed = true;
-    cf = n - 1;
-  }
+// compute_blinding_coefficients_for_round (whir_r1cs.rs:427-492) for
+// compute_for < n <= 32 by one warp: lane i takes g_i (n x 4; alphas: at least
+// compute_for entries) and the six products by powers of two run in six lanes.
+// scratch: six Fr of this warp's.  Every lane gets the result.
+__device__ __forceinline__ void warp_blinding_coeffs(const Fr* g, int n, int compute_for,
+                                                     const Fr* alphas, int lane, Fr* scratch,
+                                                     Fr out[4]) {
   Fr prefix = fr_zero(), suffix = fr_zero();
-  for (int i = 0; i < cf; i++) prefix = fr_add(prefix, dev_cubic(g + 4 * i, alphas[i]));
-  for (int i = cf + 1; i < n; i++)
-    suffix = fr_add(suffix, fr_add(dev_cubic(g + 4 * i, fr_zero()), dev_cubic(g + 4 * i, fr_one_mont())));
-  Fr pm = fr_one_mont();
-  for (int i = 0; i < n - 1 - cf; i++) pm = fr_add(pm, pm);
-  Fr sm = fr_mul(pm, fr_half_mont());
-  Fr cst = fr_add(fr_mul(pm, prefix), fr_mul(sm, suffix));
-  const Fr* cur = g + 4 * cf;
-  Fr res[4] = {fr_add(fr_mul(pm, cur[0]), cst), fr_mul(pm, cur[1]), fr_mul(pm, cur[2]),
-               fr_mul(pm, cur[3])};
-  if (all_fixed) {
-    out[0] = dev_cubic(res, alphas[cf]);
-    out[1] = out[2] = out[3] = fr_zero();
-    return;
+  if (lane < compute_for) {
+    prefix = dev_cubic(g + 4 * lane, alphas[lane]);
+  } else if (lane > compute_for && lane < n) {  // at 0 and at 1
+    const Fr* c = g + 4 * lane;
+    suffix = fr_add(fr_add(fr_add(c[0], c[0]), c[1]), fr_add(c[2], c[3]));
   }
+  __syncwarp();
+  prefix = warp_sum(prefix);
+  suffix = warp_sum(suffix);
+  const int e = n - 1 - compute_for;  // 2^e on the current terms and the prefix, 2^(e-1) on the suffix
+  Fr pow2 = fr_zero();
+  pow2.v[0] = 1u << e;
+  const Fr pm = fr_to_mont(pow2);
+  if (lane < 6) {
+    const Fr x = lane < 4 ? g[4 * compute_for + lane] : (lane == 4 ? prefix : suffix);
+    Fr w = pm;
+    if (lane == 5) w = fr_mul(pm, fr_half_mont());
+    scratch[lane] = fr_mul(x, w);
+  }
+  __syncwarp();
+  out[0] = fr_add(scratch[0], fr_add(scratch[4], scratch[5]));
 #pragma unroll
-  for (int k = 0; k < 4; k++) out[k] = res[k];
+  for (int k = 1; k < 4; k++) out[k] = scratch[k];
+  __syncwarp();
 }
 
 // The Spartan round code below multiplies 14 times per pair; inlining every
