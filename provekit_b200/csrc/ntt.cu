@@ -145,14 +145,17 @@ int roots_reserve(size_t order, const uint64_t** out) {
 // product on the integer pipe; with CTAs that stay for several tiles 3.30 ms,
 // since they do not finish together.
 // ---------------------------------------------------------------------------
+// Where a transform's first pass reads its input.
+enum : int { kFromData = 0, kFromEncode = 1, kFromReversed = 2 };
+
 // Element g of the RS-encode layout (see NttSource).
-__device__ __forceinline__ Fr source_load(const NttSource& s, uint64_t g) {
+__device__ __forceinline__ Fr encode_load(const NttSource& s, uint64_t g) {
   const uint64_t x = g % s.chunk;
   if (x < s.L * s.M) {
     const uint64_t row = x / s.M, col = x - row * s.M;
-    return fr_load_ro(s.messages, col * s.L + row);
+    return fr_load(s.messages, col * s.L + row);
   }
-  if (x - s.L * s.M < s.mask_len) return fr_load_ro(s.masks, x - s.L * s.M);
+  if (x - s.L * s.M < s.mask_len) return fr_load(s.masks, x - s.L * s.M);
   return fr_zero();
 }
 
@@ -166,19 +169,45 @@ constexpr int kPassStages = 8;
 constexpr int kTileElems = 9, kSmallTileElems = 8;
 constexpr uint64_t kSmallBelow = uint64_t(1) << 21;
 
+// x 2^-k mod p for x < 5 p and 1 <= k <= 28, below 4 p: p is 1 mod 2^28, so
+// (-x mod 2^k) p is what x lacks to a multiple of 2^k.
+__device__ __forceinline__ Fr halve(const Fr& x, int k) {
+  constexpr uint32_t P[8] = {PK_P0, PK_P1, PK_P2, PK_P3, PK_P4, PK_P5, PK_P6, PK_P7};
+  const uint32_t m = (0u - x.v[0]) & ((1u << k) - 1);
+  uint32_t E[8], O[8], S[9];
+  fr_first_row(E, O, P, m);
+#pragma unroll
+  for (int i = 0; i < 8; i++) S[i] = E[i];
+  S[8] = 0;
+  const uint32_t odd[8] = {0, O[0], O[1], O[2], O[3], O[4], O[5], O[6]};
+  tc::add9(S, odd);
+  S[8] += O[7];
+  tc::add9(S, x.v);
+  Fr r;
+#pragma unroll
+  for (int i = 0; i < 8; i++) r.v[i] = __funnelshift_r(S[i], S[i + 1], k);
+  return r;
+}
+
+// Index i of log_n bits, reversed.
+__device__ __forceinline__ uint64_t reversed(uint64_t i, int log_n) {
+  return __brevll(i) >> (64 - log_n);
+}
+
 struct PassShape {
   uint64_t U;  // lines per `high`
   int log_u, T, log_t, K;
   bool first;      // stage 0 of the pass is stage 0 of the transform: every twiddle is 1
   bool last;       // store fully reduced; other passes leave values below 5 p
+  int inverse;     // last pass of an inverse over 2^inverse points, or 0
 };
 
 // kModeB selects mode B at compile time.  In mode A every line of the CTA
 // shares `high`, so stage s reads only the 2^s twiddles roots[(high << s) |
 // grp], which stay in L1.
-template <bool kSrc, bool kModeB>
+template <int kSrc, bool kModeB>
 __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
-    ntt_pass_kernel(uint64_t* __restrict__ data, const uint64_t* __restrict__ roots,
+    ntt_pass_kernel(uint64_t* data, uint64_t* out, const uint64_t* __restrict__ roots,
                     const PassShape shape, const NttSource src) {
   extern __shared__ uint4 sm[];
   __shared__ tc::ProductShared sh;
@@ -198,8 +227,11 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
     uint64_t g;
     int sidx;
     pass_index(kModeB, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
-    if (kSrc) {
-      const Fr v = source_load(src, g);
+    if (kSrc != kFromData) {
+      // reversed: the inverse's first permutation, v[bitrev((n - g) mod n)]
+      const Fr v = kSrc == kFromEncode
+                       ? encode_load(src, g)
+                       : fr_load(src.messages, reversed((src.L - g) & (src.L - 1), (int)src.M));
       sm[sidx] = make_uint4(v.v[0], v.v[1], v.v[2], v.v[3]);
       sm[E + sidx] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
     } else {
@@ -216,8 +248,9 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
     int sidx;
     pass_index(kModeB, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     Fr v = tile_load(sm, E, sidx);
+    if (shape.inverse) v = halve(v, shape.inverse);
     if (shape.last) v = fr_reduce_once(tc::reduce_any(v));
-    fr_store(data, g, v);
+    fr_store(out, shape.inverse ? reversed(g, shape.inverse) : g, v);
   }
   tile.close();
 }
@@ -225,9 +258,12 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
 static inline uint64_t pow2_part(uint64_t x) { return x & (~x + 1); }
 
 // Run global stages [t_begin, t_end) of an N-point transform over M columns;
-// t_end is the last stage.
-int ntt_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end, const uint64_t* roots,
-               cudaStream_t stream, const NttSource* src) {
+// t_end is the last stage.  inverse: the stages of an inverse transform, which
+// reads and writes `inverse` in the inverse's orders (data is scratch between
+// passes; src describes the reads).
+static int run_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end,
+                      const uint64_t* roots, cudaStream_t stream, const NttSource* src,
+                      uint64_t* inverse) {
   const int total = t_end - t_begin;
   if (total <= 0) return PKG_OK;
   const int npasses = (total + kPassStages - 1) / kPassStages;
@@ -250,25 +286,34 @@ int ntt_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end, const
     shape.K = K;
     shape.first = t == 0;
     shape.last = pi == npasses - 1;
+    shape.inverse = inverse && shape.last ? log2_exact(N) : 0;
     const size_t smem = 32 * (T << K);
     const unsigned grid = (unsigned)(num_lines / T);
     NttSource s;
     memset(&s, 0, sizeof s);
+    int kind = kFromData;
     if (src && pi == 0) {
       s = *src;
-      if (mode_b)
-        ntt_pass_kernel<true, true><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
-      else
-        ntt_pass_kernel<true, false><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
-    } else if (mode_b) {
-      ntt_pass_kernel<false, true><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
-    } else {
-      ntt_pass_kernel<false, false><<<grid, tc::kThreads, smem, stream>>>(data, roots, shape, s);
+      kind = inverse ? kFromReversed : kFromEncode;
     }
+    uint64_t* const out = inverse && shape.last ? inverse : data;
+    void (*fn)(uint64_t*, uint64_t*, const uint64_t*, PassShape, NttSource) =
+        kind == kFromData
+            ? (mode_b ? ntt_pass_kernel<kFromData, true> : ntt_pass_kernel<kFromData, false>)
+        : kind == kFromEncode
+            ? (mode_b ? ntt_pass_kernel<kFromEncode, true> : ntt_pass_kernel<kFromEncode, false>)
+            : (mode_b ? ntt_pass_kernel<kFromReversed, true>
+                      : ntt_pass_kernel<kFromReversed, false>);
+    fn<<<grid, tc::kThreads, smem, stream>>>(data, out, roots, shape, s);
     PK_CHECK_LAUNCH("ntt_pass_kernel");
     t += K;
   }
   return PKG_OK;
+}
+
+int ntt_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end, const uint64_t* roots,
+               cudaStream_t stream, const NttSource* src) {
+  return run_stages(data, N, M, t_begin, t_end, roots, stream, src, nullptr);
 }
 
 // Validation shared by the device and host forms (reference panics ->
@@ -322,51 +367,35 @@ int ntt_nr_from_source(uint64_t* out, size_t len, size_t codeword_size, size_t n
 
 // ---------------------------------------------------------------------------
 // intt_rn: reverse_order -> values[1..].reverse() -> ntt_nr -> * n^-1 ->
-// reverse_order (ntt/src/ntt.rs:326-348), as two gathers around the NTT:
-//   v2[i] = v0[bitrev((n - i) mod n)]             (in -> tmp)
-//   v4[i] = v3[bitrev(i)] * n^-1                   (tmp -> out)
+// reverse_order (ntt/src/ntt.rs:326-348): the first pass reads
+// v0[bitrev((n - i) mod n)], the last one stores v3[i] n^-1 at bitrev(i).  (As
+// two gathers around the transform: 2^16 points 37.5 us; 2^k points' n^-1 is a
+// shift, see halve.)
 // ---------------------------------------------------------------------------
-__global__ void intt_gather_in(const uint64_t* __restrict__ src, uint64_t* __restrict__ dst,
-                               size_t n, int log_n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    size_t k = (n - i) & (n - 1);
-    size_t r = log_n ? (__brevll((unsigned long long)k) >> (64 - log_n)) : 0;
-    fr_store(dst, i, fr_load(src, r));
-  }
-}
-
-__global__ void intt_gather_out(const uint64_t* __restrict__ src, uint64_t* __restrict__ dst,
-                                size_t n, int log_n, Fr ninv) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    size_t r = log_n ? (__brevll((unsigned long long)i) >> (64 - log_n)) : 0;
-    fr_store(dst, i, fr_mul(fr_load(src, r), ninv));
-  }
-}
-
 int intt_rn_device(uint64_t* values, size_t len, cudaStream_t stream) {
   PK_REQUIRE(is_pow2(len), "intt_rn length %zu is not a power of two", len);
   PK_REQUIRE(len <= (size_t(1) << 28), "intt_rn length %zu exceeds 2^28", len);
   PK_REQUIRE(values != nullptr, "null values pointer");
   PK_REQUIRE(aligned16(values), "device buffers must be 16-byte aligned");
   if (len == 1) return PKG_OK;  // both permutations and the scale are identities
+  const uint64_t* roots = nullptr;
+  int rc = roots_reserve(len, &roots);
+  if (rc) return rc;
+  const int log_n = log2_exact(len);
+  NttSource src;
+  memset(&src, 0, sizeof src);
+  src.messages = values;
+  src.L = len;
+  src.M = (uint64_t)log_n;
+  // one pass: one CTA holds every value before it stores the first
+  static_assert(kPassStages <= kSmallTileElems, "a transform of one pass is one tile");
   Scratch tmp;
-  int rc = tmp.alloc(32 * len, stream);
-  if (rc) return rc;
-  uint64_t* t = static_cast<uint64_t*>(tmp.ptr);
-  int log_n = log2_exact(len);
-  int blocks = (int)std::min<size_t>((len + 255) / 256, (size_t)sm_count() * 16);
-  intt_gather_in<<<blocks, 256, 0, stream>>>(values, t, len, log_n);
-  PK_CHECK_LAUNCH("intt_gather_in");
-  rc = ntt_nr_device(t, len, len, 1, stream);
-  if (rc) return rc;
-  HostFr ninv = HostFr::inv(HostFr::from_u64(len));
-  Fr nv;
-  memcpy(nv.v, ninv.l, 32);
-  intt_gather_out<<<blocks, 256, 0, stream>>>(t, values, len, log_n, nv);
-  PK_CHECK_LAUNCH("intt_gather_out");
-  return PKG_OK;
+  uint64_t* between = values;
+  if (log_n > kPassStages) {
+    if ((rc = tmp.alloc(32 * len, stream))) return rc;
+    between = static_cast<uint64_t*>(tmp.ptr);
+  }
+  return run_stages(between, len, 1, 0, log_n, roots, stream, &src, values);
 }
 
 }  // namespace pk
