@@ -304,7 +304,7 @@ static int run_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end
             ? (mode_b ? ntt_pass_kernel<kFromEncode, true> : ntt_pass_kernel<kFromEncode, false>)
             : (mode_b ? ntt_pass_kernel<kFromReversed, true>
                       : ntt_pass_kernel<kFromReversed, false>);
-    fn<<<grid, tc::kThreads, smem, stream>>>(data, out, roots, shape, s);
+    PK_CUDA(launch_early(fn, grid, tc::kThreads, smem, stream, data, out, roots, shape, s));
     PK_CHECK_LAUNCH("ntt_pass_kernel");
     t += K;
   }

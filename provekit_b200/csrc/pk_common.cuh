@@ -50,6 +50,41 @@ void count_launches_undo(uint64_t n);
     }                                          \
   } while (0)
 
+// Number of SMs of the current device (cached per device).
+int sm_count();
+
+// A launch whose CTAs may start while the stream's previous kernel still runs,
+// if that kernel says so (griddepcontrol.launch_dependents); they wait for its
+// end and its writes (griddepcontrol.wait) before they touch global memory.
+// The tiled kernels set up their shared and tensor memory meanwhile.  Such a
+// kernel reads what an earlier one may have written with plain loads only:
+// ld.global.nc is not ordered after the wait.
+//
+// Early only for grids of a few CTAs or of nearly as many as fit:
+// CTAs that start beside others gather on the SMs that have the most room, and
+// between those sizes that leaves the kernel unevenly spread, already with 64
+// CTAs on the 20 SMs that 128 leave free.  2^10 points (2 x
+// 8 CTAs) 18.5 -> 12.7 us, 2^18 (3 x 1024) 61.7 -> 53.0, a commitment's small
+// tree 129 -> 118; but 2^16 points (2 x 256) 26.7 -> 43.4 and 2^16 leaves of 8
+// (512) 101 -> 132, and a tree over 2^14 leaves (128, 64, 1) 149 -> 172.
+template <class... Params, class... Args>
+cudaError_t launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t stream, Args&&... args) {
+  const unsigned sms = (unsigned)sm_count();
+  const bool early = 4 * grid.x <= sms || grid.x >= 6 * sms;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attr;
+  config.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+
 inline bool is_pow2(size_t n) { return n && !(n & (n - 1)); }
 inline int log2_exact(size_t n) {
   int k = 0;
@@ -59,8 +94,6 @@ inline int log2_exact(size_t n) {
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 inline cudaStream_t as_stream(pkg_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// Number of SMs of the current device (cached per device).
-int sm_count();
 
 // Device -> host reads of small results (sumcheck sums, roots, openings)
 // through a per-thread pinned bounce buffer, then a stream synchronisation:

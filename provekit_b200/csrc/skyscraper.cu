@@ -32,9 +32,12 @@ namespace pk {
 #define PK_LEAF_MIN_CTAS 7
 #endif
 
+// Plain loads, as everywhere in kernels of launch_early: the previous kernel may
+// still be writing when they start, and read-only loads (ld.global.nc) are not
+// ordered after griddepcontrol.wait.
 __device__ __forceinline__ Fr load_raw(const uint8_t* p) {
   const uint4* q = reinterpret_cast<const uint4*>(p);
-  uint4 a = __ldg(q), b = __ldg(q + 1);
+  uint4 a = q[0], b = q[1];
   Fr r;
   r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w;
   r.v[4] = b.x; r.v[5] = b.y; r.v[6] = b.z; r.v[7] = b.w;
@@ -97,18 +100,18 @@ struct CodewordRows {  // rows of Fr, in canonical form or as their Montgomery l
   const uint64_t* cw;
   size_t fr_per_leaf;
   __device__ __forceinline__ Fr first(size_t i) const {
-    const Fr x = fr_load_ro(cw, i * fr_per_leaf);
+    const Fr x = fr_load(cw, i * fr_per_leaf);
     return kCanonical ? fr_from_mont(x) : skytc::reduce_any(x);
   }
   __device__ __forceinline__ Fr at(size_t i, size_t k) const {
-    return fr_load_ro(cw, i * fr_per_leaf + k);
+    return fr_load(cw, i * fr_per_leaf + k);
   }
 };
 
 // Left fold of `chunks` >= 2 chunks of each message.
 template <class Messages>
 __global__ void __launch_bounds__(skytc::kThreads, skytc::kMinCtas)
-    fold_tc_kernel(const Messages msgs, size_t chunks, size_t count, uint8_t* __restrict__ out) {
+    fold_tc_kernel(const Messages msgs, size_t chunks, size_t count, uint8_t* out) {
   __shared__ skytc::Shared sh;
   skytc::SkyTile tile;
   tile.open(sh);
@@ -136,7 +139,8 @@ static int fold_tc(const Messages& msgs, size_t chunks, size_t count, uint8_t* o
                    cudaStream_t s) {
   const size_t tiles = (count + skytc::kThreads - 1) / skytc::kThreads;
   PK_REQUIRE(tiles <= 0x7fffffffu, "%zu messages exceed one launch", count);
-  fold_tc_kernel<Messages><<<(unsigned)tiles, skytc::kThreads, 0, s>>>(msgs, chunks, count, out);
+  PK_CUDA(launch_early(fold_tc_kernel<Messages>, (unsigned)tiles, skytc::kThreads, 0, s, msgs,
+                       chunks, count, out));
   PK_CHECK_LAUNCH("fold_tc_kernel");
   return PKG_OK;
 }
@@ -153,7 +157,7 @@ constexpr int kSubNodes = 2 * skytc::kThreads;
 constexpr size_t kSubtreeMax = size_t(1) << 16;
 
 __global__ void __launch_bounds__(skytc::kThreads, 5)
-    merkle_subtree_kernel(uint8_t* __restrict__ lvl, size_t n, int nodes) {
+    merkle_subtree_kernel(uint8_t* lvl, size_t n, int nodes) {
   __shared__ skytc::Shared sh;
   __shared__ uint4 buf[2 * kSubNodes];
   skytc::SkyTile tile;
@@ -239,7 +243,8 @@ int merkle_levels_device(uint8_t* layers, size_t n, cudaStream_t s) {
   }
   while (n > 1) {
     const int nodes = (int)std::min<size_t>(n, kSubNodes);
-    merkle_subtree_kernel<<<(unsigned)(n / nodes), skytc::kThreads, 0, s>>>(cur, n, nodes);
+    PK_CUDA(launch_early(merkle_subtree_kernel, (unsigned)(n / nodes), skytc::kThreads, 0, s, cur,
+                         n, nodes));
     PK_CHECK_LAUNCH("merkle_subtree_kernel");
     for (int k = nodes; k > 1; k /= 2) {
       cur += 32 * n;

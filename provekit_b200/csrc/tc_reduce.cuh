@@ -239,9 +239,12 @@ struct TileOf {
   uint32_t phase;
   bool alone;      // a wait ran out: this thread reduces without the tensor cores
 
-  // Shared: image (16-byte aligned, as long as src), mbar, tmem
+  // Shared: image (16-byte aligned, as long as src), mbar, tmem.  The stream's
+  // next kernel may start from here on; this one continues past open() when
+  // the previous kernel's writes are there (launch_early in pk_common.cuh).
   template <class Shared, int kBlocks>
   __device__ __forceinline__ void open(Shared& sh, const Image<kBlocks>& src) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     image = smem_addr(sh.image);
     mbar = smem_addr(&sh.mbar);
     phase = 0;
@@ -265,6 +268,7 @@ struct TileOf {
     cols = __shfl_sync(0xffffffffu, sh.tmem, 0);
     warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     tmem = cols + (warp << 21);  // lane 32 * warp in bits 16..31
+    asm volatile("griddepcontrol.wait;" ::: "memory");
   }
 
   __device__ __forceinline__ void close() {
