@@ -162,6 +162,51 @@ __device__ __forceinline__ Fr quotient_step(const uint32_t* S) {
   return r;
 }
 
+// a + b + h + top 2^256 mod p in [0, 1.1 p), for a total below 2^15 p (a, b, h: 8
+// words; h may be nullptr).  As quotient_step, but the quotient comes from the
+// top words alone, before the carries below them are known (they add at most 2
+// at word 7, 2^-15 of a unit of S / 2^240), and its multiple of 2^256 - p is
+// accumulated onto a and b, so nothing waits for a sum of all three.
+__device__ __forceinline__ Fr quotient_sum(const uint32_t* a, const uint32_t* b,
+                                           const uint32_t* h, uint32_t top) {
+  constexpr uint32_t kQ = 0x54a47u;
+  constexpr uint32_t N[8] = {0x0fffffffu, 0xbc1e0a6cu, 0x86468f6eu, 0xd7cc17b7u,
+                             0x7e7ea7a2u, 0x47afba49u, 0x1ece5fd6u, 0xcf9bb18du};  // 2^256 - p
+  uint32_t lo, hi;
+  asm("add.cc.u32 %0, %2, %3;\n\t"
+      "addc.u32   %1, %4, 0;"
+      : "=r"(lo), "=r"(hi)
+      : "r"(a[7]), "r"(b[7]), "r"(top));
+  if (h)
+    asm("add.cc.u32 %0, %0, %2;\n\t"
+        "addc.u32   %1, %1, 0;"
+        : "+r"(lo), "+r"(hi)
+        : "r"(h[7]));
+  const uint32_t q = __umulhi(__funnelshift_l(lo, hi, 16), kQ);
+  uint32_t E[8], O[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    E[i] = a[i];
+    O[i] = b[i];
+  }
+  fr_chain4(E, q, N[0], N[2], N[4], N[6]);
+  asm("mad.lo.cc.u32  %0, %7, %8,  %0;\n\t"
+      "madc.hi.cc.u32 %1, %7, %8,  %1;\n\t"
+      "madc.lo.cc.u32 %2, %7, %9,  %2;\n\t"
+      "madc.hi.cc.u32 %3, %7, %9,  %3;\n\t"
+      "madc.lo.cc.u32 %4, %7, %10, %4;\n\t"
+      "madc.hi.cc.u32 %5, %7, %10, %5;\n\t"
+      "madc.lo.u32    %6, %7, %11, %6;"
+      : "+r"(O[1]), "+r"(O[2]), "+r"(O[3]), "+r"(O[4]), "+r"(O[5]), "+r"(O[6]), "+r"(O[7])
+      : "r"(q), "r"(N[1]), "r"(N[3]), "r"(N[5]), "r"(N[7]));
+  Fr e;
+#pragma unroll
+  for (int i = 0; i < 8; i++) e.v[i] = E[i];
+  e = fr_add_raw(e, O);
+  if (h) e = fr_add_raw(e, h);
+  return e;
+}
+
 // Any 256-bit value to [0, 1.1 p).
 __device__ __forceinline__ Fr reduce_any(const Fr& x) {
   uint32_t S[9];

@@ -116,13 +116,9 @@ __device__ __forceinline__ void tile_stages(tc::ProductTile& tile, uint4* sm, bo
       } else {
         const uint64_t high = mode_b ? (l0 + ll) >> log_u : high_a;
         const Fr w = fr_load_ro(roots, (high << s) | (uint64_t)grp);
-        uint32_t S[9];
         tile.start(w, x1);
-        tile.finish(S);
-        if (tile.alone)
-          m = product_alone(w, x1);
-        else
-          m = tc::quotient_step(S);
+        m = tile.finish();
+        if (tile.alone) m = product_alone(w, x1);
         __syncwarp();
       }
       const Fr x0 = tile_load(sm, E, i0);

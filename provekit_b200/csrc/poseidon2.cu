@@ -175,10 +175,9 @@ static __device__ __noinline__ Fr p2_mul_alone(const Fr a, const Fr b) {
 struct P2Tile : tc::TileOf<kP2Columns> {
   // the sum at D columns d as an element below 1.1 p
   __device__ __forceinline__ Fr sum(uint32_t d) const {
-    uint32_t c[32], S[9];
+    uint32_t c[32];
     tc::tmem_ld32(tmem + d, c);
-    tc::assemble(c, S);
-    return tc::quotient_step(S);
+    return tc::columns_reduce(c);
   }
   // x^2 for x < 2^255
   __device__ __forceinline__ Fr square(const Fr& x) {

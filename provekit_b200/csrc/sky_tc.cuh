@@ -98,28 +98,21 @@ __device__ __forceinline__ uint32_t sbox4(uint32_t v) {
 // wait for l).
 __device__ __forceinline__ Fr bar_round(const Fr& l, const Fr& r, int k) {
   const Fr x = fr_reduce_once(l), t = fr_add_raw(r, kSkyRC.w[k]);
-  uint32_t S[9];
+  uint32_t y[8];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    S[i] = sbox4(x.v[i + 4]);
-    S[i + 4] = sbox4(x.v[i]);
+    y[i] = sbox4(x.v[i + 4]);
+    y[i + 4] = sbox4(x.v[i]);
   }
-  S[8] = 0;
-  add9(S, t.v);
-  return quotient_step(S);
+  return quotient_sum(y, t.v, nullptr, 0);
 }
 
-// A square round without the tensor cores (mont_r: r still to be divided by
-// 2^256), taken when the wait below runs out.
-static __device__ __noinline__ Fr square_round_alone(const Fr l, const Fr r, int k, bool mont_r) {
-  const Fr f = fr_sqr(l), c = mont_r ? fr_redc(r.v) : r;
-  uint32_t S[9];
-#pragma unroll
-  for (int i = 0; i < 8; i++) S[i] = f.v[i];
-  S[8] = 0;
-  add9(S, c.v);
-  add9(S, kSkyRC.w[k]);
-  return quotient_step(S);
+// What the tensor cores would hold, without them: l^2 2^-256 + rc of round k,
+// (mont_r) plus r 2^-256; below 3 p.
+static __device__ __noinline__ Fr square_alone(const Fr l, const Fr r, int k, bool mont_r) {
+  Fr f = fr_sqr(l);
+  if (mont_r) f = fr_add(f, fr_from_mont(r));
+  return fr_add_raw(f, kSkyRC.w[k]);
 }
 
 struct SkyTile : Tile {
@@ -159,24 +152,29 @@ struct SkyTile : Tile {
       block(2, kMontR ? 0 : 2);
       if (!kMontR) block(3, 3 + square_index(k));
     });
-    uint32_t c[32], S[9];
+    uint32_t c[32], x[8], z[8], top;
     finish(c);
     if (alone) {
-      const Fr n = square_round_alone(l, r, k, kMontR);
+      const Fr n = square_alone(l, r, k, kMontR);
 #pragma unroll
-      for (int i = 0; i < 8; i++) S[i] = n.v[i];
-      S[8] = 0;
+      for (int i = 0; i < 8; i++) {
+        x[i] = n.v[i];
+        z[i] = 0;
+      }
+      top = 0;
     } else {
-      assemble(c, S);
-      if (!kMontR) add9(S, r.v);
+      assemble(c, x, z, top);
     }
     __syncwarp();
-    if (add_parked) {
-      const uint4 u = park[0], v = park[kThreads];
-      const uint32_t t[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-      add9(S, t);
-    }
-    return quotient_step(S);
+    if (!add_parked) return quotient_sum(x, z, kMontR ? nullptr : r.v, top);
+    uint32_t H[9];
+#pragma unroll
+    for (int i = 0; i < 8; i++) H[i] = r.v[i];
+    H[8] = 0;
+    const uint4 u = park[0], v = park[kThreads];
+    const uint32_t t[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    add9(H, t);
+    return quotient_sum(x, z, H, top + H[8]);
   }
 
   // In place of compress or permute in a warp that has nothing to compress while others of

@@ -107,10 +107,12 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
 // kind::i8: s32 accumulators, unsigned bytes, K-major, N = 32, M = 128
 constexpr uint32_t kInstr = (2u << 4) | ((32u >> 3) << 17) | ((128u >> 4) << 24);
 
-// S = sum c[n] 2^(8n) for columns below 2^23: c[4j] + c[4j+1] 2^8 is below
-// 2^32 and is word j as it is; the other two columns make the same, 16 bits up.
-__device__ __forceinline__ void assemble(const uint32_t* c, uint32_t* S) {
-  uint32_t x[8], y[8], z[9];
+// sum c[n] 2^(8n) = x + z + top 2^256 for columns below 2^23: c[4j] + c[4j+1] 2^8
+// is below 2^32 and is word j of x as it is; the other two columns make the
+// same, 16 bits up, as z.
+__device__ __forceinline__ void assemble(const uint32_t* c, uint32_t* x, uint32_t* z,
+                                         uint32_t& top) {
+  uint32_t y[8];
 #pragma unroll
   for (int j = 0; j < 8; j++) {
     x[j] = c[4 * j] + (c[4 * j + 1] << 8);
@@ -119,21 +121,14 @@ __device__ __forceinline__ void assemble(const uint32_t* c, uint32_t* S) {
   z[0] = y[0] << 16;
 #pragma unroll
   for (int j = 1; j < 8; j++) z[j] = __funnelshift_l(y[j - 1], y[j], 16);
-  z[8] = y[7] >> 16;
-  asm("add.cc.u32  %0, %9,  %17;\n\t"
-      "addc.cc.u32 %1, %10, %18;\n\t"
-      "addc.cc.u32 %2, %11, %19;\n\t"
-      "addc.cc.u32 %3, %12, %20;\n\t"
-      "addc.cc.u32 %4, %13, %21;\n\t"
-      "addc.cc.u32 %5, %14, %22;\n\t"
-      "addc.cc.u32 %6, %15, %23;\n\t"
-      "addc.cc.u32 %7, %16, %24;\n\t"
-      "addc.u32    %8, %25, 0;"
-      : "=r"(S[0]), "=r"(S[1]), "=r"(S[2]), "=r"(S[3]), "=r"(S[4]), "=r"(S[5]), "=r"(S[6]),
-        "=r"(S[7]), "=r"(S[8])
-      : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]),
-        "r"(z[0]), "r"(z[1]), "r"(z[2]), "r"(z[3]), "r"(z[4]), "r"(z[5]), "r"(z[6]), "r"(z[7]),
-        "r"(z[8]));
+  top = y[7] >> 16;
+}
+
+// The element that the columns hold, below 1.1 p.
+__device__ __forceinline__ Fr columns_reduce(const uint32_t* c) {
+  uint32_t x[8], z[8], top;
+  assemble(c, x, z, top);
+  return quotient_sum(x, z, nullptr, top);
 }
 
 __device__ __forceinline__ void tmem_st2(uint32_t t, const uint32_t* v) {
@@ -456,8 +451,8 @@ struct ProductShared {
 };
 
 // Montgomery products through a Tile opened with kProductImage: start() after
-// the operands are known, finish() for the sum S (9 words, below 2^14 p) with
-// S = a b 2^-256 mod p; a < p, b < 2^256.
+// the operands are known, finish() for a b 2^-256 mod p below 1.1 p
+// (meaningless where the thread is alone); any 256-bit a, b.
 struct ProductTile : Tile {
   __device__ __forceinline__ void start(const Fr& a, const Fr& b) {
     put_product(tmem + 32, a, b);
@@ -468,10 +463,10 @@ struct ProductTile : Tile {
       block(3, 3);
     });
   }
-  __device__ __forceinline__ void finish(uint32_t* S) {
+  __device__ __forceinline__ Fr finish() {
     uint32_t c[32];
     Tile::finish(c);
-    assemble(c, S);
+    return columns_reduce(c);
   }
 };
 
