@@ -34,7 +34,7 @@ namespace pk {
 constexpr int kMsgs = 8;         // RS messages per job (folding factor 3)
 constexpr int kLogInvRate = 2;   // rate 1/4
 constexpr int kMaxM0 = 30;
-constexpr int kScThreads = 256;  // sumcheck round CTA size
+constexpr int kScThreads = kQuadThreads;  // sumcheck round CTA size
 constexpr int kScCtaCap = 64;    // CTAs per job per round
 
 struct PassDesc {  // one job's share of one grouped NTT pass
@@ -319,21 +319,14 @@ __global__ void batch_eq_combine_kernel(const RangeDesc* __restrict__ rd,
   }
 }
 
-__device__ __forceinline__ Fr shfl_down_fr(const Fr& x, int off) {
-  Fr r;
-#pragma unroll
-  for (int i = 0; i < 8; i++) r.v[i] = __shfl_down_sync(0xffffffffu, x.v[i], off);
-  return r;
-}
-
 // One sumcheck round for every job with rounds left.  Each CTA belongs to one
 // job (descriptor `count` = pairs q, `begin` = first CTA); per-CTA partial
 // sums of (f0, f(-1), f(inf)) go to the job's partial slots.
-template <bool kFold>
+template <bool kFold, bool kQuads>
 __global__ void __launch_bounds__(kScThreads) batch_sc_round_kernel(
     const RangeDesc* __restrict__ rd, const uint64_t* __restrict__ begins, uint32_t nd,
     const JobDev* __restrict__ jobs, const ScState* __restrict__ st, uint32_t round) {
-  const RangeDesc d = rd[find_desc(begins, nd, blockIdx.x)];
+  const RangeDesc& d = rd[find_desc(begins, nd, blockIdx.x)];
   const JobDev& jb = jobs[d.job];
   const uint64_t size = round == 0 ? jb.n : (jb.n >> (round - 1));  // live table length
   const uint64_t q = kFold ? size / 4 : size / 2;
@@ -342,28 +335,22 @@ __global__ void __launch_bounds__(kScThreads) batch_sc_round_kernel(
   Fr fold = fr_zero();
   if (kFold) fold = st[d.job].alpha[round - 1];
   uint64_t* const tabs[4] = {jb.a, jb.b, jb.c, jb.eq};
-  Fr acc[3] = {fr_zero(), fr_zero(), fr_zero()};
-  for (uint64_t j = (uint64_t)cta * blockDim.x + threadIdx.x; j < q;
-       j += (uint64_t)nctas * blockDim.x)
-    spartan_pair<kFold>(tabs, j, q, fold, acc);
-  __shared__ Fr wsum[kScThreads / 32][3];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-    for (int k = 0; k < 3; k++) acc[k] = fr_add(acc[k], shfl_down_fr(acc[k], off));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < 3; k++) wsum[warp][k] = acc[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    Fr s3[3] = {fr_zero(), fr_zero(), fr_zero()};
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++)
-#pragma unroll
-      for (int k = 0; k < 3; k++) s3[k] = fr_add(s3[k], wsum[w][k]);
-#pragma unroll
-    for (int k = 0; k < 3; k++) fr_store(jb.part, (uint64_t)cta * 3 + k, s3[k]);
+  Fr sums[3] = {fr_zero(), fr_zero(), fr_zero()};
+  if (kQuads) {
+    __shared__ FrShared sh[3];
+    quad_sums(spartan_quads<kFold>(tabs, (size_t)cta * kQuadPairs, (size_t)nctas * kQuadPairs, q,
+                                   fold, sh),
+              sums);
+  } else {
+    for (uint64_t j = (uint64_t)cta * blockDim.x + threadIdx.x; j < q;
+         j += (uint64_t)nctas * blockDim.x)
+      spartan_pair<kFold>(tabs, j, q, fold, sums);
+    __syncwarp();
   }
+  block_sum<3>(sums);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < 3; k++) fr_store(jb.part, (uint64_t)cta * 3 + k, sums[k]);
 }
 
 // Round bookkeeping for every job still running: sum the CTA partials, build
@@ -586,6 +573,14 @@ static int upload_grouped(pkg_batch* b, std::vector<RangeDesc>& v, Grouped& g, u
   return PKG_OK;
 }
 
+// Whether round r, by its largest job, takes four lanes per pair.
+static bool round_quads(const pkg_batch* b, uint32_t r) {
+  uint64_t q = 0;
+  for (const JobDev& jb : b->jobs)
+    if (r < jb.m0) q = std::max<uint64_t>(q, r == 0 ? jb.n / 2 : (jb.n >> (r - 1)) / 4);
+  return q <= kQuadMaxPairs;
+}
+
 // Build every grouped launch's descriptor tables for the current tuning.
 static int batch_plan(pkg_batch* b) {
   const size_t nj = b->jobs.size();
@@ -632,7 +627,8 @@ static int batch_plan(pkg_batch* b) {
       if (r >= jb.m0) continue;
       const uint64_t size = r == 0 ? jb.n : (jb.n >> (r - 1));
       const uint64_t q = r == 0 ? size / 2 : size / 4;
-      uint64_t ctas = std::min<uint64_t>((q + kScThreads - 1) / kScThreads, kScCtaCap);
+      const uint64_t per = round_quads(b, r) ? kQuadPairs : kScThreads;
+      uint64_t ctas = std::min<uint64_t>((q + per - 1) / per, kScCtaCap);
       b->round_ctas[(size_t)r * nj + j] = ctas;
       RangeDesc d = {0, ctas, nullptr, nullptr, (uint32_t)j, 0};
       rd_rounds.back().push_back(d);
@@ -729,12 +725,12 @@ static int enqueue_sumchecks(pkg_batch* b, cudaStream_t s) {
   PK_CHECK_LAUNCH("batch_eq_combine_kernel");
   for (uint32_t r = 0; r < b->max_m0; r++) {
     const Grouped& g = b->rounds[r];
-    if (r == 0)
-      batch_sc_round_kernel<false><<<(unsigned)g.total, kScThreads, 0, s>>>(
-          g.d_desc, g.d_begin, g.n, b->d_jobs, b->d_state, r);
-    else
-      batch_sc_round_kernel<true><<<(unsigned)g.total, kScThreads, 0, s>>>(
-          g.d_desc, g.d_begin, g.n, b->d_jobs, b->d_state, r);
+    const bool quads = round_quads(b, r);
+    const auto kernel =
+        r == 0 ? (quads ? batch_sc_round_kernel<false, true> : batch_sc_round_kernel<false, false>)
+               : (quads ? batch_sc_round_kernel<true, true> : batch_sc_round_kernel<true, false>);
+    kernel<<<(unsigned)g.total, kScThreads, 0, s>>>(g.d_desc, g.d_begin, g.n, b->d_jobs, b->d_state,
+                                                   r);
     PK_CHECK_LAUNCH("batch_sc_round_kernel");
     batch_sc_finish_round_kernel<<<jb_blocks, skytc::kThreads, 0, s>>>(b->d_state, b->d_jobs, nj, r,
                                                           b->d_nctas + (size_t)r * nj);

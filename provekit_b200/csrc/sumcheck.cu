@@ -46,6 +46,18 @@ __global__ void __launch_bounds__(kRedThreads) spartan_round_kernel(Tables4 tabs
   block_finish<3>(acc, ro);
 }
 
+// The same with four lanes per pair.
+template <bool kFold>
+__global__ void __launch_bounds__(kQuadThreads) spartan_quad_kernel(Tables4 tabs, size_t q,
+                                                                     Fr fold, const RedOut ro) {
+  __shared__ FrShared sh[3];
+  Fr sums[3];
+  quad_sums(spartan_quads<kFold>(tabs.t, (size_t)blockIdx.x * kQuadPairs,
+                                 (size_t)gridDim.x * kQuadPairs, q, fold, sh),
+            sums);
+  block_finish<3>(sums, ro);
+}
+
 // eq over a block of variables: out[x] = prod_i (bit_i(x) ? r_i : 1 - r_i)
 // with r_0 on the most significant of nr bits.
 __global__ void eq_small_kernel(const uint64_t* __restrict__ r, int nr, uint64_t* __restrict__ out) {
@@ -236,7 +248,7 @@ __global__ void widen_kernel(const uint32_t* __restrict__ in, size_t n, unsigned
 
 // One Spartan round on device tables; the round kernel writes 3 Fr (f0,
 // f(-1), f(inf)) to out (the thread's fused slots, whose ticket it takes).
-// part: >= red_grid(q) * 3 Fr of scratch.
+// part: >= round_grid(q) * 3 Fr of scratch.
 int spartan_round_device(uint64_t* a, uint64_t* b, uint64_t* c, uint64_t* eq, size_t size,
                          const uint64_t* fold_host, uint64_t* part, uint64_t* out,
                          cudaStream_t s, unsigned* ticket) {
@@ -249,12 +261,18 @@ int spartan_round_device(uint64_t* a, uint64_t* b, uint64_t* c, uint64_t* eq, si
   if (fold_host) {
     memcpy(f.v, fold_host, 32);
     q = size / 4;
-    g = red_grid(q);
-    spartan_round_kernel<true><<<g, kRedThreads, 0, s>>>(tabs, q, f, ro);
+    g = round_grid(q);
+    if (q <= kQuadMaxPairs)
+      spartan_quad_kernel<true><<<g, kQuadThreads, 0, s>>>(tabs, q, f, ro);
+    else
+      spartan_round_kernel<true><<<g, kRedThreads, 0, s>>>(tabs, q, f, ro);
   } else {
     q = size / 2;
-    g = red_grid(q);
-    spartan_round_kernel<false><<<g, kRedThreads, 0, s>>>(tabs, q, f, ro);
+    g = round_grid(q);
+    if (q <= kQuadMaxPairs)
+      spartan_quad_kernel<false><<<g, kQuadThreads, 0, s>>>(tabs, q, f, ro);
+    else
+      spartan_round_kernel<false><<<g, kRedThreads, 0, s>>>(tabs, q, f, ro);
   }
   PK_CHECK_LAUNCH("spartan_round_kernel");
   return PKG_OK;
@@ -666,7 +684,7 @@ extern "C" int pkg_spartan_sumcheck(uint64_t* a, uint64_t* b, uint64_t* c, size_
   }
   // scratch: eq table (n Fr), partials; each round's sums go to the
   // thread's fused slots
-  const int gmax = red_grid(n / 2);
+  const int gmax = std::max(round_grid(n / 2), round_grid(std::min(n / 2, kQuadMaxPairs)));
   FusedSlots fs;
   int rc = fused_slots(&fs);
   if (rc) return rc;

@@ -124,4 +124,79 @@ __device__ __forceinline__ void spartan_pair(uint64_t* const (&tabs)[4], size_t 
   acc[2] = fr_add(acc[2], fr_mul_call(fr_sub(x1, x0), dab));
 }
 
+// Rounds of at most this many pairs take four lanes per pair.  Spartan rounds of
+// 2^12, 2^14, 2^15 and 2^16 pairs: 13, 17, 24 and 36 us, against 22, 23, 23 and
+// 33 with a thread per pair; WHIR rounds of 2^12, 2^14 and 2^15: 10, 12 and 18
+// against 15, 16 and 17.
+constexpr size_t kQuadMaxPairs = size_t(1) << 14;
+
+// Sumcheck rounds with four lanes per pair.  A lane folds one table (Spartan) or
+// one of the four values (WHIR), the quad exchanges what it has through shared
+// memory, and a lane each makes a sum's product: 4 and 2 dependent products
+// where one thread has 14 and 7 (small rounds are bound by that chain).
+constexpr int kQuadThreads = 256;                // 64 pairs at a time
+constexpr int kQuadPairs = kQuadThreads / 4;
+
+struct FrShared {  // a value per thread as two 16-byte halves
+  uint4 lo[kQuadThreads], hi[kQuadThreads];
+  __device__ __forceinline__ void put(int i, const Fr& x) {
+    lo[i] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
+    hi[i] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
+  }
+  __device__ __forceinline__ Fr get(int i) const {
+    const uint4 a = lo[i], b = hi[i];
+    Fr x;
+    x.v[0] = a.x; x.v[1] = a.y; x.v[2] = a.z; x.v[3] = a.w;
+    x.v[4] = b.x; x.v[5] = b.y; x.v[6] = b.z; x.v[7] = b.w;
+    return x;
+  }
+};
+
+// The Spartan closure (whir_r1cs.rs:552-558) over pairs (t[j], t[j + q]) of the
+// tables a, b, c, eq, j = first, first + step, .., as spartan_pair.  Lane k < 3 of
+// a quad returns its share of sum k.  first: the CTA's first pair; all threads
+// of the CTA call it together.
+template <bool kFold>
+__device__ __forceinline__ Fr spartan_quads(uint64_t* const (&tabs)[4], size_t first, size_t step,
+                                            size_t q, const Fr& fold, FrShared (&sh)[3]) {
+  const int lane = threadIdx.x & 3, quad = threadIdx.x & ~3;
+  uint64_t* const t = lane < 2 ? (lane == 0 ? tabs[0] : tabs[1]) : (lane == 2 ? tabs[2] : tabs[3]);
+  Fr acc = fr_zero();
+  for (size_t base = first; base < q; base += step) {
+    const size_t j = base + (threadIdx.x >> 2);
+    if (j < q) {
+      Fr x0 = fr_load(t, j), x1 = fr_load(t, j + q);
+      if (kFold) {
+        const Fr d0 = fr_sub(fr_load(t, j + 2 * q), x0), d1 = fr_sub(fr_load(t, j + 3 * q), x1);
+        x0 = fr_add(x0, fr_mul(fold, d0));
+        x1 = fr_add(x1, fr_mul(fold, d1));
+        fr_store(t, j, x0);
+        fr_store(t, j + q, x1);
+      }
+      sh[0].put(threadIdx.x, x0);
+      sh[1].put(threadIdx.x, fr_sub(fr_add(x0, x0), x1));
+      sh[2].put(threadIdx.x, fr_sub(x1, x0));
+    }
+    __syncwarp();
+    if (j < q && lane < 3) {
+      const FrShared& v = sh[lane];
+      Fr ab = fr_mul(v.get(quad), v.get(quad + 1));
+      if (lane < 2) ab = fr_sub(ab, v.get(quad + 2));
+      acc = fr_add(acc, fr_mul(ab, v.get(quad + 3)));
+    }
+    __syncwarp();
+  }
+  return acc;
+}
+
+// CTAs for a round of q pairs, at most 4 per SM (the partials' room).
+inline int round_grid(size_t q) { return red_grid(q <= kQuadMaxPairs ? 4 * q : q); }
+
+// As three sums for block_sum: lane k < 3 of a quad holds a share of sum k.
+__device__ __forceinline__ void quad_sums(const Fr& acc, Fr (&v)[3]) {
+  const int lane = threadIdx.x & 3;
+#pragma unroll
+  for (int k = 0; k < 3; k++) v[k] = lane == k ? acc : fr_zero();
+}
+
 }  // namespace pk

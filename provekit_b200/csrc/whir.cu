@@ -25,6 +25,7 @@
 #include "internal.cuh"
 #include "pk_common.cuh"
 #include "reduce.cuh"
+#include "sumcheck_device.cuh"
 
 namespace pk {
 
@@ -195,6 +196,43 @@ __global__ void __launch_bounds__(kRedThreads, 2) whir_round_kernel(
     acc[2] = fr_add(acc[2], whir_mul(f2, w2));
   }
   block_finish<3>(acc, ro);
+}
+
+// The same with four lanes per pair (sumcheck_device.cuh).
+template <bool kFold>
+__global__ void __launch_bounds__(kQuadThreads) whir_quad_kernel(
+    uint64_t* __restrict__ f, uint64_t* __restrict__ w, size_t q,
+    const __grid_constant__ FrParams<1> A, const RedOut ro) {
+  __shared__ FrShared sh;
+  const int lane = threadIdx.x & 3, quad = threadIdx.x & ~3;
+  uint64_t* const t = lane < 2 ? f : w;  // f0, f1, w0, w1
+  const Fr alpha = param_fr(A, 0);
+  Fr acc = fr_zero();
+  for (size_t base = (size_t)blockIdx.x * kQuadPairs; base < q;
+       base += (size_t)gridDim.x * kQuadPairs) {
+    const size_t i = base + (threadIdx.x >> 2), at = i + (lane & 1) * q;
+    if (i < q) {
+      Fr x = fr_load(t, at);
+      if (kFold) {
+        x = fr_add(x, fr_mul(alpha, fr_sub(fr_load(t, at + 2 * q), x)));
+        fr_store(t, at, x);
+      }
+      sh.put(threadIdx.x, x);
+    }
+    __syncwarp();
+    if (i < q && lane < 3) {
+      Fr x = sh.get(quad + (lane == 0 ? 0 : 1)), y = sh.get(quad + (lane == 0 ? 2 : 3));
+      if (lane == 2) {
+        x = fr_sub(fr_add(x, x), sh.get(quad));
+        y = fr_sub(fr_add(y, y), sh.get(quad + 2));
+      }
+      acc = fr_add(acc, fr_mul(x, y));
+    }
+    __syncwarp();
+  }
+  Fr sums[3];
+  quad_sums(acc, sums);
+  block_finish<3>(sums, ro);
 }
 
 // tables[j][x] = scale_j * prod_i (bit i of x, top first ? p_j[i] : 1 - p_j[i])
@@ -485,7 +523,7 @@ extern "C" int pkg_whir_sumcheck_round(uint64_t* f, uint64_t* w, size_t size, co
   PK_REQUIRE(f && w && out && aligned16(f) && aligned16(w), "null or unaligned pointer");
   cudaStream_t s = as_stream(stream);
   const size_t q = fold ? size / 4 : size / 2;
-  const int g = red_grid(q);
+  const int g = round_grid(q);
   FusedSlots fs;
   int rc = fused_slots(&fs);
   if (rc) return rc;
@@ -494,10 +532,10 @@ extern "C" int pkg_whir_sumcheck_round(uint64_t* f, uint64_t* w, size_t size, co
   memset(&A, 0, sizeof A);
   if (fold) memcpy(A.v[0], fold, 32);
   const RedOut ro = {part, fs.ticket, fs.dev, fused_next_seq()};
-  if (fold)
-    whir_round_kernel<true><<<g, kRedThreads, 0, s>>>(f, w, q, A, ro);
-  else
-    whir_round_kernel<false><<<g, kRedThreads, 0, s>>>(f, w, q, A, ro);
+  const auto kernel = q <= kQuadMaxPairs ? (fold ? whir_quad_kernel<true> : whir_quad_kernel<false>)
+                                         : (fold ? whir_round_kernel<true> : whir_round_kernel<false>);
+  static_assert(kQuadThreads == kRedThreads, "one CTA size");
+  kernel<<<g, kRedThreads, 0, s>>>(f, w, q, A, ro);
   PK_CHECK_LAUNCH("whir_round_kernel");
   return fused_read(out, fs, 96, s);
 }
