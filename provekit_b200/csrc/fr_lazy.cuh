@@ -1,165 +1,180 @@
-// fr_lazy.cuh -- exact sums of BN254 Fr Montgomery products on the FP64
-// pipe, reduced once per sum.
+// fr_lazy.cuh -- exact sums of products of 256-bit values on the integer pipe,
+// reduced once per sum.
 //
 // A sum S = sum_k a_k b_k of products of Montgomery-form values is needed
-// reduced only once.  The products are accumulated as exact unreduced
-// integers in binary64 columns and one Montgomery reduction follows,
-// instead of one per product (fr_f64.cuh): per term 144 digit products and
-// 24 digit conversions instead of ~350 binary64 instructions.
+// reduced only once: its products are added up as integers, and one Montgomery
+// reduction follows instead of one per product.
 //
-// Digits are 22 bits (12 per operand, 264 >= 256 bits), held as exact
-// doubles:
-//  * a digit product is < 2^44 and a column receives at most 12 of them per
-//    term, so a term adds < 12 * 2^44 < 2^47.6 to a column;
-//  * carry() splits every column into its low 22 bits and the rest and moves
-//    the rest one column up, all columns at once (no ripple): a column is
-//    then < 2^22 + 2^31; kCarryEvery = 32 terms between carries keep every
-//    column below 2^31.1 + 32 * 2^47.6 < 2^52.6 < 2^53, so every fma is exact;
-//  * finish() ripples the carries into 24 exact 22-bit digits of T = S and
-//    divides by 2^264 in twelve Montgomery steps: p = 1 mod 2^28 makes
-//    -p^-1 = -1 mod 2^22, so the step's digit for the low column T_s is
-//    (-T_s) mod 2^22, read off a round-up add of 2^74 (ulp 2^22), and
-//    T_s + q = u carries u / 2^22 up.  The quotient V = (T + Q p) / 2^264 <
-//    T / 2^264 + p; with every operand < p, T < K p^2 for K terms, and V <
-//    (K p / 2^264 + 1) p < 2p for K <= kMaxTerms (p / 2^264 < 1 / 1354), so
-//    one conditional subtraction finishes.
-// The result is S * 2^-264 mod p: callers fold the missing 2^8 into an
-// operand (a coefficient times 2^8) or multiply the result by kMont2e8
-// (2^8 in Montgomery form) with one Montgomery product.
-// Every constant is a power of two or a 22-bit digit of p; nothing depends
-// on the rounding of an inexact operation.
+// The words a_i b_j of a product are added to two accumulators, those with i + j
+// even to one and the rest to the other, so that each product and its addition
+// is one 64-bit multiply-add onto an aligned pair.  The products with the same
+// i - j lie two words apart, so they form one carry chain; a chain ends above the
+// highest word that it wrote, and the carry out of it is counted in a word of its
+// own instead of running on to the top.  A term is 64 multiply-adds and 15
+// counts, 256 cycles of the multiplier per warp: half of a Montgomery product,
+// and half of the 144 binary64 digit products and 24 conversions per term that
+// stood here before.  Alone a term takes 310 cycles.
 #pragma once
-#include "fr.cuh"
+#include "fr_sum.cuh"
 
 namespace pk {
 namespace lazy {
 
-constexpr int kD = 12;           // 22-bit digits per operand
-constexpr int kCols = 24;        // product columns 0..22, carry column 23
-constexpr int kCarryEvery = 32;  // terms between carry() calls
-constexpr int kMaxTerms = 1024;  // terms per finish() (operands < p)
+constexpr int kMaxTerms = 1024;  // terms per finish(): the sum is below 2^15 p 2^256
 
-constexpr double kTwo52 = 4503599627370496.0;         // 2^52
-constexpr double kTwo74 = 18889465931478580854784.0;  // 2^74 (ulp 2^22)
-constexpr double kInv22 = 1.0 / 4194304.0;            // 2^-22
-
-// 2^8 in Montgomery form (2^264 mod p), 64-bit limbs
-constexpr uint64_t kMont2e8[4] = {0xf6e31f8c9ffffab6ULL, 0x5d7570ac31329faeULL,
-                                  0x276f48b709e2a349ULL, 0x0d791464ef86e357ULL};
-
-// p in 22-bit digits, least significant first (digit 0 is 1).
-__device__ __forceinline__ double pdig(int j) {
-  constexpr double P[kD] = {1.0,       1462208.0, 1326623.0, 3038244.0, 2639993.0, 3449039.0,
-                            1578373.0, 1142176.0, 2734160.0, 312960.0,  321326.0,  3097.0};
-  return P[j];
-}
-
-__device__ __forceinline__ double dbl(uint32_t v) {
-  return __hiloint2double(0x43300000, (int)v) - kTwo52;
-}
-
-// the twelve 22-bit digits of a 256-bit value, least significant first
-__device__ __forceinline__ void digits(const Fr& a, double* A) {
-  const uint32_t M = 0x3FFFFFu;
-  A[0] = dbl(a.v[0] & M);                                 // bits   0..21
-  A[1] = dbl(__funnelshift_r(a.v[0], a.v[1], 22) & M);   // bits  22..43
-  A[2] = dbl(__funnelshift_r(a.v[1], a.v[2], 12) & M);   // bits  44..65
-  A[3] = dbl(__funnelshift_r(a.v[2], a.v[3], 2) & M);    // bits  66..87
-  A[4] = dbl(__funnelshift_r(a.v[2], a.v[3], 24) & M);   // bits  88..109
-  A[5] = dbl(__funnelshift_r(a.v[3], a.v[4], 14) & M);   // bits 110..131
-  A[6] = dbl(__funnelshift_r(a.v[4], a.v[5], 4) & M);    // bits 132..153
-  A[7] = dbl(__funnelshift_r(a.v[4], a.v[5], 26) & M);   // bits 154..175
-  A[8] = dbl(__funnelshift_r(a.v[5], a.v[6], 16) & M);   // bits 176..197
-  A[9] = dbl(__funnelshift_r(a.v[6], a.v[7], 6) & M);    // bits 198..219
-  A[10] = dbl(__funnelshift_r(a.v[6], a.v[7], 28) & M);  // bits 220..241
-  A[11] = dbl(a.v[7] >> 18);                              // bits 242..255
-}
+// One multiply-add of a chain onto the pair (l, h); the first one starts the carry.
+#define PK_FIRST(l, h, a, b) "mad.lo.cc.u32 " l "," a "," b "," l ";\n\tmadc.hi.cc.u32 " h "," a "," b "," h ";\n\t"
+#define PK_NEXT(l, h, a, b) "madc.lo.cc.u32 " l "," a "," b "," l ";\n\tmadc.hi.cc.u32 " h "," a "," b "," h ";\n\t"
+#define PK_COUNT(c) "addc.u32 " c "," c ",0;\n\t"
 
 struct Acc {
-  double c[kCols];
+  uint32_t e[16];  // words 0..15
+  uint32_t o[14];  // words 1..14
+  uint32_t c[8];   // carries into words 9..16
 
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int i = 0; i < kCols; i++) c[i] = 0.0;
+    for (int i = 0; i < 16; i++) e[i] = 0;
+#pragma unroll
+    for (int i = 0; i < 14; i++) o[i] = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) c[i] = 0;
   }
 
-  // c += A * B (digit forms)
-  __device__ __forceinline__ void mac(const double* A, const double* B) {
-#pragma unroll
-    for (int i = 0; i < kD; i++)
-#pragma unroll
-      for (int j = 0; j < kD; j++) c[i + j] = fma(A[i], B[j], c[i + j]);
-  }
-
+  // += a b, for any 256-bit a and b
   __device__ __forceinline__ void mac(const Fr& a, const Fr& b) {
-    double A[kD], B[kD];
-    digits(a, A);
-    digits(b, B);
-    mac(A, B);
+    asm(
+        PK_FIRST("%0", "%1", "%20", "%28")
+        PK_NEXT("%2", "%3", "%21", "%29")
+        PK_NEXT("%4", "%5", "%22", "%30")
+        PK_NEXT("%6", "%7", "%23", "%31")
+        PK_NEXT("%8", "%9", "%24", "%32")
+        PK_NEXT("%10", "%11", "%25", "%33")
+        PK_NEXT("%12", "%13", "%26", "%34")
+        PK_NEXT("%14", "%15", "%27", "%35")
+        PK_COUNT("%19")
+        PK_FIRST("%2", "%3", "%22", "%28")
+        PK_NEXT("%4", "%5", "%23", "%29")
+        PK_NEXT("%6", "%7", "%24", "%30")
+        PK_NEXT("%8", "%9", "%25", "%31")
+        PK_NEXT("%10", "%11", "%26", "%32")
+        PK_NEXT("%12", "%13", "%27", "%33")
+        PK_COUNT("%18")
+        PK_FIRST("%2", "%3", "%20", "%30")
+        PK_NEXT("%4", "%5", "%21", "%31")
+        PK_NEXT("%6", "%7", "%22", "%32")
+        PK_NEXT("%8", "%9", "%23", "%33")
+        PK_NEXT("%10", "%11", "%24", "%34")
+        PK_NEXT("%12", "%13", "%25", "%35")
+        PK_COUNT("%18")
+        PK_FIRST("%4", "%5", "%24", "%28")
+        PK_NEXT("%6", "%7", "%25", "%29")
+        PK_NEXT("%8", "%9", "%26", "%30")
+        PK_NEXT("%10", "%11", "%27", "%31")
+        PK_COUNT("%17")
+        PK_FIRST("%4", "%5", "%20", "%32")
+        PK_NEXT("%6", "%7", "%21", "%33")
+        PK_NEXT("%8", "%9", "%22", "%34")
+        PK_NEXT("%10", "%11", "%23", "%35")
+        PK_COUNT("%17")
+        PK_FIRST("%6", "%7", "%26", "%28")
+        PK_NEXT("%8", "%9", "%27", "%29")
+        PK_COUNT("%16")
+        PK_FIRST("%6", "%7", "%20", "%34")
+        PK_NEXT("%8", "%9", "%21", "%35")
+        PK_COUNT("%16")
+        : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]),
+          "+r"(e[7]), "+r"(e[8]), "+r"(e[9]), "+r"(e[10]), "+r"(e[11]), "+r"(e[12]),
+          "+r"(e[13]), "+r"(e[14]), "+r"(e[15]), "+r"(c[1]), "+r"(c[3]), "+r"(c[5]),
+          "+r"(c[7])
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]),
+          "r"(a.v[6]), "r"(a.v[7]), "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]),
+          "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+    asm(
+        PK_FIRST("%0", "%1", "%19", "%26")
+        PK_NEXT("%2", "%3", "%20", "%27")
+        PK_NEXT("%4", "%5", "%21", "%28")
+        PK_NEXT("%6", "%7", "%22", "%29")
+        PK_NEXT("%8", "%9", "%23", "%30")
+        PK_NEXT("%10", "%11", "%24", "%31")
+        PK_NEXT("%12", "%13", "%25", "%32")
+        PK_COUNT("%17")
+        PK_FIRST("%0", "%1", "%18", "%27")
+        PK_NEXT("%2", "%3", "%19", "%28")
+        PK_NEXT("%4", "%5", "%20", "%29")
+        PK_NEXT("%6", "%7", "%21", "%30")
+        PK_NEXT("%8", "%9", "%22", "%31")
+        PK_NEXT("%10", "%11", "%23", "%32")
+        PK_NEXT("%12", "%13", "%24", "%33")
+        PK_COUNT("%17")
+        PK_FIRST("%2", "%3", "%21", "%26")
+        PK_NEXT("%4", "%5", "%22", "%27")
+        PK_NEXT("%6", "%7", "%23", "%28")
+        PK_NEXT("%8", "%9", "%24", "%29")
+        PK_NEXT("%10", "%11", "%25", "%30")
+        PK_COUNT("%16")
+        PK_FIRST("%2", "%3", "%18", "%29")
+        PK_NEXT("%4", "%5", "%19", "%30")
+        PK_NEXT("%6", "%7", "%20", "%31")
+        PK_NEXT("%8", "%9", "%21", "%32")
+        PK_NEXT("%10", "%11", "%22", "%33")
+        PK_COUNT("%16")
+        PK_FIRST("%4", "%5", "%23", "%26")
+        PK_NEXT("%6", "%7", "%24", "%27")
+        PK_NEXT("%8", "%9", "%25", "%28")
+        PK_COUNT("%15")
+        PK_FIRST("%4", "%5", "%18", "%31")
+        PK_NEXT("%6", "%7", "%19", "%32")
+        PK_NEXT("%8", "%9", "%20", "%33")
+        PK_COUNT("%15")
+        PK_FIRST("%6", "%7", "%25", "%26")
+        PK_COUNT("%14")
+        PK_FIRST("%6", "%7", "%18", "%33")
+        PK_COUNT("%14")
+        : "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]),
+          "+r"(o[7]), "+r"(o[8]), "+r"(o[9]), "+r"(o[10]), "+r"(o[11]), "+r"(o[12]),
+          "+r"(o[13]), "+r"(c[0]), "+r"(c[2]), "+r"(c[4]), "+r"(c[6])
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]),
+          "r"(a.v[6]), "r"(a.v[7]), "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]),
+          "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
   }
 
-  // every column to its low 22 bits plus the carry of the column below
-  __device__ __forceinline__ void carry() {
-    double hi[kCols];
-#pragma unroll
-    for (int i = 0; i < kCols; i++) {
-      const double w = __dadd_rz(c[i], kTwo74) - kTwo74;  // floor(c / 2^22) * 2^22
-      hi[i] = w * kInv22;
-      c[i] -= w;
-    }
-#pragma unroll
-    for (int i = 1; i < kCols; i++) c[i] += hi[i - 1];
-  }
-
-  // sum * 2^-264 mod p, fully reduced (at most kMaxTerms terms, operands < p)
+  // sum * 2^-256 mod p, fully reduced
   __device__ __forceinline__ Fr finish() const {
-    double T[kCols];
-    double x = 0.0;
-#pragma unroll
-    for (int i = 0; i < kCols; i++) {  // exact 22-bit digits (ripple)
-      x += c[i];
-      const double w = __dadd_rz(x, kTwo74) - kTwo74;
-      T[i] = x - w;
-      x = w * kInv22;
-    }
-#pragma unroll
-    for (int s = 0; s < kD; s++) {  // twelve 22-bit Montgomery steps
-      const double u = __dadd_ru(T[s], kTwo74) - kTwo74;
-      const double q = u - T[s];
-      T[s + 1] = fma(u, kInv22, T[s + 1]);
-#pragma unroll
-      for (int j = 1; j < kD; j++) T[s + j] = fma(q, pdig(j), T[s + j]);
-    }
-    // V = T[12..23] < 2p < 2^255 as exact 22-bit digits, then 32-bit limbs
-    uint32_t d[kD];
-    x = 0.0;
-#pragma unroll
-    for (int i = 0; i < kD; i++) {
-      x += T[kD + i];
-      const double w = __dadd_rz(x, kTwo74) - kTwo74;
-      d[i] = (uint32_t)__double2loint((x - w) + kTwo52);
-      x = w * kInv22;
-    }
-    Fr r;
-    r.v[0] = d[0] | (d[1] << 22);
-    r.v[1] = (d[1] >> 10) | (d[2] << 12);
-    r.v[2] = (d[2] >> 20) | (d[3] << 2) | (d[4] << 24);
-    r.v[3] = (d[4] >> 8) | (d[5] << 14);
-    r.v[4] = (d[5] >> 18) | (d[6] << 4) | (d[7] << 26);
-    r.v[5] = (d[7] >> 6) | (d[8] << 16);
-    r.v[6] = (d[8] >> 16) | (d[9] << 6) | (d[10] << 28);
-    r.v[7] = (d[10] >> 4) | (d[11] << 18);
-    return fr_reduce_once(r);
+    uint32_t t[17];
+    t[0] = e[0];
+    asm("add.cc.u32  %0, %9,  %17;\n\t"
+        "addc.cc.u32 %1, %10, %18;\n\t"
+        "addc.cc.u32 %2, %11, %19;\n\t"
+        "addc.cc.u32 %3, %12, %20;\n\t"
+        "addc.cc.u32 %4, %13, %21;\n\t"
+        "addc.cc.u32 %5, %14, %22;\n\t"
+        "addc.cc.u32 %6, %15, %23;\n\t"
+        "addc.cc.u32 %7, %16, %24;\n\t"
+        "addc.u32    %8, 0, 0;"
+        : "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]),
+          "=r"(t[8]), "=r"(t[9])
+        : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(e[8]),
+          "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]));
+    // words 8..16: e and o with the carry of the words below, then the counts
+    uint32_t h[9] = {t[8], e[9], e[10], e[11], e[12], e[13], e[14], e[15], 0};
+    const uint32_t up[8] = {0, o[8], o[9], o[10], o[11], o[12], o[13], 0};
+    const uint32_t carry[8] = {0, t[9], 0, 0, 0, 0, 0, 0};
+    tc::add9(h, up);
+    tc::add9(h, carry);
+    const uint32_t low[8] = {0, c[0], c[1], c[2], c[3], c[4], c[5], c[6]};
+    tc::add9(h, low);
+    h[8] += c[7];
+    // (low words + M p) / 2^256 <= p, then S / 2^256 < 2^15 p by one quotient step
+    const Fr r = fr_redc(t);
+    tc::add9(h, r.v);
+    return fr_reduce_once(tc::quotient_step(h));
   }
 };
 
-// kMont2e8 as device 32-bit limbs
-__device__ __forceinline__ Fr mont_2e8() {
-  Fr r;
-  r.v[0] = 0x9ffffab6u; r.v[1] = 0xf6e31f8cu; r.v[2] = 0x31329faeu; r.v[3] = 0x5d7570acu;
-  r.v[4] = 0x09e2a349u; r.v[5] = 0x276f48b7u; r.v[6] = 0xef86e357u; r.v[7] = 0x0d791464u;
-  return r;
-}
+#undef PK_FIRST
+#undef PK_NEXT
+#undef PK_COUNT
 
 }  // namespace lazy
 }  // namespace pk

@@ -185,29 +185,24 @@ __global__ void hadamard_pad_kernel(const uint64_t* __restrict__ a, const uint64
     fr_store(c, i, i < n ? fr_mul(fr_load_ro(a, i), fr_load_ro(b, i)) : fr_zero());
 }
 
-// The products are summed unreduced (fr_lazy.cuh) and reduced once per
-// thread; each CTA's sum is then scaled by 2^8 (the lazy reduction divides
-// by 2^264 where a Montgomery product divides by 2^256).
-__global__ void __launch_bounds__(kRedThreads) dot_kernel(const uint64_t* __restrict__ a,
-                                                        const uint64_t* __restrict__ b, size_t n,
-                                                        const RedOut ro) {
+// The products are summed unreduced (fr_lazy.cuh) and reduced once per thread.
+__global__ void __launch_bounds__(kRedThreads, 2) dot_kernel(const uint64_t* __restrict__ a,
+                                                             const uint64_t* __restrict__ b,
+                                                             size_t n, const RedOut ro) {
   Fr acc[1] = {fr_zero()};
-  lazy::Acc la;
-  la.zero();
-  int terms = 0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    la.mac(fr_load_ro(a, i), fr_load_ro(b, i));
-    if (++terms % lazy::kCarryEvery == 0) la.carry();
-    if (terms == lazy::kMaxTerms) {
-      acc[0] = fr_add(acc[0], la.finish());
-      la.zero();
-      terms = 0;
-    }
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+#pragma unroll 1
+  while (i < n) {
+    const size_t left = (n - i + step - 1) / step;
+    const int terms = left < (size_t)lazy::kMaxTerms ? (int)left : lazy::kMaxTerms;
+    lazy::Acc la;
+    la.zero();
+#pragma unroll 2
+    for (int k = 0; k < terms; k++, i += step) la.mac(fr_load_ro(a, i), fr_load_ro(b, i));
+    acc[0] = fr_add(acc[0], la.finish());
   }
-  if (terms) acc[0] = fr_add(acc[0], la.finish());
-  const Fr s8 = lazy::mont_2e8();
-  block_finish<1>(acc, ro, &s8);
+  block_finish<1>(acc, ro);
 }
 
 // ---- CSR transpose: count, exclusive scan, scatter ------------------------
@@ -371,8 +366,8 @@ static int read_err_flag(uint32_t* d_err, cudaStream_t s, const char* what) {
 int dot_device(const uint64_t* a, const uint64_t* b, size_t n, uint64_t* out, uint64_t* part,
                cudaStream_t s, unsigned* ticket) {
   PK_REQUIRE(ticket && out, "dot_device needs the thread's fused slots");
-  dot_kernel<<<red_grid(n), kRedThreads, 0, s>>>(a, b, n,
-                                                 RedOut{part, ticket, out, fused_next_seq()});
+  const int grid = std::min(red_grid(n), 2 * sm_count());  // resident at once
+  dot_kernel<<<grid, kRedThreads, 0, s>>>(a, b, n, RedOut{part, ticket, out, fused_next_seq()});
   PK_CHECK_LAUNCH("dot_kernel");
   return PKG_OK;
 }

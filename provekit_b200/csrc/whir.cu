@@ -68,9 +68,10 @@ __global__ void whir_fold_coeffs_kernel(const uint64_t* __restrict__ c, size_t L
                                         uint64_t* __restrict__ out) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < L;
        i += (size_t)gridDim.x * blockDim.x) {
-    Fr acc = fr_load_ro(c, i);
-    for (int j = 1; j < m; j++) acc = fr_add(acc, fr_mul(param_fr(W, j), fr_load_ro(c, j * L + i)));
-    fr_store(out, i, acc);
+    lazy::Acc acc;
+    acc.zero();
+    for (int j = 1; j < m; j++) acc.mac(param_fr(W, j), fr_load_ro(c, j * L + i));
+    fr_store(out, i, fr_add(fr_load_ro(c, i), acc.finish()));
   }
 }
 
@@ -80,10 +81,10 @@ __global__ void whir_fold_rows_kernel(const uint64_t* __restrict__ rows, size_t 
                                       uint64_t* __restrict__ out) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nrows;
        i += (size_t)gridDim.x * blockDim.x) {
-    Fr acc = fr_load_ro(rows, i * m);
-    for (int j = 1; j < m; j++)
-      acc = fr_add(acc, fr_mul(param_fr(W, j), fr_load_ro(rows, i * m + j)));
-    fr_store(out, i, acc);
+    lazy::Acc acc;
+    acc.zero();
+    for (int j = 1; j < m; j++) acc.mac(param_fr(W, j), fr_load_ro(rows, i * m + j));
+    fr_store(out, i, fr_add(fr_load_ro(rows, i * m), acc.finish()));
   }
 }
 
@@ -269,60 +270,65 @@ __global__ void expand_points_kernel(const uint64_t* __restrict__ raw, size_t np
   }
 }
 
-// w[b] += sum_j hi_j[b >> nlo] lo_j[b & (2^nlo - 1)]
-__global__ void eq_accumulate_kernel(uint64_t* __restrict__ w, size_t n, int nlo,
-                                     const uint64_t* __restrict__ hi, size_t nhi_entries,
-                                     const uint64_t* __restrict__ lo, size_t npts) {
-  const size_t nlo_entries = size_t(1) << nlo;
-  for (size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x; b < n;
-       b += (size_t)gridDim.x * blockDim.x) {
-    // two independent products per step
-    const size_t bh = b >> nlo, bl = b & (nlo_entries - 1);
-    Fr acc = fr_load(w, b), acc2 = fr_zero();
-    size_t j = 0;
-    for (; j + 1 < npts; j += 2) {
-      acc = fr_add(acc, fr_mul(fr_load_ro(hi, j * nhi_entries + bh),
-                                   fr_load_ro(lo, j * nlo_entries + bl)));
-      acc2 = fr_add(acc2, fr_mul(fr_load_ro(hi, (j + 1) * nhi_entries + bh),
-                                 fr_load_ro(lo, (j + 1) * nlo_entries + bl)));
-    }
-    if (j < npts)
-      acc = fr_add(acc, fr_mul(fr_load_ro(hi, j * nhi_entries + bh),
-                                   fr_load_ro(lo, j * nlo_entries + bl)));
-    fr_store(w, b, fr_add(acc, acc2));
-  }
-}
-
-// The same sum with the products accumulated unreduced (fr_lazy.cuh) and
-// reduced once per chunk of lazy::kMaxTerms points: the hi tables carry the
-// coefficients times 2^8, which the lazy reduction's 2^-264 takes back to
-// a Montgomery product's 2^-256.
-__global__ void __launch_bounds__(128, 4) eq_accumulate_lazy_kernel(
+// w[b] += sum_j hi_j[b >> nlo] lo_j[b & (2^nlo - 1)], the products of an entry
+// summed unreduced (fr_lazy.cuh).  2^split threads share an entry's points, so that
+// a short table still fills the chip; those of one entry lie 256 / 2^split apart,
+// and a warp's loads stay in line.  Bound by the multiplier (256 cycles per warp
+// and point): 2^18 entries of 118 points 446 us with binary64 sums, 283 now; 2^14 of
+// 40 32 -> 12, 2^21 of two (a product each before) 115 -> 82.
+constexpr int kEqThreads = 128;
+__global__ void __launch_bounds__(kEqThreads, 4) eq_accumulate_kernel(
     uint64_t* __restrict__ w, size_t n, int nlo, const uint64_t* __restrict__ hi,
-    size_t nhi_entries, const uint64_t* __restrict__ lo, size_t npts) {
+    size_t nhi_entries, const uint64_t* __restrict__ lo, size_t npts, int split) {
+  __shared__ FrShared sh;
   const size_t nlo_entries = size_t(1) << nlo;
-  for (size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x; b < n;
-       b += (size_t)gridDim.x * blockDim.x) {
-    const size_t bh = b >> nlo, bl = b & (nlo_entries - 1);
-    Fr sum = fr_load(w, b);
-    for (size_t j0 = 0; j0 < npts; j0 += lazy::kMaxTerms) {
-      const size_t j1 = npts - j0 < (size_t)lazy::kMaxTerms ? npts : j0 + lazy::kMaxTerms;
+  const unsigned per = kEqThreads >> split, part = threadIdx.x / per;
+  const size_t b = blockIdx.x * (size_t)per + threadIdx.x % per;
+  Fr sum = fr_zero();
+  if (b < n) {
+    const size_t bh = b >> nlo, bl = b & (nlo_entries - 1), step = size_t(1) << split;
+    size_t j = part;
+#pragma unroll 1
+    while (j < npts) {
+      const size_t left = (npts - j + step - 1) >> split;
+      const int terms = left < (size_t)lazy::kMaxTerms ? (int)left : lazy::kMaxTerms;
       lazy::Acc acc;
       acc.zero();
-#pragma unroll 1
-      for (size_t j = j0; j < j1; j++) {
+#pragma unroll 2
+      for (int i = 0; i < terms; i++, j += step)
         acc.mac(fr_load_ro(hi, j * nhi_entries + bh), fr_load_ro(lo, j * nlo_entries + bl));
-        if ((j - j0) % lazy::kCarryEvery == lazy::kCarryEvery - 1) acc.carry();
-      }
       sum = fr_add(sum, acc.finish());
     }
-    fr_store(w, b, sum);
   }
+  if (split) {
+    sh.put(threadIdx.x, sum);
+    __syncthreads();
+    if (part) return;
+#pragma unroll 1
+    for (unsigned k = per; k < kEqThreads; k += per) sum = fr_add(sum, sh.get(threadIdx.x + k));
+  }
+  if (b < n) fr_store(w, b, fr_add(fr_load(w, b), sum));
 }
 
-// Points at and above which the lazy sum is cheaper than a product per term
-// (its one reduction per entry costs about a product).
-constexpr size_t kLazyEqMinPoints = 4;
+// Threads per entry: the number (at least kEqMinPoints points each) with the least
+// waves of CTAs times products per thread, the reduction of its sum counted as two.
+// 2^18 entries of 118 points: one thread 288 us (3.5 waves), two 283; 2^14 entries of
+// 40: one 21.8, four 12.4.
+constexpr size_t kEqMinPoints = 8;
+static int eq_split(size_t n, size_t npts) {
+  const size_t resident = 4 * (size_t)sm_count();
+  size_t best = 0;
+  int split = 0;
+  for (int k = 0; k <= 3 && (k == 0 || (npts >> k) >= kEqMinPoints); k++) {
+    const size_t per = kEqThreads >> k, ctas = (n + per - 1) / per;
+    const size_t cost = (ctas + resident - 1) / resident * ((npts >> k) + 2);
+    if (k == 0 || cost < best) {
+      best = cost;
+      split = k;
+    }
+  }
+  return split;
+}
 
 }  // namespace pk
 
@@ -563,31 +569,17 @@ int eq_accumulate_device(uint64_t* w, size_t nv, const uint64_t* points, const u
     expand_points_kernel<<<ew_grid(npts), 256, 0, s>>>(d_raw, npts, nv, d_pts);
     PK_CHECK_LAUNCH("expand_points_kernel");
   }
-  // hi tables carry the coefficient (times 2^8 for the lazy sum), lo tables
-  // are plain eq tables
-  const bool use_lazy = npts >= kLazyEqMinPoints;
-  if (use_lazy) {
-    // pageable: staged before cudaMemcpyAsync returns
-    std::vector<HostFr> cf8(npts);
-    const HostFr m8 = HostFr::from_limbs(lazy::kMont2e8);
-    for (size_t j = 0; j < npts; j++) cf8[j] = HostFr::mul(HostFr::from_limbs(coeffs + 4 * j), m8);
-    PK_CUDA(cudaMemcpyAsync(d_cf, cf8[0].l, 32 * npts, cudaMemcpyHostToDevice, s));
-  } else {
-    PK_CUDA(cudaMemcpyAsync(d_cf, coeffs, 32 * npts, cudaMemcpyHostToDevice, s));
-  }
+  // hi tables carry the coefficient, lo tables are plain eq tables
+  PK_CUDA(cudaMemcpyAsync(d_cf, coeffs, 32 * npts, cudaMemcpyHostToDevice, s));
   eq_tables_kernel<<<ew_grid(npts * nh), 256, 0, s>>>(d_pts, nv, 0, nhi, d_cf, npts, d_hi);
   PK_CHECK_LAUNCH("eq_tables_kernel");
   eq_tables_kernel<<<ew_grid(npts * nl), 256, 0, s>>>(d_pts, nv, nhi, nlo, nullptr, npts, d_lo);
   PK_CHECK_LAUNCH("eq_tables_kernel");
-  if (use_lazy) {
-    const int grid = (int)std::max<size_t>(
-        1, std::min<size_t>((n + 127) / 128, (size_t)sm_count() * 4 * 8));
-    eq_accumulate_lazy_kernel<<<grid, 128, 0, s>>>(w, n, nlo, d_hi, nh, d_lo, npts);
-    PK_CHECK_LAUNCH("eq_accumulate_lazy_kernel");
-  } else {
-    eq_accumulate_kernel<<<ew_grid(n), 256, 0, s>>>(w, n, nlo, d_hi, nh, d_lo, npts);
-    PK_CHECK_LAUNCH("eq_accumulate_kernel");
-  }
+  const int split = eq_split(n, npts);
+  const size_t per = kEqThreads >> split;
+  eq_accumulate_kernel<<<(unsigned)((n + per - 1) / per), kEqThreads, 0, s>>>(w, n, nlo, d_hi, nh,
+                                                                             d_lo, npts, split);
+  PK_CHECK_LAUNCH("eq_accumulate_kernel");
   // host sources in pinned memory must outlive their async copies; pageable
   // ones are staged before cudaMemcpyAsync returns
   if (sync) PK_CUDA(cudaStreamSynchronize(s));
