@@ -37,75 +37,104 @@ static_assert(sizeof(HostFr) == 32, "vectors of HostFr are arrays of 4 x u64 lim
 
 // ---- subset transforms ----------------------------------------------------
 // Zeta: v[b | 2^i] += v[b]; mobius^T: v[b] -= v[b | 2^i], over every index
-// bit i.  A pass covers bits [lo, lo + nb): each CTA stages a tile of 2^nb
+// bit i.  A pass covers bits [lo, lo + nb): each CTA takes a tile of 2^nb
 // rows (those bits) x 2^logw consecutive indices (the low bits, for
-// coalesced 32-byte runs) in shared memory as two planes of 16-byte halves,
-// runs its nb stages of additions there and writes the tile back.  The
-// transform is memory-bound, so the pass count is what costs: a tile of
-// kSubsetTile entries takes 10 bits in the first pass and 7 in each later
-// one (21 bits: 3 passes).
+// coalesced 32-byte runs): 10 bits in the first pass and up to 7 in each later one
+// (21 bits: 3 passes).  A thread adds over two bits of four entries at a time:
+// the top two from global memory, the next pairs through shared memory (two
+// planes of 16-byte halves), and the last step writes the tile back.  With one
+// bit per step a pass of 2^21 entries took 58 us (first) and 43 us, bound by
+// shared memory and barriers; with two 34 and 29 us (moving 128 MB: 20).
 constexpr int kSubsetLogTile = 10;
 constexpr int kSubsetTile = 1 << kSubsetLogTile;  // Fr per CTA (32 KiB)
-constexpr int kSubsetLogW = 3;                    // 8 consecutive indices after the first pass
+constexpr int kSubsetLogW = 3;                    // at least 8 consecutive indices after the first pass
+constexpr int kSubsetThreads = kSubsetTile / 4;
 
-__device__ __forceinline__ Fr tile_load(const uint4* t0, const uint4* t1, int e) {
-  const uint4 a = t0[e], b = t1[e];
-  Fr r;
-  r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w;
-  r.v[4] = b.x; r.v[5] = b.y; r.v[6] = b.z; r.v[7] = b.w;
-  return r;
+// Where entry e lies, so that the eight threads of a 128-byte access meet eight
+// different 16-byte columns whichever two bits of e the access leaves out.
+__device__ __forceinline__ int subset_slot(int e) {
+  return e ^ ((e >> 3) & 1) ^ (((e >> 4) & 1) * 6);
 }
 
-__device__ __forceinline__ void tile_store(uint4* t0, uint4* t1, int e, const Fr& x) {
-  t0[e] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-  t1[e] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
+struct SubsetTile {
+  uint4 lo[kSubsetTile], hi[kSubsetTile];
+};
+
+// Over bit b of e, and with kPair over bit b + 1 as well.
+template <bool kZeta, bool kPair>
+__device__ __forceinline__ void subset_step(SubsetTile& tile, uint64_t* v, size_t base, int lo,
+                                            int logw, int E, int b, bool first, bool last) {
+  constexpr int kN = kPair ? 4 : 2;
+  const int low = (1 << b) - 1;
+  for (int g = threadIdx.x; g < E / kN; g += kSubsetThreads) {
+    const int e0 = ((g & ~low) * kN) | (g & low);
+    Fr x[kN];
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+      const int e = e0 | (i << b);
+      if (first) {
+        x[i] = fr_load(v, base + ((size_t)(e >> logw) << lo) + (e & ((1 << logw) - 1)));
+      } else {
+        const uint4 p = tile.lo[subset_slot(e)], q = tile.hi[subset_slot(e)];
+        x[i].v[0] = p.x; x[i].v[1] = p.y; x[i].v[2] = p.z; x[i].v[3] = p.w;
+        x[i].v[4] = q.x; x[i].v[5] = q.y; x[i].v[6] = q.z; x[i].v[7] = q.w;
+      }
+    }
+#pragma unroll
+    for (int d = 1; d < kN; d *= 2)
+#pragma unroll
+      for (int i = 0; i < kN; i++)
+        if (!(i & d)) {
+          if (kZeta)
+            x[i | d] = fr_add(x[i | d], x[i]);
+          else
+            x[i] = fr_sub(x[i], x[i | d]);
+        }
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+      const int e = e0 | (i << b);
+      if (last) {
+        fr_store(v, base + ((size_t)(e >> logw) << lo) + (e & ((1 << logw) - 1)), x[i]);
+      } else {
+        tile.lo[subset_slot(e)] = make_uint4(x[i].v[0], x[i].v[1], x[i].v[2], x[i].v[3]);
+        tile.hi[subset_slot(e)] = make_uint4(x[i].v[4], x[i].v[5], x[i].v[6], x[i].v[7]);
+      }
+    }
+  }
+  __syncthreads();
 }
 
 template <bool kZeta>
-__global__ void __launch_bounds__(256) subset_tile_kernel(uint64_t* __restrict__ v, int lo, int nb,
-                                                          int logw) {
-  __shared__ uint4 t0[kSubsetTile], t1[kSubsetTile];
-  const int E = 1 << (nb + logw), W = 1 << logw;
-  // this CTA: a block of W low indices (of 2^(lo - logw)) and a high part
+__global__ void __launch_bounds__(kSubsetThreads, 4) subset_tile_kernel(uint64_t* __restrict__ v,
+                                                                        int lo, int nb, int logw) {
+  __shared__ SubsetTile tile;
+  const int E = 1 << (nb + logw);
+  // this CTA: a block of 2^logw low indices (of 2^(lo - logw)) and a high part
   const size_t lblocks_log = (size_t)(lo - logw);
   const size_t lb = blockIdx.x & ((size_t(1) << lblocks_log) - 1);
   const size_t hi = (size_t)blockIdx.x >> lblocks_log;
   const size_t base = (hi << (lo + nb)) | (lb << logw);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    const uint4* q = reinterpret_cast<const uint4*>(
-        v + 4 * (base + ((size_t)(e >> logw) << lo) + (e & (W - 1))));
-    t0[e] = q[0];
-    t1[e] = q[1];
+  if (nb == 1) {
+    subset_step<kZeta, false>(tile, v, base, lo, logw, E, logw, true, true);
+    return;
   }
-  __syncthreads();
+  // bits [logw, top) remain after the first step: pairs, then one if it is left
+  const int top = logw + nb - 2;
+  subset_step<kZeta, true>(tile, v, base, lo, logw, E, top, true, nb == 2);
+  int b = logw;
 #pragma unroll 1
-  for (int b = 0; b < nb; b++) {
-    for (int p = threadIdx.x; p < E / 2; p += blockDim.x) {
-      const int c = p & (W - 1), rp = p >> logw;
-      const int r = ((rp >> b) << (b + 1)) | (rp & ((1 << b) - 1));  // row with bit b clear
-      const int e0 = (r << logw) | c, e1 = ((r | (1 << b)) << logw) | c;
-      const Fr x0 = tile_load(t0, t1, e0), x1 = tile_load(t0, t1, e1);
-      if (kZeta)
-        tile_store(t0, t1, e1, fr_add(x1, x0));
-      else
-        tile_store(t0, t1, e0, fr_sub(x0, x1));
-    }
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    uint4* q = reinterpret_cast<uint4*>(v + 4 * (base + ((size_t)(e >> logw) << lo) + (e & (W - 1))));
-    q[0] = t0[e];
-    q[1] = t1[e];
-  }
+  for (; b + 2 <= top; b += 2)
+    subset_step<kZeta, true>(tile, v, base, lo, logw, E, b, false, b + 2 == top);
+  if (b < top) subset_step<kZeta, false>(tile, v, base, lo, logw, E, b, false, true);
 }
 
 template <bool kZeta>
 static int subset_transform_device(uint64_t* v, unsigned n, cudaStream_t s) {
   for (unsigned lo = 0; lo < n;) {
-    const int logw = lo == 0 ? 0 : (int)std::min<unsigned>(lo, kSubsetLogW);
-    const int nb = (int)std::min<unsigned>(kSubsetLogTile - logw, n - lo);
+    const int nb = (int)std::min<unsigned>(lo ? kSubsetLogTile - kSubsetLogW : kSubsetLogTile, n - lo);
+    const int logw = (int)std::min<unsigned>(lo, kSubsetLogTile - nb);  // whole tiles
     const size_t ctas = size_t(1) << (n - nb - logw);
-    subset_tile_kernel<kZeta><<<(unsigned)ctas, 256, 0, s>>>(v, (int)lo, nb, logw);
+    subset_tile_kernel<kZeta><<<(unsigned)ctas, kSubsetThreads, 0, s>>>(v, (int)lo, nb, logw);
     PK_CHECK_LAUNCH("subset_tile_kernel");
     lo += nb;
   }
