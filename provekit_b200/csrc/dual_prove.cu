@@ -253,15 +253,13 @@ extern "C" int pkg_dual_prove_finish(pkg_dual_prove* st, const uint64_t* w2, pkg
 
   // witness bounds over the whole witness and the zk sumcheck with w1's
   // blinding (prove_noir, whir_r1cs.rs:143-187)
-  const size_t nparts = 4 * (size_t)sm_count();
   Scratch s_tab, s_misc, s_eq, s_alph, s_st;
   if ((rc = s_tab.alloc(32 * 3 * n0, s))) return rc;
-  if ((rc = s_misc.alloc(256 + 32 * nparts, s))) return rc;
+  if ((rc = s_misc.alloc(256, s))) return rc;
   uint64_t* ta = static_cast<uint64_t*>(s_tab.ptr);
   uint64_t* tb = ta + 4 * n0;
   uint64_t* tc = tb + 4 * n0;
   uint32_t* err = static_cast<uint32_t*>(s_misc.ptr);
-  uint64_t* part = reinterpret_cast<uint64_t*>(static_cast<uint8_t*>(s_misc.ptr) + 256);
   PK_CUDA(cudaMemsetAsync(err, 0, 4, s));
   if ((rc = witness_bounds_device(r1cs, st->witness, n0, ta, tb, tc, err, s))) return rc;
   rc = pkg_spartan_sumcheck(ta, tb, tc, m0, st->g.data(), st->g.data(), &st->t, &sp->r[0][0],
@@ -323,6 +321,7 @@ extern "C" int pkg_dual_prove_finish(pkg_dual_prove* st, const uint64_t* w2, pkg
   const bool cached = r1cs->row_ptr_t[0] && r1cs->row_ptr_t[1] && r1cs->row_ptr_t[2];
   FusedSlots fs;
   if ((rc = fused_slots(&fs))) return rc;
+  DotJob jobs[kMaxDots];
   for (int k = 0; k < 3; k++) {
     Scratch s_t;
     const uint64_t* rp_t = r1cs->row_ptr_t[k];
@@ -352,13 +351,12 @@ extern "C" int pkg_dual_prove_finish(pkg_dual_prove* st, const uint64_t* w2, pkg
     if (w2_size)
       PK_CUDA(cudaMemcpyAsync(a2, alph + 4 * w1_size, 32 * w2_size, cudaMemcpyDeviceToDevice, s));
     // compute_alpha_evals (prefix_covector.rs:212-223) on each part
-    if ((rc = dot_device(a1, st->poly[0], w1_size, fs.dev + 4 * k, part, s, fs.ticket))) return rc;
-    if ((rc = dot_device(a2, st->poly[1], w2_size, fs.dev + 4 * (3 + k), part, s, fs.ticket)))
-      return rc;
+    jobs[k] = {a1, st->poly[0], w1_size};
+    jobs[3 + k] = {a2, st->poly[1], w2_size};
   }
-  if (nchal &&  // compute_challenge_eval (prefix_covector.rs:326-338) on w2
-      (rc = dot_device(st2 + 4 * 3 * n, st->poly[1], n, fs.dev + 4 * 6, part, s, fs.ticket)))
-    return rc;
+  // compute_challenge_eval (prefix_covector.rs:326-338) on w2
+  if (nchal) jobs[6] = {st2 + 4 * 3 * n, st->poly[1], n};
+  if ((rc = dots_device(jobs, nchal ? 7 : 6, fs.dev, fs, s))) return rc;
   uint64_t sums[7][4];
   if ((rc = fused_read(sums, fs, 32 * (nchal ? 7 : 6), s))) return rc;
   memcpy(sp->evals, sums, 96);

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "../../include/provekit_b200.h"
+#include "pk_common.cuh"
 
 namespace pk {
 
@@ -38,10 +39,16 @@ int eq_accumulate_device(uint64_t* w, size_t nv, const uint64_t* points, const u
 int open_rows_device(const uint64_t* codeword, size_t fr_per_row, size_t num_rows,
                      const uint8_t* layers, const uint64_t* indices, size_t nq, uint64_t* rows,
                      uint8_t* paths, cudaStream_t s, bool sync = true);
-// <a, b> to out, a slot of the thread's fused slots (FusedSlots: out within
-// dev, ticket its ticket), in one launch; part: red_grid(n) Fr of scratch.
-int dot_device(const uint64_t* a, const uint64_t* b, size_t n, uint64_t* out, uint64_t* part,
-               cudaStream_t s, unsigned* ticket);
+// Up to kMaxDots dot products <a, b> of n entries each in one launch; their values go
+// to out, out + 4, .., slots of the thread's fused slots fs (out within fs.dev).
+constexpr int kMaxDots = 8;
+struct DotJob {
+  const uint64_t* a;
+  const uint64_t* b;
+  size_t n;
+};
+int dots_device(const DotJob* jobs, int count, uint64_t* out, const FusedSlots& fs,
+                cudaStream_t s);
 
 // The WHIR prover's round loop (pkg_whir_prove); values (host, ncov Fr) are
 // the statements' values when the caller already has them, else nullptr;

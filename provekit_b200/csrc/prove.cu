@@ -190,12 +190,8 @@ static int spartan_prove_impl(const pkg_r1cs* r1cs, const uint64_t* witness,
   clk.mark(0);
 
   // ---- witness bounds (sumcheck.rs:163-179)
-  // partial sums of dot_device (<= 4 * SMs CTAs); its results go to the
-  // thread's fused slots
-  const size_t nparts = 4 * (size_t)sm_count();
-  if ((rc = s_misc.alloc(256 + 32 * nparts, s))) return rc;
+  if ((rc = s_misc.alloc(256, s))) return rc;
   uint32_t* err = static_cast<uint32_t*>(s_misc.ptr);
-  uint64_t* part = reinterpret_cast<uint64_t*>(static_cast<uint8_t*>(s_misc.ptr) + 256);
   PK_CUDA(cudaMemsetAsync(err, 0, 4, s));
   // a = A w, b = B w, c = a o b, zero-padded to 2^m0: one launch
   if ((rc = witness_bounds_device(r1cs, witness, n0, ta, tb, tc, err, s))) return rc;
@@ -273,28 +269,44 @@ static int spartan_prove_impl(const pkg_r1cs* r1cs, const uint64_t* witness,
     }
     if ((rc = spmv_device(rp_t, cl_t, vl_t, nw, nc, eq, alph, err, s, r1cs->nnz[k]))) return rc;
     // create_weights_and_evaluations (:623-642): the zero padding adds nothing
-    if ((rc = dot_device(alph, poly, nw, fs.dev + 4 * k, part, s, fs.ticket))) return rc;
+    if (!whir) {
+      const DotJob job = {alph, poly, nw};
+      if ((rc = dots_device(&job, 1, fs.dev + 4 * k, fs, s))) return rc;
+    }
   }
-  // the three evaluations read back at once, then absorbed in order
-  if ((rc = fused_read(&out->evals[0][0], fs, 96, s))) return rc;
+  // the public weight and the blinding covector expand_powers::<4>(alpha)
+  // at the blinding offset (OffsetCovector, prefix_covector.rs:90-112)
+  std::vector<uint64_t> xpow(4 * (np + 1)), bw(16 * m0);
+  if (np) public_weight_host(pubw.data(), np, out->public_x, xpow.data(), out->public_eval);
+  // the dot products with w, and for whir-ZK every statement's value on the
+  // blinding polynomial g (over the entries where its covector is not zero)
+  uint64_t sums[kMaxDots][4];
+  int ndots = 3;
+  if (whir) {
+    if (np)
+      PK_CUDA(cudaMemcpyAsync(cov, xpow.data(), 32 * (np + 1), cudaMemcpyHostToDevice, s));
+    blinding_weights_host(&out->alpha[0][0], m0, bw.data());
+    uint64_t* blind = cov + 4 * n * (sbase + 3) + 4 * w1_size;
+    PK_CUDA(cudaMemcpyAsync(blind, bw.data(), 32 * 4 * m0, cudaMemcpyHostToDevice, s));
+    DotJob jobs[kMaxDots];
+    for (size_t k = 0; k < 3; k++) jobs[k] = {cov + 4 * n * (sbase + k), poly, nw};
+    if (nb == 2) {
+      if (np) jobs[ndots++] = {cov, mask, np + 1};
+      for (size_t k = 0; k < 3; k++) jobs[ndots++] = {cov + 4 * n * (sbase + k), mask, nw};
+      jobs[ndots++] = {blind, mask + 4 * w1_size, 4 * m0};
+    }
+    // host sources above are pageable: staged before the copies returned
+    if ((rc = dots_device(jobs, ndots, fs.dev, fs, s))) return rc;
+  }
+  // read back at once, then absorbed in order
+  if ((rc = fused_read(sums, fs, 32 * (size_t)ndots, s))) return rc;
+  memcpy(out->evals, sums, 96);
   for (int k = 0; k < 3; k++) pkg_transcript_absorb(&out->transcript, out->evals[k]);
   // the public weight's evaluation <[1, x, .., x^np], w> and its message
   // (compute_public_weight_evaluation, :654-663, :275-282)
-  std::vector<uint64_t> xpow(4 * (np + 1));
-  if (np) {
-    public_weight_host(pubw.data(), np, out->public_x, xpow.data(), out->public_eval);
-    pkg_transcript_absorb(&out->transcript, out->public_eval);
-  }
+  if (np) pkg_transcript_absorb(&out->transcript, out->public_eval);
   clk.mark(4);
   if (whir) {
-    // the public weight and the blinding covector expand_powers::<4>(alpha)
-    // at the blinding offset (OffsetCovector, prefix_covector.rs:90-112)
-    if (np)
-      PK_CUDA(cudaMemcpyAsync(cov, xpow.data(), 32 * (np + 1), cudaMemcpyHostToDevice, s));
-    std::vector<uint64_t> bw(16 * m0);
-    blinding_weights_host(&out->alpha[0][0], m0, bw.data());
-    PK_CUDA(cudaMemcpyAsync(cov + 4 * n * (sbase + 3) + 4 * w1_size, bw.data(), 32 * 4 * m0,
-                            cudaMemcpyHostToDevice, s));
     // statement values of w: [public_eval?, evals, blinding_eval]; for
     // whir-ZK also every statement's value on the blinding polynomial g
     std::vector<uint64_t> vals(4 * nstm * nb);
@@ -305,11 +317,7 @@ static int spartan_prove_impl(const pkg_r1cs* r1cs, const uint64_t* witness,
     }
     memcpy(vals.data() + at, &out->evals[0][0], 96);
     memcpy(vals.data() + at + 12, out->blinding_eval, 32);
-    for (size_t k = 0; nb == 2 && k < nstm; k++)
-      if ((rc = dot_device(cov + 4 * n * k, mask, n, fs.dev + 4 * k, part, s, fs.ticket)))
-        return rc;
-    if (nb == 2 && (rc = fused_read(vals.data() + 4 * nstm, fs, 32 * nstm, s))) return rc;
-    // host sources above are pageable: staged before the copies returned
+    if (nb == 2) memcpy(vals.data() + 4 * nstm, sums[3], 32 * nstm);
     pkg_transcript tw = out->transcript;
     if ((rc = whir_prove_device(whir, &tw, poly, cw, layers, ood_points, cov, nstm, vals.data(),
                                 nullptr, whir_proof, s)))
