@@ -236,37 +236,85 @@ __global__ void __launch_bounds__(kQuadThreads) whir_quad_kernel(
   block_finish<3>(sums, ro);
 }
 
-// tables[j][x] = scale_j * prod_i (bit i of x, top first ? p_j[i] : 1 - p_j[i])
-// over k variables; p_j = pts + 4 (j * stride + first).
-__global__ void eq_tables_kernel(const uint64_t* __restrict__ pts, size_t stride, size_t first,
-                                 int k, const uint64_t* __restrict__ scale, size_t npts,
-                                 uint64_t* __restrict__ tables) {
-  const size_t per = size_t(1) << k;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < npts * per;
-       t += (size_t)gridDim.x * blockDim.x) {
-    const size_t j = t / per, x = t % per;
-    Fr acc = scale ? fr_load_ro(scale, j) : fr_one_mont();
-    for (int i = 0; i < k; i++) {
-      const Fr p = fr_load_ro(pts, j * stride + first + i);
-      const bool bit = (x >> (k - 1 - i)) & 1;
-      acc = fr_mul(acc, bit ? p : fr_sub(fr_one_mont(), p));
-    }
-    fr_store(tables, t, acc);
+// The equality tables of a point (p_0, .., p_nv-1), the top variable first: entry x of
+// a run of variables is prod_i (bit i of x ? p_i : 1 - p_i), over the first nhi
+// variables times the point's coefficient (hi) and over the rest (lo).
+// in: npts coefficients, then the points, each nv coordinates (expanded) or one z
+// for p_nv-1-i = z^(2^i) (ExpandFromUnivariate,
+// recursive-verifier/app/utilities/utilities.go:183-191).
+// A row of CTAs per point.  An entry is one product of two entries of tables over half
+// of its variables each, which a CTA builds first: bound by the chain of nv squarings
+// and about eight products.  With a launch each for the squarings, the hi and the lo
+// tables, and a product per variable, 119 points of 18 variables took 38 us
+// and one 30; now 15 and 16.
+constexpr int kEqSub = 8;  // variables per half: all of them up to nv = 32
+constexpr int kEqMaxVars = 40;
+
+struct EqHalves {  // of k variables: the first `rest` one by one, then a, then b
+  int rest, a, b;
+  __device__ __forceinline__ explicit EqHalves(int k) {
+    a = (k + 1) / 2 < kEqSub ? (k + 1) / 2 : kEqSub;
+    b = k - a < kEqSub ? k - a : kEqSub;
+    rest = k - a - b;
   }
+};
+
+__device__ __forceinline__ Fr eq_factor(const Fr& p, bool bit) {
+  return bit ? p : fr_sub(fr_one_mont(), p);
 }
 
-// out[j nv + nv - 1 - i] = z_j^(2^i): the expansion of each univariate point
-// into nv coordinates, the top variable first (ExpandFromUnivariate,
-// recursive-verifier/app/utilities/utilities.go:183-191).
-__global__ void expand_points_kernel(const uint64_t* __restrict__ raw, size_t npts, size_t nv,
-                                     uint64_t* __restrict__ out) {
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < npts;
-       j += (size_t)gridDim.x * blockDim.x) {
-    Fr acc = fr_load_ro(raw, j);
-    for (size_t i = 0; i < nv; i++) {
-      fr_store(out, j * nv + nv - 1 - i, acc);
-      acc = fr_sqr(acc);
+__global__ void __launch_bounds__(256) eq_tables_kernel(const uint64_t* __restrict__ in,
+                                                        size_t npts, int nv, bool expanded,
+                                                        int nhi, uint64_t* __restrict__ hi,
+                                                        uint64_t* __restrict__ lo) {
+  __shared__ Fr p[kEqMaxVars], sub[4 << kEqSub];
+  const size_t j = blockIdx.x;
+  if (expanded) {
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) p[i] = fr_load_ro(in, npts + j * nv + i);
+  } else if (threadIdx.x == 0 && nv) {
+    Fr z = fr_load_ro(in, npts + j);
+    for (int i = nv - 1; i > 0; i--) {
+      p[i] = z;
+      z = fr_sqr(z);
     }
+    p[0] = z;
+  }
+  __syncthreads();
+  const EqHalves h(nhi), l(nv - nhi);
+  // the halves: hi's a and b, then lo's
+  const int end0 = 1 << h.a, end1 = end0 + (1 << h.b), end2 = end1 + (1 << l.a),
+            end3 = end2 + (1 << l.b);
+  for (int t = threadIdx.x; t < end3; t += blockDim.x) {
+    int x = t, first = h.rest, k = h.a;
+    if (t >= end2) {
+      x = t - end2, first = nhi + l.rest + l.a, k = l.b;
+    } else if (t >= end1) {
+      x = t - end1, first = nhi + l.rest, k = l.a;
+    } else if (t >= end0) {
+      x = t - end0, first = h.rest + h.a, k = h.b;
+    }
+    Fr acc = t < end0 ? fr_load_ro(in, j) : fr_one_mont();
+    if (k && t >= end0) {
+      acc = eq_factor(p[first], (x >> (k - 1)) & 1);
+      first++, k--;
+    }
+#pragma unroll 1
+    for (; k > 0; first++, k--) acc = fr_mul(acc, eq_factor(p[first], (x >> (k - 1)) & 1));
+    sub[t] = acc;
+  }
+  __syncthreads();
+  const size_t nh = size_t(1) << nhi, nl = size_t(1) << (nv - nhi);
+  for (size_t e = blockIdx.y * (size_t)blockDim.x + threadIdx.x; e < nh + nl;
+       e += (size_t)gridDim.y * blockDim.x) {
+    const bool high = e < nh;
+    const size_t x = high ? e : e - nh;
+    const EqHalves& s = high ? h : l;
+    Fr v = fr_mul(sub[(high ? 0 : end1) + ((x >> s.b) & ((1 << s.a) - 1))],
+                  sub[(high ? end0 : end2) + (x & ((1 << s.b) - 1))]);
+#pragma unroll 1
+    for (int i = 0; i < s.rest; i++)
+      v = fr_mul(v, eq_factor(p[(high ? 0 : nhi) + i], (x >> (s.a + s.b + s.rest - 1 - i)) & 1));
+    fr_store(high ? hi : lo, j * (high ? nh : nl) + x, v);
   }
 }
 
@@ -553,35 +601,28 @@ int eq_accumulate_device(uint64_t* w, size_t nv, const uint64_t* points, const u
   const int nhi = (int)(nv + 1) / 2, nlo = (int)nv - nhi;
   const size_t nh = size_t(1) << nhi, nl = size_t(1) << nlo, n = size_t(1) << nv;
   Scratch scr;
-  const size_t pts_fr = npts * (nv ? nv : 1);
-  // [expanded points | coefficients | hi tables | lo tables | raw points]
-  int rc = scr.alloc(32 * (pts_fr + npts + npts * (nh + nl) + (expanded ? 0 : npts)), s);
+  // [coefficients | points | hi tables | lo tables], the first two in one copy
+  const size_t pts_fr = nv == 0 ? 0 : expanded ? npts * nv : npts, in_fr = npts + pts_fr;
+  int rc = scr.alloc(32 * (in_fr + npts * (nh + nl)), s);
   if (rc) return rc;
-  uint64_t* d_pts = static_cast<uint64_t*>(scr.ptr);
-  uint64_t* d_cf = d_pts + 4 * pts_fr;
-  uint64_t* d_hi = d_cf + 4 * npts;
+  uint64_t* d_in = static_cast<uint64_t*>(scr.ptr);
+  uint64_t* d_hi = d_in + 4 * in_fr;
   uint64_t* d_lo = d_hi + 4 * npts * nh;
-  if (nv && expanded) {
-    PK_CUDA(cudaMemcpyAsync(d_pts, points, 32 * npts * nv, cudaMemcpyHostToDevice, s));
-  } else if (nv) {
-    uint64_t* d_raw = d_lo + 4 * npts * nl;
-    PK_CUDA(cudaMemcpyAsync(d_raw, points, 32 * npts, cudaMemcpyHostToDevice, s));
-    expand_points_kernel<<<ew_grid(npts), 256, 0, s>>>(d_raw, npts, nv, d_pts);
-    PK_CHECK_LAUNCH("expand_points_kernel");
-  }
-  // hi tables carry the coefficient, lo tables are plain eq tables
-  PK_CUDA(cudaMemcpyAsync(d_cf, coeffs, 32 * npts, cudaMemcpyHostToDevice, s));
-  eq_tables_kernel<<<ew_grid(npts * nh), 256, 0, s>>>(d_pts, nv, 0, nhi, d_cf, npts, d_hi);
-  PK_CHECK_LAUNCH("eq_tables_kernel");
-  eq_tables_kernel<<<ew_grid(npts * nl), 256, 0, s>>>(d_pts, nv, nhi, nlo, nullptr, npts, d_lo);
+  std::vector<uint64_t> in(4 * in_fr);
+  memcpy(in.data(), coeffs, 32 * npts);
+  if (pts_fr) memcpy(in.data() + 4 * npts, points, 32 * pts_fr);
+  // pageable: staged before the copy returns
+  PK_CUDA(cudaMemcpyAsync(d_in, in.data(), 32 * in_fr, cudaMemcpyHostToDevice, s));
+  PK_REQUIRE(npts < (size_t(1) << 31), "too many points (%zu)", npts);
+  const size_t rows = std::min<size_t>((nh + nl + 1023) / 1024, 65535);
+  eq_tables_kernel<<<dim3((unsigned)npts, (unsigned)rows), 256, 0, s>>>(d_in, npts, (int)nv,
+                                                                        expanded, nhi, d_hi, d_lo);
   PK_CHECK_LAUNCH("eq_tables_kernel");
   const int split = eq_split(n, npts);
   const size_t per = kEqThreads >> split;
   eq_accumulate_kernel<<<(unsigned)((n + per - 1) / per), kEqThreads, 0, s>>>(w, n, nlo, d_hi, nh,
                                                                              d_lo, npts, split);
   PK_CHECK_LAUNCH("eq_accumulate_kernel");
-  // host sources in pinned memory must outlive their async copies; pageable
-  // ones are staged before cudaMemcpyAsync returns
   if (sync) PK_CUDA(cudaStreamSynchronize(s));
   return PKG_OK;
 }

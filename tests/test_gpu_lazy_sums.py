@@ -43,3 +43,16 @@ def test_fold_of_largest_values(k):
     alpha = np.broadcast_to(np.array(to_limbs(P - 1), np.uint64), (max(k, 1), 4)).copy()
     got = fold_coeffs(dev(c), k, alpha).cpu().numpy().view(np.uint64)
     assert np.array_equal(got.reshape(-1, 4), O.whir_fold_coeffs(c, k, alpha))
+
+
+@pytest.mark.parametrize("nv,npts", [(0, 3), (1, 2), (2, 5), (3, 1), (7, 9), (12, 3), (19, 2)])
+def test_equality_tables(nv, npts):
+    """Halves of every length from none, points as coordinates (a proof's univariate
+    points are expanded in the same kernel: whole proofs)."""
+    w = O.sample_fr(70 + nv, 1 << nv)
+    pts, cf = O.sample_fr(71 + nv, max(npts * nv, 1)), O.sample_fr(72, npts)
+    pts[0] = np.array(to_limbs(P - 1), np.uint64)
+    dw = dev(w)
+    eq_accumulate(dw, nv, pts, cf)
+    assert O.lib().pko_eq_accumulate(O.p64(w), nv, O.p64(pts), O.p64(cf), npts) == 0
+    assert np.array_equal(dw.cpu().numpy().view(np.uint64), w)
