@@ -248,6 +248,8 @@ int fused_slots(FusedSlots* f) {
     cudaError_t e = cudaStreamCreateWithFlags(&z, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
       e = cudaMemsetAsync(t, 0, 256, z);
+      if (e == cudaSuccess)  // the PoW word: no nonce
+        e = cudaMemsetAsync(static_cast<uint8_t*>(t) + bytes - 256, 0xff, 8, z);
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(static_cast<uint8_t*>(t) + 8, &word_dev, sizeof word_dev,
                             cudaMemcpyHostToDevice, z);

@@ -20,6 +20,7 @@
 #include "host_stage.cuh"
 #include "internal.cuh"
 #include "pk_common.cuh"
+#include "reduce.cuh"
 #include "rs_internal.cuh"
 #include "skyscraper.cuh"
 #include "sky_tc.cuh"
@@ -283,24 +284,47 @@ int merkle_tree_fr_device(const uint64_t* cw, size_t fr_per_leaf, size_t num_lea
 }
 
 // ---- PoW -----------------------------------------------------------------
-__global__ void pow_kernel(Fr challenge, Fr threshold, uint64_t base, uint64_t n,
-                           unsigned long long* best) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t nonce = base + i;
-    Fr r = fr_zero();
-    r.v[0] = (uint32_t)nonce;
-    r.v[1] = (uint32_t)(nonce >> 32);
-    Fr h = sky_compress(challenge, r);
-    bool lt = false;
+// Candidate nonces base + 128 b .. base + 128 b + 127 in CTA b; kTile: as a tile
+// (sky_tc.cuh).
+// The CTA that takes the last ticket hands the smallest solution so far to the host
+// (reduce.cuh's completion word) and leaves the ticket and *best as they were found.
+template <bool kTile>
+__global__ void __launch_bounds__(skytc::kThreads, kTile ? 8 : 1)
+    pow_kernel(Fr challenge, Fr threshold, uint64_t base, unsigned long long* best, RedOut ro) {
+  const uint64_t nonce = base + blockIdx.x * (uint64_t)skytc::kThreads + threadIdx.x;
+  Fr r = fr_zero();
+  r.v[0] = (uint32_t)nonce;
+  r.v[1] = (uint32_t)(nonce >> 32);
+  Fr h;
+  if constexpr (kTile) {
+    __shared__ skytc::Shared sh;
+    skytc::SkyTile tile;
+    tile.open(sh);
+    h = fr_reduce_once(tile.compress<false>(skytc::reduce_any(challenge), r));
+    tile.close();
+  } else {
+    h = sky_compress(challenge, r);
+  }
+  bool lt = false;
 #pragma unroll
-    for (int k = 7; k >= 0; k--) {  // less_than, arithmetic.rs:447-456
-      if (h.v[k] != threshold.v[k]) {
-        lt = h.v[k] < threshold.v[k];
-        break;
-      }
+  for (int k = 7; k >= 0; k--) {  // less_than, arithmetic.rs:447-456
+    if (h.v[k] != threshold.v[k]) {
+      lt = h.v[k] < threshold.v[k];
+      break;
     }
-    if (lt) atomicMin(best, (unsigned long long)nonce);
+  }
+  if (lt) atomicMin(best, (unsigned long long)nonce);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(ro.ticket, 1u) == gridDim.x - 1) {
+      __threadfence();
+      *reinterpret_cast<volatile unsigned long long*>(ro.out) = atomicExch(best, ~0ULL);
+      *ro.ticket = 0u;
+      volatile unsigned* word = *reinterpret_cast<unsigned* const*>(ro.ticket + 2);
+      __threadfence_system();  // the nonce before the completion word
+      *word = ro.seq;
+    }
   }
 }
 
@@ -316,23 +340,28 @@ int pow_solve_device(const uint64_t challenge[4], const uint64_t threshold[4], c
   bool thr_zero = true;
   for (int i = 0; i < 8; i++) thr_zero &= (t.v[i] == 0);
   PK_REQUIRE(!thr_zero, "threshold 0 admits no nonce");
-  // the best nonce in the thread's own PoW word (after the fused
-  // reductions' partials, which it never overlaps): no pool allocation per PoW
+  // the best nonce in the thread's own PoW word (all ones between searches; after
+  // the fused reductions' partials, which it never overlaps): no pool allocation per PoW
   FusedSlots fs;
   int rc = fused_slots(&fs);
   if (rc) return rc;
-  unsigned long long* d_best = fs.pow;
-  PK_CUDA(cudaMemsetAsync(d_best, 0xff, sizeof(unsigned long long), s));
   const unsigned long long none = ~0ULL;
   unsigned long long best = none;
   const uint64_t max_batch = uint64_t(1) << 22;
   uint64_t batch = uint64_t(1) << 13;
   for (uint64_t base = 0; best == none; base += batch, batch = std::min(batch * 4, max_batch)) {
     if (base > (uint64_t(1) << 62)) break;
-    const int grid = (int)std::min<uint64_t>((uint64_t)sm_count() * 8, (batch + 255) / 256);
-    pow_kernel<<<grid, 256, 0, s>>>(c, t, base, batch, d_best);
+    // the first batch is one compression's latency either way, and a tile's constants
+    // and tensor memory cost more than it saves (proofs 2 us longer per search); a
+    // 20-bit search takes 793 us without tiles and 483 with
+    const unsigned grid = (unsigned)(batch / skytc::kThreads);
+    const RedOut ro = {fs.part, fs.ticket, fs.dev, fused_next_seq()};
+    if (base == 0)
+      pow_kernel<false><<<grid, skytc::kThreads, 0, s>>>(c, t, base, fs.pow, ro);
+    else
+      PK_CUDA(launch_early(pow_kernel<true>, grid, skytc::kThreads, 0, s, c, t, base, fs.pow, ro));
     PK_CHECK_LAUNCH("pow_kernel");
-    if ((rc = read_small(&best, d_best, sizeof best, s))) return rc;
+    if ((rc = fused_read(&best, fs, sizeof best, s))) return rc;
   }
   if (best == none) {
     set_last_error("no nonce found");
