@@ -50,6 +50,11 @@ struct DotJob {
 int dots_device(const DotJob* jobs, int count, uint64_t* out, const FusedSlots& fs,
                 cudaStream_t s);
 
+// out[i npts + j] = polynomial i (n >= 1 coefficients, stride entries apart) at point j;
+// points and out: host.  Synchronous.
+int poly_eval_device(const uint64_t* coeffs, size_t n, size_t stride, size_t polys,
+                     const uint64_t* points, size_t npts, uint64_t* out, cudaStream_t s);
+
 // The WHIR prover's round loop (pkg_whir_prove); values (host, ncov Fr) are
 // the statements' values when the caller already has them, else nullptr;
 // hat (device, 2^n Fr, overwritten) is zeta(coeffs) when the caller already

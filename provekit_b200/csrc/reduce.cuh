@@ -105,23 +105,21 @@ __device__ __forceinline__ void block_sum(Fr (&v)[K]) {
   }
 }
 
-// Where a reduction kernel's CTAs leave their sums.  part: one partial per
-// CTA (K Fr each), summed by sum_partials_kernel.  With a ticket, the kernel
-// finishes the sum itself: every CTA takes a ticket after storing its
-// partial, and the CTA that takes the last one adds all partials, writes the
-// K sums to out (device or mapped host memory) and resets the counter for the
-// next launch -- one launch instead of two, no copy when out is mapped.
+// Where a reduction kernel's CTAs leave their sums.  Every CTA takes a ticket after
+// storing its partial (K Fr), and the CTA that takes the last one adds all partials,
+// writes the K sums to out (mapped host memory) and resets the counter for the next
+// launch.
 //
-// A fused launch also announces its completion to the host: after writing
-// the sums, the last CTA stores seq (fused_next_seq(), nonzero) into a word
-// of mapped host memory whose device address sits in the ticket's block
-// (ticket + 2, see fused_slots), so fused_read can poll that word instead of
-// waiting for the stream.
+// It also announces its completion to the host: after writing the sums, the
+// last CTA stores seq (fused_next_seq(), nonzero) into a word of mapped host
+// memory whose device address sits in the ticket's block (ticket + 2, see
+// fused_slots), so fused_read can poll that word instead of waiting for the
+// stream.
 struct RedOut {
   uint64_t* part;
-  unsigned* ticket;  // nullptr: partials only
+  unsigned* ticket;
   uint64_t* out;
-  unsigned seq;      // 0: no completion word
+  unsigned seq;  // 0: no completion word
 };
 
 // 32 bytes through L2 only: partials other CTAs wrote during this launch.
@@ -134,23 +132,30 @@ __device__ __forceinline__ Fr fr_load_cg(const uint64_t* base, size_t idx) {
   return r;
 }
 
-// The end of a reduction kernel: block sum, the CTA's partial, and with a
-// ticket the last CTA's final sum.  Every thread of the CTA calls it.
+// One thread of the last CTA, after its stores to out: the ticket as it was found, then
+// the completion word.
+__device__ __forceinline__ void announce(const RedOut& ro) {
+  *ro.ticket = 0u;
+  if (ro.seq) {
+    volatile unsigned* word = *reinterpret_cast<unsigned* const*>(ro.ticket + 2);
+    __threadfence_system();  // the sums before the completion word
+    *word = ro.seq;
+  }
+}
+
+// The end of a reduction kernel: block sum, the CTA's partial, and the last CTA's final
+// sum.  Every thread of the CTA calls it.
 template <int K>
 __device__ __forceinline__ void block_finish(Fr (&v)[K], const RedOut& ro) {
   __shared__ bool last;
   block_sum<K>(v);
-  const bool alone = ro.ticket && gridDim.x == 1;  // this CTA's sum is the sum
-  if (threadIdx.x == 0 && !alone) {
+  if (gridDim.x != 1) {  // else this CTA's sum is the sum
+    if (threadIdx.x == 0) {
 #pragma unroll
-    for (int k = 0; k < K; k++) fr_store(ro.part, (size_t)blockIdx.x * K + k, v[k]);
-    if (ro.ticket) {
+      for (int k = 0; k < K; k++) fr_store(ro.part, (size_t)blockIdx.x * K + k, v[k]);
       __threadfence();
       last = atomicAdd(ro.ticket, 1u) == gridDim.x - 1;
     }
-  }
-  if (!ro.ticket) return;
-  if (!alone) {
     __syncthreads();
     if (!last) return;
     __threadfence();
@@ -164,29 +169,33 @@ __device__ __forceinline__ void block_finish(Fr (&v)[K], const RedOut& ro) {
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < K; k++) fr_store(ro.out, k, v[k]);
-    if (!alone) *ro.ticket = 0u;
-    if (ro.seq) {
-      volatile unsigned* word = *reinterpret_cast<unsigned* const*>(ro.ticket + 2);
-      __threadfence_system();  // the sums before the completion word
-      *word = ro.seq;
-    }
+    announce(ro);
   }
 }
 
-template <int K>
-__global__ void __launch_bounds__(kRedThreads) sum_partials_kernel(const uint64_t* __restrict__ part,
-                                                                 int nparts,
-                                                                 uint64_t* __restrict__ out) {
-  Fr v[K];
-#pragma unroll
-  for (int k = 0; k < K; k++) v[k] = fr_zero();
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = fr_add(v[k], fr_load(part, (size_t)i * K + k));
-  block_sum<K>(v);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < K; k++) fr_store(out, k, v[k]);
+// The end of a kernel with several sums, each over a run of CTAs: thread 0's sum is this
+// CTA's partial, and warp w of the last CTA adds the partials first .. end - 1 of sum w
+// (count <= the CTA's warps; each thread passes its warp's run).
+__device__ __forceinline__ void runs_finish(const Fr& sum, const RedOut& ro, int count,
+                                            unsigned first, unsigned end) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    fr_store(ro.part, blockIdx.x, sum);
+    __threadfence();
+    last = atomicAdd(ro.ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < count) {
+    Fr x = fr_zero();
+    for (unsigned k = first + lane; k < end; k += 32) x = fr_add(x, fr_load_cg(ro.part, k));
+    x = warp_sum(x);
+    if (lane == 0) fr_store(ro.out, warp, x);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) announce(ro);
 }
 
 // CTAs for a reduction over n items (at most 4 per SM).

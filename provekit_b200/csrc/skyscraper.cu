@@ -320,10 +320,7 @@ __global__ void __launch_bounds__(skytc::kThreads, kTile ? 8 : 1)
     if (atomicAdd(ro.ticket, 1u) == gridDim.x - 1) {
       __threadfence();
       *reinterpret_cast<volatile unsigned long long*>(ro.out) = atomicExch(best, ~0ULL);
-      *ro.ticket = 0u;
-      volatile unsigned* word = *reinterpret_cast<unsigned* const*>(ro.ticket + 2);
-      __threadfence_system();  // the nonce before the completion word
-      *word = ro.seq;
+      announce(ro);
     }
   }
 }

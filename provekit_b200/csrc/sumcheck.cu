@@ -202,7 +202,6 @@ struct DotBatch {
 
 __global__ void __launch_bounds__(kRedThreads, 2) dots_kernel(const __grid_constant__ DotBatch J,
                                                               const RedOut ro) {
-  __shared__ bool last;
   int j = 0;
   while (j + 1 < J.count && blockIdx.x >= J.first[j + 1]) j++;
   const uint64_t* a = J.job[j].a;
@@ -223,30 +222,9 @@ __global__ void __launch_bounds__(kRedThreads, 2) dots_kernel(const __grid_const
     sum[0] = fr_add(sum[0], acc.finish());
   }
   block_sum<1>(sum);
-  if (threadIdx.x == 0) {
-    fr_store(ro.part, blockIdx.x, sum[0]);
-    __threadfence();
-    last = atomicAdd(ro.ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   static_assert(kMaxDots <= kRedThreads / 32, "a warp per dot product");
-  if (warp < J.count) {
-    Fr x = fr_zero();
-    for (unsigned k = J.first[warp] + lane; k < J.first[warp + 1]; k += 32)
-      x = fr_add(x, fr_load_cg(ro.part, k));
-    x = warp_sum(x);
-    if (lane == 0) fr_store(ro.out, warp, x);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *ro.ticket = 0u;
-    volatile unsigned* word = *reinterpret_cast<unsigned* const*>(ro.ticket + 2);
-    __threadfence_system();  // the sums before the completion word
-    *word = ro.seq;
-  }
+  const int w = threadIdx.x >> 5;
+  runs_finish(sum[0], ro, J.count, J.first[w], J.first[w + 1]);
 }
 
 // ---- CSR transpose: count, exclusive scan, scatter ------------------------

@@ -88,50 +88,57 @@ __global__ void whir_fold_rows_kernel(const uint64_t* __restrict__ rows, size_t 
   }
 }
 
-// CTA b owns the C coefficients [bC, (b + 1)C) (C a multiple of the CTA
-// size); its thread j takes bC + j + 256k for k = 0, 1, ..: Horner in
-// y = z^256 from the top.  A power tree in shared memory combines the 256
-// thread values, level l joining neighbours 2^l apart with z^(2^l), to
-// sum_j acc_j z^j; thread 0 scales it by z^(bC) (from the squares
-// z^(C 2^b)), and the CTA values are summed.  Per coefficient one product,
-// per thread one more: a per-thread z^t would cost up to log2(threads)
-// products per thread, more than the coefficients at mid sizes.
-// P.v[0] = z^256, P.v[1 + l] = z^(2^l) (l < 8), P.v[9 + b] = z^(C 2^b).
-constexpr int kEvalTreeLevels = 8;  // kRedThreads = 2^8
-constexpr int kEvalScaleBits = 10;  // CTAs < 2^10
-static_assert(kRedThreads == 1 << kEvalTreeLevels, "one tree level per thread-index bit");
+// Up to kMaxEvalPolys polynomials of n coefficients (stride apart) at one point z, a
+// run of g CTAs each.  CTA b of a run owns the coefficients [bC, (b + 1)C), C = 256 per;
+// its thread j takes bC + j + 256k for k = 0, 1, ..: an unreduced sum (fr_lazy.cuh)
+// with the weights y^k, y = z^256, Horner in y^kEvalWeights above that many.  The
+// thread's sum is scaled by z^j and the CTA's by z^(bC), each one product of two
+// powers that the host computed.  The CTA that takes the last ticket adds the CTAs'
+// sums, a warp per polynomial.  Two of 2^21 coefficients: 110 -> 57 us; one of 2^12: 18 -> 11 (Horner, a power tree
+// over the CTA and a launch per polynomial before).
+constexpr int kMaxEvalPolys = 8;
+constexpr int kEvalWeights = 32;
+constexpr int kEvalRunBits = 5;  // CTAs per polynomial < 16 * 2^5
+struct EvalPowers {
+  uint32_t y[kEvalWeights + 1][8];           // z^(256k)
+  uint32_t j_lo[16][8], j_hi[16][8];         // z^k, z^(16k)
+  uint32_t b_lo[16][8], b_hi[1 << kEvalRunBits][8];  // z^(Ck), z^(16Ck)
+};
+static_assert(kRedThreads == 256, "a thread's power is two of 16");
 
-__global__ void __launch_bounds__(kRedThreads) poly_eval_kernel(
-    const uint64_t* __restrict__ c, size_t n, size_t C,
-    const __grid_constant__ FrParams<1 + kEvalTreeLevels + kEvalScaleBits> P, const RedOut ro) {
-  __shared__ Fr tree[kRedThreads];
-  const unsigned j = threadIdx.x;
-  const size_t c0 = blockIdx.x * C;
-  Fr acc = fr_zero();
-  if (c0 + j < n) {
-    const Fr y = param_fr(P, 0);
-    const size_t end = n < c0 + C ? n : c0 + C;
-    for (size_t k = (end - 1 - c0 - j) / kRedThreads + 1; k-- > 0;)
-      acc = fr_add(fr_mul(acc, y), fr_load_ro(c, c0 + j + (size_t)kRedThreads * k));
-  }
-  Fr scale = fr_one_mont();
-  if (j == 0)
-    for (int b = 0; b < kEvalScaleBits; b++)
-      if ((blockIdx.x >> b) & 1) scale = fr_mul(scale, param_fr(P, 1 + kEvalTreeLevels + b));
-  tree[j] = acc;
-  __syncthreads();
+__device__ __forceinline__ Fr power(const uint32_t (&w)[8]) {
+  Fr r;
+#pragma unroll
+  for (int i = 0; i < 8; i++) r.v[i] = w[i];
+  return r;
+}
+
+__global__ void __launch_bounds__(kRedThreads, 2) poly_eval_kernel(
+    const uint64_t* __restrict__ coeffs, size_t n, size_t stride, int polys, unsigned g, size_t per,
+    const __grid_constant__ EvalPowers P, const RedOut ro) {
+  const unsigned j = threadIdx.x, b = blockIdx.x % g;
+  const uint64_t* c = coeffs + 4 * stride * (blockIdx.x / g);
+  const size_t at = b * per * kRedThreads + j;
+  const size_t end = n < (b + 1) * per * kRedThreads ? n : (b + 1) * per * kRedThreads;
+  const size_t mine = at < end ? (end - at + kRedThreads - 1) / kRedThreads : 0;
+  Fr sum[1] = {fr_zero()};
+  size_t k0 = mine ? (mine - 1) / kEvalWeights * kEvalWeights : 0;
 #pragma unroll 1
-  for (int l = 0; l < kEvalTreeLevels; l++) {
-    const unsigned half = kRedThreads >> (l + 1);
-    Fr v;
-    if (j < half) v = fr_add(tree[2 * j], fr_mul(param_fr(P, 1 + l), tree[2 * j + 1]));
-    __syncthreads();
-    if (j < half) tree[j] = v;
-    __syncthreads();
+  for (size_t left = mine; left > 0; left = k0, k0 -= left ? kEvalWeights : 0) {
+    const int terms = (int)(left - k0);
+    lazy::Acc acc;
+    acc.zero();
+#pragma unroll 2
+    for (int k = 0; k < terms; k++)
+      acc.mac(power(P.y[k]), fr_load_ro(c, at + (k0 + k) * kRedThreads));
+    const Fr run = acc.finish();
+    sum[0] = left == mine ? run : fr_add(fr_mul(sum[0], power(P.y[kEvalWeights])), run);
   }
-  Fr out[1] = {fr_zero()};
-  if (j == 0) out[0] = fr_mul(tree[0], scale);
-  block_finish<1>(out, ro);
+  sum[0] = fr_mul(sum[0], fr_mul(power(P.j_lo[j & 15]), power(P.j_hi[j >> 4])));
+  block_sum<1>(sum);
+  if (j == 0) sum[0] = fr_mul(sum[0], fr_mul(power(P.b_lo[b & 15]), power(P.b_hi[b >> 4])));
+  static_assert(kMaxEvalPolys <= kRedThreads / 32, "a warp per polynomial");
+  runs_finish(sum[0], ro, polys, (j >> 5) * g, (j >> 5) * g + g);
 }
 
 // path[q depth + l] = node (idx[q] >> l) ^ 1 of level l
@@ -411,6 +418,58 @@ extern "C" int pkg_whir_fold_rows(const uint64_t* rows, size_t nrows, unsigned k
   return PKG_OK;
 }
 
+namespace pk {
+static void put_powers(uint32_t (*out)[8], size_t count, const HostFr& x) {
+  HostFr w = HostFr::one();
+  for (size_t k = 0; k < count; k++) {
+    memcpy(out[k], w.l, 32);
+    w = HostFr::mul(w, x);
+  }
+}
+
+int poly_eval_device(const uint64_t* coeffs, size_t n, size_t stride, size_t polys,
+                     const uint64_t* points, size_t npts, uint64_t* out, cudaStream_t s) {
+  FusedSlots fs;
+  int rc = fused_slots(&fs);
+  if (rc) return rc;
+  std::vector<uint64_t> vals(4 * kFusedSlotFr);
+  for (size_t i0 = 0; i0 < polys; i0 += kMaxEvalPolys) {
+    const size_t np = std::min<size_t>(polys - i0, kMaxEvalPolys);
+    // all polynomials' CTAs resident at once, at least a coefficient per thread
+    const size_t gmax = std::min<size_t>(std::max<size_t>(1, 2 * (size_t)sm_count() / np),
+                                         16 << kEvalRunBits);
+    const size_t per = (n + kRedThreads * gmax - 1) / (kRedThreads * gmax);
+    const size_t C = per * kRedThreads, g = (n + C - 1) / C;
+    // a launch per point; their values are read once the slots are full
+    const size_t chunk = kFusedSlotFr / np;
+    for (size_t j0 = 0; j0 < npts; j0 += chunk) {
+      const size_t m = std::min(chunk, npts - j0);
+      for (size_t j = 0; j < m; j++) {
+        const HostFr z = HostFr::from_limbs(points + 4 * (j0 + j));
+        EvalPowers P;
+        memset(&P, 0, sizeof P);
+        put_powers(P.j_lo, 16, z);
+        const HostFr z16 = HostFr::pow_u64(z, 16), y = HostFr::pow_u64(z16, 16);
+        put_powers(P.j_hi, 16, z16);
+        put_powers(P.y, std::min<size_t>(per, kEvalWeights) + 1, y);
+        const HostFr zc = HostFr::pow_u64(y, per);
+        put_powers(P.b_lo, std::min<size_t>(g, 16), zc);
+        put_powers(P.b_hi, (g + 15) / 16, HostFr::pow_u64(zc, 16));
+        const RedOut ro = {fs.part, fs.ticket, fs.dev + 4 * np * j, fused_next_seq()};
+        poly_eval_kernel<<<(unsigned)(g * np), kRedThreads, 0, s>>>(
+            coeffs + 4 * stride * i0, n, stride, (int)np, (unsigned)g, per, P, ro);
+        PK_CHECK_LAUNCH("poly_eval_kernel");
+      }
+      if ((rc = fused_read(vals.data(), fs, 32 * np * m, s))) return rc;
+      for (size_t j = 0; j < m; j++)
+        for (size_t i = 0; i < np; i++)
+          memcpy(out + 4 * ((i0 + i) * npts + j0 + j), vals.data() + 4 * (np * j + i), 32);
+    }
+  }
+  return PKG_OK;
+}
+}  // namespace pk
+
 extern "C" int pkg_poly_eval_many(const uint64_t* coeffs, size_t n, const uint64_t* points,
                                   size_t npts, uint64_t* out, pkg_stream_t stream) {
   if (npts == 0) return PKG_OK;
@@ -421,50 +480,7 @@ extern "C" int pkg_poly_eval_many(const uint64_t* coeffs, size_t n, const uint64
   }
   PK_REQUIRE(coeffs && aligned16(coeffs), "null or unaligned coefficients");
   PK_REQUIRE(n < (size_t(1) << 40), "too many coefficients");
-  cudaStream_t s = as_stream(stream);
-  // at least kEvalMin coefficients per thread, up to 4 CTAs per SM (and
-  // fewer than 2^kEvalScaleBits CTAs); C coefficients per CTA
-  constexpr size_t kEvalMin = 4;
-  const size_t gmax = std::min<size_t>((size_t)sm_count() * 4, (size_t(1) << kEvalScaleBits) - 1);
-  size_t g = std::max<size_t>(1, std::min(gmax, (n + kRedThreads * kEvalMin - 1) /
-                                                    (kRedThreads * kEvalMin)));
-  const size_t per = (n + kRedThreads * g - 1) / (kRedThreads * g);
-  const size_t C = per * kRedThreads;
-  g = (n + C - 1) / C;
-  // up to kFusedSlotFr points: each launch writes its value to the thread's
-  // fused slots; more points: partials, one summing launch per point
-  FusedSlots fs;
-  int rc = fused_slots(&fs);
-  if (rc) return rc;
-  const bool fused = npts <= kFusedSlotFr;
-  Scratch scr;
-  if (!fused && (rc = scr.alloc(32 * ((size_t)g + npts), s))) return rc;
-  uint64_t* part = fused ? fs.part : static_cast<uint64_t*>(scr.ptr);
-  uint64_t* d_out = fused ? fs.dev : part + 4 * (size_t)g;
-  for (size_t j = 0; j < npts; j++) {
-    const HostFr z = HostFr::from_limbs(points + 4 * j);
-    FrParams<1 + kEvalTreeLevels + kEvalScaleBits> P;
-    HostFr sq = z;
-    for (int l = 0; l < kEvalTreeLevels; l++) {  // z^(2^l), then z^256
-      put_param(P, 1 + l, sq);
-      sq = HostFr::mul(sq, sq);
-    }
-    put_param(P, 0, sq);
-    sq = HostFr::pow_u64(z, C);
-    for (int b = 0; b < kEvalScaleBits; b++) {  // z^(C 2^b)
-      put_param(P, 1 + kEvalTreeLevels + b, sq);
-      sq = HostFr::mul(sq, sq);
-    }
-    const RedOut ro = {part, fused ? fs.ticket : nullptr, fused ? d_out + 4 * j : nullptr,
-                       fused ? fused_next_seq() : 0u};
-    poly_eval_kernel<<<(unsigned)g, kRedThreads, 0, s>>>(coeffs, n, C, P, ro);
-    PK_CHECK_LAUNCH("poly_eval_kernel");
-    if (!fused) {
-      sum_partials_kernel<1><<<1, kRedThreads, 0, s>>>(part, (int)g, d_out + 4 * j);
-      PK_CHECK_LAUNCH("sum_partials_kernel");
-    }
-  }
-  return fused ? fused_read(out, fs, 32 * npts, s) : read_small(out, d_out, 32 * npts, s);
+  return poly_eval_device(coeffs, n, 0, 1, points, npts, out, as_stream(stream));
 }
 
 extern "C" int pkg_merkle_open(const uint8_t* layers, size_t num_leaves, const uint64_t* indices,

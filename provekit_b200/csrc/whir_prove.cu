@@ -786,9 +786,9 @@ extern "C" int pkg_whir_commit_ood(const pkg_whir_params* p, pkg_transcript* t,
   for (unsigned j = 0; j < o; j++) pkg_transcript_squeeze(t, ood_points + 4 * j);
   // f_i(z_j), polynomial by polynomial (parseBatchedCommitment,
   // recursive-verifier/app/circuit/mtUtilities.go:51-76)
-  for (unsigned i = 0; o && i < p->batch_size; i++) {
-    int rc = pkg_poly_eval_many(coeffs + 4 * N * i, N, ood_points, o, commit_words + 4 + 4 * o * i,
-                                stream);
+  if (o) {
+    const int rc =
+        poly_eval_device(coeffs, N, N, p->batch_size, ood_points, o, commit_words + 4, s);
     if (rc) return rc;
   }
   for (unsigned j = 0; j < o * p->batch_size; j++)
