@@ -94,8 +94,8 @@ __global__ void whir_fold_rows_kernel(const uint64_t* __restrict__ rows, size_t 
 // with the weights y^k, y = z^256, Horner in y^kEvalWeights above that many.  The
 // thread's sum is scaled by z^j and the CTA's by z^(bC), each one product of two
 // powers that the host computed.  The CTA that takes the last ticket adds the CTAs'
-// sums, a warp per polynomial.  Two of 2^21 coefficients: 110 -> 57 us; one of 2^12: 18 -> 11 (Horner, a power tree
-// over the CTA and a launch per polynomial before).
+// sums, a warp per polynomial.  Two of 2^21 coefficients: 110 -> 57 us; one of 2^12:
+// 18 -> 11 (Horner, a power tree over the CTA and a launch per polynomial before).
 constexpr int kMaxEvalPolys = 8;
 constexpr int kEvalWeights = 32;
 constexpr int kEvalRunBits = 5;  // CTAs per polynomial < 16 * 2^5
