@@ -27,12 +27,6 @@
 
 namespace pk {
 
-// CTAs of 128 threads per SM the leaf kernel is compiled for (its register
-// budget: 7 -> 72 registers).
-#ifndef PK_LEAF_MIN_CTAS
-#define PK_LEAF_MIN_CTAS 7
-#endif
-
 // Plain loads, as everywhere in kernels of launch_early: the previous kernel may
 // still be writing when they start, and read-only loads (ld.global.nc) are not
 // ordered after griddepcontrol.wait.
@@ -65,9 +59,12 @@ __global__ void compress_many_kernel(const uint8_t* __restrict__ in, size_t n,
 // consecutive Fr).  Canonical encoding converts each Montgomery element
 // (x*2^256 -> x) before hashing; Montgomery encoding hashes the raw limbs.
 // A one-element leaf is the element itself (hash_many(32) copies).
+// For the leaves that tiles do not pay for (tc_wanted).
+constexpr int kLeafMinCtas = 7;  // per SM: 72 registers
 template <bool kCanonical>
-__global__ void __launch_bounds__(128, PK_LEAF_MIN_CTAS) leaf_fold_fr_kernel(const uint64_t* __restrict__ cw, size_t fr_per_leaf,
-                                    size_t count, uint8_t* __restrict__ out) {
+__global__ void __launch_bounds__(128, kLeafMinCtas)
+    leaf_fold_fr_kernel(const uint64_t* __restrict__ cw, size_t fr_per_leaf, size_t count,
+                        uint8_t* __restrict__ out) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count;
        i += (size_t)gridDim.x * blockDim.x) {
     const size_t base = i * fr_per_leaf;
