@@ -34,27 +34,35 @@ PROVE_UNIT = "proofs/s"
 METRIC = ("WHIR commit throughput, Spartan+WHIR prover hot path: 2^20 Fr coefficients -> "
           "RS rate-1/4 coset NTT -> 2^22 evaluations -> Skyscraper Merkle tree (bit-exact)")
 UNIT = "commits/s"
-IMAD_PER_MONT = 264  # mad.lo/madc.hi/mul.lo per 8x32 CIOS product (fr.cuh: 8 x (16 + 16 + 1))
-# binary64 instructions per Fr operation of the FP64-pipe routines (fr_f64.cuh):
-# digit conversion 11 per operand, digit products (121 general, 66 + 10
-# doublings for a square), ten 24-bit Montgomery steps of 14, and the 16-bit
-# step plus normalisation (69).
-F64_PER_MUL = 22 + 121 + 140 + 69      # 352
-F64_PER_SQR = 11 + 66 + 10 + 140 + 69  # 296
-# integer multiply-adds of one Montgomery->canonical REDC (fr.cuh
-# fr_from_mont: 8 x (1 + 16)); B200 runs them on the same throughput as the
-# binary64 fmas (a kernel mixing the two runs at the rate of either alone),
-# so the leaf kernel's multiply work is its squarings plus these.
-IMAD_PER_REDC = 8 * (1 + 16)  # 136
-# dram__bytes_read.sum + dram__bytes_write.sum of one leaf_fold_fr_kernel launch
-# from an ncu capture of this workload (the leaf kernel's WHIR-commit profile
-# summary under profiles/), keyed by (log2 coeffs, folding factor, log inv rate).
-LEAF_TRAFFIC_BYTES = {(20, 4, 2): 134.264064e6 + 6.855168e6}
-# the same for the whole proof's witness commitment (whir-ZK: 2^20 leaves of
-# 16 Fr, the witness and blinding polynomials of m = 21 at rate 1/4), from an
-# ncu capture of the default command (the leaf kernel's whole-proof profile
-# summary under profiles/).
-LEAF_TRAFFIC_PROVE_BYTES = 537195264 + 33959680
+# 64-bit multiply-adds (32 x 32 + 64) of the kernels' Fr operations.  In the tiled
+# kernels the Montgomery reduction is a matrix product on the tensor cores and a
+# quotient step of 8 is left of it; elsewhere a product is 64 and its reduction 64,
+# and a term of an unreduced sum is 64.
+WIDE_PER_SQR = 36 + 8  # tiled: 28 cross and 8 diagonal products
+WIDE_PER_MUL = 64 + 8  # tiled
+WIDE_PER_MUL_SIMT = 64 + 64
+WIDE_PER_TERM = 64
+# A 64-bit multiply-add takes the multiplier two of the slots that the measured 32-bit
+# multiply-add (pkg_measure_imad_rate) takes one of.
+SLOTS_PER_WIDE = 2
+# Poseidon2 (t = 4, rf = 8, rp = 56), tiled: an s-box is two squares and a product; a
+# partial round has one, and reduces the other three elements of its matrix product.
+WIDE_PER_POSEIDON2 = (8 * 4 + 56) * (2 * WIDE_PER_SQR + WIDE_PER_MUL) + 56 * 3 * 8
+# dram__bytes_read.sum + dram__bytes_write.sum of one fold_tc_kernel launch from an ncu
+# capture of this shape (the fold kernel's profile summary under profiles/), keyed by
+# (log2 coeffs, folding factor, log inv rate).
+LEAF_TRAFFIC_BYTES = {(20, 4, 2): 134.298e6 + 6.458e6}
+# the same for the whole proof's witness commitment (whir-ZK: 2^20 leaves of 16 Fr, the
+# witness and blinding polynomials of m = 21 at rate 1/4).
+LEAF_TRAFFIC_PROVE_BYTES = 536.947e6 + 31.544e6
+
+
+def wide_rate(L):
+    """64-bit multiply-adds per second of this GPU (half of the measured 32-bit rate)."""
+    from provekit_b200._lib import check
+    imad = ctypes.c_double(0)
+    check(L.pkg_measure_imad_rate(ctypes.byref(imad)))
+    return imad.value / SLOTS_PER_WIDE
 
 
 def parse_args():
@@ -468,22 +476,14 @@ def run_b200(a):
             dist.destroy_process_group()
         return
 
-    # ---- roofline of the dominant kernel (Merkle leaf fold): its Fr
-    # arithmetic runs on the FP64 pipe, so the bound is the measured fma rate
-    # over the binary64 instructions the squarings and conversions need.
-    imad = ctypes.c_double(0)
-    check(L.pkg_measure_imad_rate(ctypes.byref(imad)))
-    dfma = ctypes.c_double(0)
-    check(L.pkg_measure_dfma_rate(ctypes.byref(dfma)))
-    mont_peak = imad.value / IMAD_PER_MONT
+    # ---- roofline of the dominant kernel (Merkle leaf fold): bound by the integer
+    # multiplier, so the measured multiply-add rate over what the squarings need (the
+    # leaves' Montgomery -> canonical conversions ride in the reductions).
+    peak = wide_rate(L)
     num_leaves = cw_len
-    mont_per_leaf_launch = num_leaves * ((M - 1) * 14 + M)
-    # the squarings' binary64 instructions plus the M Montgomery->canonical
-    # REDCs per leaf (integer multiply-adds on the same shared throughput)
-    f64_per_leaf_launch = num_leaves * ((M - 1) * 14 * F64_PER_SQR + M * IMAD_PER_REDC)
+    wide_per_launch = num_leaves * (M - 1) * 14 * WIDE_PER_SQR
     leaf_avg_s = statistics.mean(leaf_ms) * 1e-3
-    achieved = mont_per_leaf_launch / leaf_avg_s
-    f64_achieved = f64_per_leaf_launch / leaf_avg_s
+    achieved = wide_per_launch / leaf_avg_s
     ntt_stages = (msg_len << a.log_inv_rate).bit_length() - 1 - a.log_inv_rate
     ntt_mont = (total_fr // 2) * ntt_stages
     enc_avg_s = statistics.mean(enc_ms) * 1e-3
@@ -503,24 +503,17 @@ def run_b200(a):
         "data": "synthetic (ChaCha20-seeded uniform Fr, Montgomery form)",
         "config": workload_config(a),
         "roofline": {
-            "kernel": "leaf_fold_fr_kernel (Skyscraper leaf hashing)", "bound": "fp64",
-            "achieved": f64_achieved / 1e12, "peak": dfma.value / 1e12, "unit": "T multiply-op/s",
-            "frac": f64_achieved / dfma.value,
+            "kernel": "fold_tc_kernel (Skyscraper leaf hashing)", "bound": "int_mul",
+            "achieved": achieved / 1e12, "peak": peak / 1e12,
+            "unit": "T 64-bit multiply-add/s", "frac": achieved / peak,
             "traffic": LEAF_TRAFFIC_BYTES.get((a.log_coeffs, a.folding_factor, a.log_inv_rate)),
             "traffic_algorithmic": 32 * total_fr + 32 * num_leaves,
-            "peak_source": f"measured binary64 fma rate {dfma.value / 1e12:.3f} T/s "
-                           "(pkg_measure_dfma_rate, this GPU, this run)",
-            "algorithmic": f"{num_leaves} leaves x ({M - 1} compressions x 14 squarings x "
-                           f"{F64_PER_SQR} binary64 instructions + {M} Montgomery->canonical "
-                           f"REDCs x {IMAD_PER_REDC} integer multiply-adds) = "
-                           f"{f64_per_leaf_launch} multiply-pipe instructions per launch "
-                           f"({mont_per_leaf_launch} Fr products and REDCs); the integer "
-                           "multiply-adds share the binary64 fma throughput on B200",
-            "achieved_gmont_per_s": achieved / 1e9,
-            "int_pipe_alt": {"peak_gmont_per_s": mont_peak / 1e9, "frac": achieved / mont_peak,
-                             "note": f"the same products against the IMAD roofline (measured "
-                                     f"{imad.value / 1e12:.3f} T/s / {IMAD_PER_MONT} per CIOS "
-                                     "product), the bound of the integer-pipe routines"},
+            "peak_source": f"measured 32-bit multiply-add rate "
+                           f"{peak * SLOTS_PER_WIDE / 1e12:.3f} T/s (pkg_measure_imad_rate, this "
+                           "GPU, this run), two slots per 64-bit multiply-add",
+            "algorithmic": f"{num_leaves} leaves x {M - 1} compressions x 14 squarings x "
+                           f"{WIDE_PER_SQR} 64-bit multiply-adds = {wide_per_launch} per launch; "
+                           "the reductions' byte products run on the tensor cores",
         },
         "kernels": {
             "rs_encode_ms": statistics.mean(enc_ms), "merkle_leaves_ms": statistics.mean(leaf_ms),
@@ -785,10 +778,9 @@ def run_prove(a):
         if dist is not None:
             dist.destroy_process_group()
         return
-    dfma = ctypes.c_double(0)
-    check(L.pkg_measure_dfma_rate(ctypes.byref(dfma)))
-    f64_per_launch = rows * ((M - 1) * 14 * F64_PER_SQR + M * IMAD_PER_REDC)
-    f64_achieved = f64_per_launch / leaf_s
+    peak = wide_rate(L)
+    wide_per_launch = rows * (M - 1) * 14 * WIDE_PER_SQR
+    achieved = wide_per_launch / leaf_s
 
     cpu = None
     parity = {"result": "not checked in this run (the oracle leg runs on rank 0 at N=1 only)"}
@@ -819,16 +811,14 @@ def run_prove(a):
     proof_bytes = 8 * proof.shape[0]
 
     # the project's other targets, measured in the same run: the 2^24 NTT
-    # against both rooflines, the batched form on the 256-job mix against
+    # against its roofline, the batched form on the 256-job mix against
     # the same jobs one at a time, and the served form under an open-loop
     # Poisson stream against sequential plain proving
     north = None
     if a.gpus == 1 and not a.no_targets:
         north = {}
-        imad = ctypes.c_double(0)
-        check(L.pkg_measure_imad_rate(ctypes.byref(imad)))
         with torch.cuda.device(dev):
-            north["ntt_2p24"] = ntt_measure(L, stream, flush, 24, 10, 3, dfma.value, imad.value)
+            north["ntt_2p24"] = ntt_measure(L, stream, flush, 24, 10, 3, peak)
         torch.cuda.empty_cache()
         t0 = time.perf_counter()
         b = batched_compare(batched_sizes(a.seed, 256), a.seed, 3, 3)
@@ -857,7 +847,7 @@ def run_prove(a):
             "n_gpus": a.gpus, "steps": a.steps, "warmup": a.warmup,
             "ms_per_step": total_max / a.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "u32/f64 (BN254 Fr: 8x32-bit limbs, products on the FP64 pipe)",
+            "dtype": "u32 (BN254 Fr: 8x32-bit limbs, reductions as u8 tensor-core products)",
             "data": "synthetic R1CS (pkg_synthetic_r1cs, seeded)",
             "config": prove_config(a, h, wp, proof_bytes),
             "host_generation_s": gen_s,
@@ -865,19 +855,18 @@ def run_prove(a):
             "latency_ms": {"p50": p50_max, "p99": p99_max,
                            "note": "per-proof device time, worst rank"},
             "roofline": {
-                "kernel": f"leaf_fold_fr_kernel (Skyscraper leaf hashing of the witness "
+                "kernel": f"fold_tc_kernel (Skyscraper leaf hashing of the witness "
                           f"commitment: {rows} leaves of {M} Fr)",
-                "bound": "fp64", "achieved": f64_achieved / 1e12, "peak": dfma.value / 1e12,
-                "unit": "T multiply-op/s", "frac": f64_achieved / dfma.value,
+                "bound": "int_mul", "achieved": achieved / 1e12, "peak": peak / 1e12,
+                "unit": "T 64-bit multiply-add/s", "frac": achieved / peak,
                 "traffic": LEAF_TRAFFIC_PROVE_BYTES,
                 "traffic_algorithmic": 32 * rows * M + 32 * rows,
-                "peak_source": f"measured binary64 fma rate {dfma.value / 1e12:.3f} T/s "
-                               "(pkg_measure_dfma_rate, this GPU, this run)",
-                "algorithmic": f"{rows} leaves x ({M - 1} compressions x 14 squarings x "
-                               f"{F64_PER_SQR} binary64 instructions + {M} Montgomery->"
-                               f"canonical REDCs x {IMAD_PER_REDC} integer multiply-adds) = "
-                               f"{f64_per_launch} multiply-pipe instructions per launch; the "
-                               "integer multiply-adds share the binary64 fma throughput on B200",
+                "peak_source": f"measured 32-bit multiply-add rate "
+                               f"{peak * SLOTS_PER_WIDE / 1e12:.3f} T/s (pkg_measure_imad_rate, "
+                               "this GPU, this run), two slots per 64-bit multiply-add",
+                "algorithmic": f"{rows} leaves x {M - 1} compressions x 14 squarings x "
+                               f"{WIDE_PER_SQR} 64-bit multiply-adds = {wide_per_launch} per "
+                               "launch; the reductions' byte products run on the tensor cores",
                 "launch_ms": leaf_s * 1e3,
             },
             "stages_ms_last_step": stage_ms, "whir_phases_ms_last_step": whir_ms,
@@ -1227,7 +1216,7 @@ def run_served(a):
                       "sequential plain-GPU proving",
             "value": max(s["served"]["proofs_per_s"] for s in sweeps), "unit": "proofs/s",
             "n_gpus": 1, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "u32/f64 (BN254 Fr: 8x32-bit limbs, products on the FP64 pipe)",
+            "dtype": "u32 (BN254 Fr: 8x32-bit limbs, reductions as u8 tensor-core products)",
             "data": "synthetic R1CS (pkg_synthetic_r1cs)",
             "config": {"workload": "served", "whir": "ff 3, rate 1/4, 128 bits, 10 PoW bits",
                        "requests": len(reqs), "log2_constraints": logs,
@@ -1304,15 +1293,14 @@ def dual_measure(L, stream, flush, seed, steps, warmup):
 
 
 # ---------------------------------------------------------------------------
-# NTT: 2^24 (the size whose FP64-roofline fraction is the transform's target)
+# NTT: 2^24 (the size whose roofline fraction is the transform's target)
 # and the 2^16 single-vector transform.
 # ---------------------------------------------------------------------------
-def ntt_measure(L, stream, flush, logn, steps, warmup, dfma_rate, imad_rate):
+def ntt_measure(L, stream, flush, logn, steps, warmup, peak):
     """ntt_nr at 2^logn (one vector, L2 flushed between steps, CUDA events on
     the launching stream) and intt_rn on its output with the round trip
-    checked; throughput against the FP64-pipe roofline (measured DFMA rate /
-    binary64 instructions per product) and the integer-pipe one (measured
-    IMAD rate / 264 per 8x32 CIOS product)."""
+    checked; throughput against the multiplier's roofline (peak: measured 64-bit
+    multiply-adds per second, WIDE_PER_MUL per butterfly)."""
     import numpy as np
     import torch
 
@@ -1354,34 +1342,28 @@ def ntt_measure(L, stream, flush, logn, steps, warmup, dfma_rate, imad_rate):
     rate = products / (ms * 1e-3)
     del d, src_t
     return {"log2_n": logn, "ms": ms, "fr_per_s": n / (ms * 1e-3), "gmont_per_s": rate / 1e9,
-            "frac_fp64": rate / (dfma_rate / F64_PER_MUL),
-            "frac_int": rate / (imad_rate / IMAD_PER_MONT),
-            "peak_gmont_fp64": dfma_rate / F64_PER_MUL / 1e9,
-            "peak_gmont_int": imad_rate / IMAD_PER_MONT / 1e9,
-            "hbm_gbs": 2 * 32 * n * ((logn + 8) // 9) / (ms * 1e-3) / 1e9,
+            "frac": rate / (peak / WIDE_PER_MUL), "peak_gmont": peak / WIDE_PER_MUL / 1e9,
+            "frac_untiled": rate / (peak / WIDE_PER_MUL_SIMT),
+            "hbm_gbs": 2 * 32 * n * ((logn + 7) // 8) / (ms * 1e-3) / 1e9,
             "intt_rn_ms": ms_inv, "round_trip_ok": ok,
             "note": "CUDA events around one ntt_nr launch sequence, L2 flushed (256 MiB write) "
-                    "before each; frac_fp64 against the measured binary64 fma rate / "
-                    f"{F64_PER_MUL} per product (the butterflies multiply on the FP64 pipe), "
-                    f"frac_int against the measured IMAD rate / {IMAD_PER_MONT} per 8x32 CIOS "
-                    "product (the integer-pipe roofline)"}
+                    f"before each; frac against the measured multiply-add rate / {WIDE_PER_MUL} "
+                    "64-bit multiply-adds per butterfly (its reduction runs on the tensor "
+                    f"cores), frac_untiled against {WIDE_PER_MUL_SIMT} (the reduction on the "
+                    "multiplier too)"}
 
 
 def run_ntt(a):
     import torch
 
     from provekit_b200 import _lib
-    from provekit_b200._lib import check
 
     L = _lib.lib()
     torch.cuda.set_device(0)
     stream = torch.cuda.Stream()
-    imad = ctypes.c_double(0)
-    check(L.pkg_measure_imad_rate(ctypes.byref(imad)))
-    dfma = ctypes.c_double(0)
-    check(L.pkg_measure_dfma_rate(ctypes.byref(dfma)))
+    peak = wide_rate(L)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
-    out = {logn: ntt_measure(L, stream, flush, logn, a.steps, a.warmup, dfma.value, imad.value)
+    out = {logn: ntt_measure(L, stream, flush, logn, a.steps, a.warmup, peak)
            for logn in (24, 16)}
     line = {"metric": "BN254 Fr ntt_nr throughput, 2^24 (roofline target) and 2^16 (single vector)",
             "value": out[24]["fr_per_s"], "unit": "Fr/s", "n_gpus": 1, "steps": a.steps,
@@ -1389,16 +1371,14 @@ def run_ntt(a):
             "scaling": "weak", "vs_baseline": None, "dtype": "u32 (BN254 Fr, 8x32-bit limbs)",
             "data": "synthetic (ChaCha20-seeded Fr)",
             "config": {"workload": "ntt", "log2_n": 24, "l2": "flushed between steps"},
-            "roofline": {"kernel": "ntt_pass_kernel", "bound": "fp64",
-                         "achieved": out[24]["gmont_per_s"],
-                         "peak": out[24]["peak_gmont_fp64"],
-                         "unit": "Gmont/s", "frac": out[24]["frac_fp64"],
+            "roofline": {"kernel": "ntt_pass_kernel", "bound": "int_mul",
+                         "achieved": out[24]["gmont_per_s"], "peak": out[24]["peak_gmont"],
+                         "unit": "Gmont/s", "frac": out[24]["frac"],
                          "algorithmic": f"(n/2) log2 n Montgomery products per transform, "
-                                        f"{F64_PER_MUL} binary64 instructions each",
-                         "peak_source": f"measured binary64 fma rate {dfma.value / 1e12:.3f} T/s "
-                                        f"(pkg_measure_dfma_rate) / {F64_PER_MUL}",
-                         "int_pipe_alt": {"peak_gmont_per_s": out[24]["peak_gmont_int"],
-                                          "frac": out[24]["frac_int"]}},
+                                        f"{WIDE_PER_MUL} 64-bit multiply-adds each",
+                         "peak_source": f"measured 64-bit multiply-add rate {peak / 1e12:.3f} T/s "
+                                        f"(pkg_measure_imad_rate / {SLOTS_PER_WIDE}) / "
+                                        f"{WIDE_PER_MUL}"},
             "ntt_2p24": out[24], "ntt_2p16": out[16]}
     print(json.dumps(line), flush=True)
 
@@ -1420,7 +1400,7 @@ def run_dual(a):
             "value": r["proofs_per_s"], "unit": "proofs/s", "n_gpus": 1, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": r["ms"], "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "u32/f64 (BN254 Fr: 8x32-bit limbs, products on the FP64 pipe)",
+            "dtype": "u32 (BN254 Fr: 8x32-bit limbs, reductions as u8 tensor-core products)",
             "data": "synthetic R1CS with challenges (pkg_synthetic_r1cs_dual, seeded)",
             "config": {"workload": "dual", "description": r["config"],
                        "l2": "flushed: 256 MiB device write before each step"},
@@ -1443,8 +1423,7 @@ def run_whir_ops(a):
     L = _lib.lib()
     torch.cuda.set_device(0)
     stream = torch.cuda.Stream()
-    dfma = ctypes.c_double(0)
-    check(L.pkg_measure_dfma_rate(ctypes.byref(dfma)))
+    peak = wide_rate(L)
     m, k, lr = 21, 3, 2
     n = 1 << m
 
@@ -1498,7 +1477,7 @@ def run_whir_ops(a):
         stream.synchronize()
         ms = statistics.mean(e0.elapsed_time(e1) for e0, e1 in evs)
         res[name] = {"ms": ms, "gmont_per_s": products / (ms * 1e-3) / 1e9,
-                     "fp64_frac": products * F64_PER_MUL / (ms * 1e-3) / dfma.value,
+                     "int_mul_frac": products * WIDE_PER_TERM / (ms * 1e-3) / peak,
                      "hbm_gbs": nbytes / (ms * 1e-3) / 1e9}
     line = {"metric": "WHIR prove-round operations (device), first-round sizes of the 2^20-"
                       "constraint prove core: m = 21, folding factor 3, rate 1/4",
@@ -1509,7 +1488,7 @@ def run_whir_ops(a):
             "data": "synthetic (ChaCha20-seeded Fr)",
             "config": {"workload": "whir_ops", "m": m, "folding_factor": k, "log_inv_rate": lr,
                        "l2": "flushed between steps"},
-            "ops": res, "dfma_rate_tops": dfma.value / 1e12,
+            "ops": res, "wide_rate_tops": peak / 1e12,
             "note": "synchronous ops (poly_eval, sumcheck_round, eq_accumulate, merkle_open) "
                     "include their host read-back"}
     print(json.dumps(line), flush=True)
@@ -1529,8 +1508,7 @@ def run_poseidon2(a):
     L = _lib.lib()
     torch.cuda.set_device(0)
     stream = torch.cuda.Stream()
-    dfma = ctypes.c_double(0)
-    check(L.pkg_measure_dfma_rate(ctypes.byref(dfma)))
+    peak = wide_rate(L)
     n = 1 << 22
     h = np.zeros((4 * n, 4), np.uint64)
     check(L.pkg_sample_fr(17, 4 * n, h.ctypes.data, 1))
@@ -1557,24 +1535,19 @@ def run_poseidon2(a):
 
     ms_perm = timed(lambda: poseidon2_permutation_many(st, stream=stream))
     ms_hash = timed(lambda: poseidon2_hash_many(src[: 3 * ((4 * n) // 3)], 3, out=out, stream=stream))
-    # products per permutation: full rounds 8 x 4 s-boxes (x^5: 2 squares + 1
-    # product), partial rounds 56 x 1 s-box, plus the internal layer's 4
-    # diagonal products in each of the 56 partial rounds
-    prod_perm = 8 * 4 * 3 + 56 * 3 + 56 * 4
-    fp64 = prod_perm * F64_PER_MUL
     line = {"metric": "Poseidon2 (BN254, t = 4) permutations/s over 2^22 states",
             "value": n / (ms_perm * 1e-3), "unit": "permutations/s", "n_gpus": 1,
             "steps": a.steps, "warmup": a.warmup, "ms_per_step": ms_perm,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "u32 (BN254 Fr, 8x32-bit limbs)", "data": "synthetic (ChaCha20-seeded Fr)",
             "config": {"workload": "poseidon2", "states": n, "l2": "flushed between steps"},
-            "roofline": {"kernel": "poseidon2 permutation kernel", "bound": "fp64",
-                         "achieved": n * fp64 / (ms_perm * 1e-3) / 1e12,
-                         "peak": dfma.value / 1e12, "unit": "T fp64-op/s",
-                         "frac": n * fp64 / (ms_perm * 1e-3) / dfma.value,
-                         "algorithmic": f"{prod_perm} Fr products per permutation at "
-                                        f"{F64_PER_MUL} binary64 instructions (squares counted as "
-                                        "products: an upper bound on the work)"},
+            "roofline": {"kernel": "poseidon2 permutation kernel", "bound": "int_mul",
+                         "achieved": n * WIDE_PER_POSEIDON2 / (ms_perm * 1e-3) / 1e12,
+                         "peak": peak / 1e12, "unit": "T 64-bit multiply-add/s",
+                         "frac": n * WIDE_PER_POSEIDON2 / (ms_perm * 1e-3) / peak,
+                         "algorithmic": f"{WIDE_PER_POSEIDON2} 64-bit multiply-adds per "
+                                        "permutation (88 s-boxes, the partial rounds' matrix "
+                                        "products as terms of the tensor-core reductions)"},
             "hash_rate_per_s": ((4 * n) // 3) / (ms_hash * 1e-3),
             "hash_note": "poseidon2_hash of 3-element inputs (one permutation each)"}
     print(json.dumps(line), flush=True)
