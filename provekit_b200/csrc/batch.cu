@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
     sm[E + sidx] = in[1];  // high 16 bytes: plane 1
   }
   __syncthreads();
-  tile_stages(tile, sm, mode_b, K, T, log_t, log_u, l0, high_a, d.first != 0, roots);
+  tile_stages<false>(tile, sm, mode_b, K, T, log_t, log_u, l0, high_a, d.first != 0, roots);
   const bool last = d.last != 0;
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;

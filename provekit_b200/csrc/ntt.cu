@@ -205,8 +205,14 @@ struct PassShape {
 // kModeB selects mode B at compile time.  In mode A every line of the CTA
 // shares `high`, so stage s reads only the 2^s twiddles roots[(high << s) |
 // grp], which stay in L1.
-template <int kSrc, bool kModeB>
-__global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
+//
+// kAhead, for grids that leave two CTAs per SM or fewer: a stage's twiddle is loaded
+// during the stage before, with the registers that the missing CTAs leave (2^10 points
+// 12.9 -> 11.9 us, 2^16 26.5 -> 25.0); larger grids hide the load behind other CTAs, and eight
+// of them have no registers for it (2^24 2.85 -> 2.92 ms).
+constexpr int kAheadCtas = 2;
+template <int kSrc, bool kModeB, bool kAhead>
+__global__ void __launch_bounds__(tc::kThreads, kAhead ? kAheadCtas : tc::kMaxCtas)
     ntt_pass_kernel(uint64_t* data, uint64_t* out, const uint64_t* __restrict__ roots,
                     const PassShape shape, const NttSource src) {
   extern __shared__ uint4 sm[];
@@ -241,7 +247,7 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
     }
   }
   __syncthreads();
-  tile_stages(tile, sm, kModeB, K, T, log_t, log_u, l0, high_a, shape.first, roots);
+  tile_stages<kAhead>(tile, sm, kModeB, K, T, log_t, log_u, l0, high_a, shape.first, roots);
   // ---- store ----
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
@@ -253,6 +259,13 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
     fr_store(out, shape.inverse ? reversed(g, shape.inverse) : g, v);
   }
   tile.close();
+}
+
+using PassKernel = void (*)(uint64_t*, uint64_t*, const uint64_t*, PassShape, NttSource);
+template <int kSrc>
+static PassKernel pass_kernel(bool mode_b, bool ahead) {
+  if (ahead) return mode_b ? ntt_pass_kernel<kSrc, true, true> : ntt_pass_kernel<kSrc, false, true>;
+  return mode_b ? ntt_pass_kernel<kSrc, true, false> : ntt_pass_kernel<kSrc, false, false>;
 }
 
 static inline uint64_t pow2_part(uint64_t x) { return x & (~x + 1); }
@@ -297,13 +310,10 @@ static int run_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end
       kind = inverse ? kFromReversed : kFromEncode;
     }
     uint64_t* const out = inverse && shape.last ? inverse : data;
-    void (*fn)(uint64_t*, uint64_t*, const uint64_t*, PassShape, NttSource) =
-        kind == kFromData
-            ? (mode_b ? ntt_pass_kernel<kFromData, true> : ntt_pass_kernel<kFromData, false>)
-        : kind == kFromEncode
-            ? (mode_b ? ntt_pass_kernel<kFromEncode, true> : ntt_pass_kernel<kFromEncode, false>)
-            : (mode_b ? ntt_pass_kernel<kFromReversed, true>
-                      : ntt_pass_kernel<kFromReversed, false>);
+    const bool ahead = grid <= kAheadCtas * (unsigned)sm_count();
+    const PassKernel fn = kind == kFromData     ? pass_kernel<kFromData>(mode_b, ahead)
+                          : kind == kFromEncode ? pass_kernel<kFromEncode>(mode_b, ahead)
+                                                : pass_kernel<kFromReversed>(mode_b, ahead);
     PK_CUDA(launch_early(fn, grid, tc::kThreads, smem, stream, data, out, roots, shape, s));
     PK_CHECK_LAUNCH("ntt_pass_kernel");
     t += K;

@@ -90,12 +90,23 @@ __device__ __forceinline__ void loose_butterfly(const Fr& x0, const Fr& m, Fr& y
 
 // The K stages of a pass over a tile of E = T << K elements in shared memory,
 // 128 butterflies at a time (all tc::kThreads threads call it).  first: stage 0
-// is stage 0 of the transform, whose twiddles are all 1.
+// is stage 0 of the transform, whose twiddles are all 1.  kAhead: the next twiddle is
+// loaded beside the matrix product (ntt.cu says where).
+template <bool kAhead>
 __device__ __forceinline__ void tile_stages(tc::ProductTile& tile, uint4* sm, bool mode_b, int K,
                                             int T, int log_t, int log_u, uint64_t l0,
                                             uint64_t high_a, bool first,
                                             const uint64_t* __restrict__ roots) {
   const int E = T << K, half = E >> 1;
+  Fr ahead = fr_zero();
+  // the twiddle of this thread's butterfly from b0 on in stage s
+  const auto twiddle = [&](int s, int b0) {
+    const int b = b0 + (int)threadIdx.x;
+    const int bb = b < half ? b : 0;
+    const uint64_t high = mode_b ? (l0 + (bb & (T - 1))) >> log_u : high_a;
+    return fr_load_ro(roots, (high << s) | (uint64_t)((bb >> log_t) >> (K - 1 - s)));
+  };
+  if (kAhead && !first) ahead = twiddle(0, 0);
 #pragma unroll 1
   for (int s = 0; s < K; s++) {
     const int log_h = K - 1 - s;
@@ -110,13 +121,22 @@ __device__ __forceinline__ void tile_stages(tc::ProductTile& tile, uint4* sm, bo
       const int j0 = (grp << (log_h + 1)) + (pp & ((1 << log_h) - 1));
       const int i0 = j0 * T + ll, i1 = i0 + (T << log_h);
       const Fr x1 = tile_load(sm, E, i1);
+      const bool end = b0 + tc::kThreads >= half;  // of the stage
+      const int s2 = end ? s + 1 : s, b2 = end ? 0 : b0 + tc::kThreads;
       Fr m;
       if (first && s == 0) {
         m = fr_reduce_once(x1);
+        if (kAhead && end && s2 < K) ahead = twiddle(s2, b2);
       } else {
-        const uint64_t high = mode_b ? (l0 + ll) >> log_u : high_a;
-        const Fr w = fr_load_ro(roots, (high << s) | (uint64_t)grp);
+        Fr w;
+        if (kAhead) {
+          w = ahead;
+        } else {
+          const uint64_t high = mode_b ? (l0 + ll) >> log_u : high_a;
+          w = fr_load_ro(roots, (high << s) | (uint64_t)grp);
+        }
         tile.start(w, x1);
+        if (kAhead && s2 < K) ahead = twiddle(s2, b2);
         m = tile.finish();
         if (tile.alone) m = product_alone(w, x1);
         __syncwarp();

@@ -62,3 +62,11 @@ def test_encode(M, L, masks, log_cw):
     assert rc == 0
     got = RSFr().interleaved_encode(dev(m), dev(k) if masks else None, 1 << log_cw)
     assert np.array_equal(got.cpu().numpy().view(np.uint64), exp)
+
+
+@pytest.mark.parametrize("log_n", [1, 9, 10, 16, 17])
+def test_inverse_of_both_grids(log_n):
+    """Up to two CTAs of a pass per SM (2^16) and above."""
+    a = values(1 << log_n, log_n, "edges")
+    d = ntt_nr(dev(a), 1 << log_n, 1)
+    assert np.array_equal(intt_rn(d).cpu().numpy().view(np.uint64), a)
