@@ -21,7 +21,7 @@ int witness_bounds_device(const pkg_r1cs* r1cs, const uint64_t* w, size_t padded
 int spmv_device(const uint64_t* row_ptr, const uint32_t* cols, const uint64_t* vals,
                 size_t num_rows, size_t num_cols, const uint64_t* x, uint64_t* y, uint32_t* err,
                 cudaStream_t s, size_t nnz);
-// eq(r, .) over the first num_entries points; sync: wait for the copy of r
+// eq(r, .) over the first num_entries points; sync: wait for the result
 int eq_hypercube_device(const uint64_t* r_host, size_t nr, size_t num_entries, uint64_t* out,
                         cudaStream_t s, bool sync = true);
 // Skyscraper PoW on stream s (synchronous): generic::solve's answer.

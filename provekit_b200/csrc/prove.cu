@@ -233,7 +233,6 @@ static int spartan_prove_impl(const pkg_r1cs* r1cs, const uint64_t* witness,
   uint64_t* eq = static_cast<uint64_t*>(s_eq.ptr);
   uint64_t* cov = static_cast<uint64_t*>(s_alph.ptr);
   if (whir) PK_CUDA(cudaMemsetAsync(cov, 0, 32 * nstm * n, s));
-  // out->alpha stays valid and unchanged until the evaluations' read below
   if ((rc = eq_hypercube_device(&out->alpha[0][0], m0, nc, eq, s, false))) return rc;
   // public weights: the public inputs' hash into the transcript, then x
   std::vector<uint64_t> pubw(4 * (np + 1));  // w[0 ..= np], Montgomery form

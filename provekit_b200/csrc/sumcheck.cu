@@ -59,28 +59,53 @@ __global__ void __launch_bounds__(kQuadThreads) spartan_quad_kernel(Tables4 tabs
   block_finish<3>(sums, ro);
 }
 
-// eq over a block of variables: out[x] = prod_i (bit_i(x) ? r_i : 1 - r_i)
-// with r_0 on the most significant of nr bits.
-__global__ void eq_small_kernel(const uint64_t* __restrict__ r, int nr, uint64_t* __restrict__ out) {
-  size_t n = size_t(1) << nr;
-  for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < n;
-       x += (size_t)gridDim.x * blockDim.x) {
-    Fr acc = fr_one_mont();
-    for (int i = 0; i < nr; i++) {
-      Fr ri = fr_load_ro(r, i);
-      Fr f = ((x >> (nr - 1 - i)) & 1) ? ri : fr_sub(fr_one_mont(), ri);
-      acc = fr_mul(acc, f);
-    }
-    fr_store(out, x, acc);
+// out[x] = prod_i (bit i of x, the top one first ? r_i : 1 - r_i) for x < n <= 2^nr.  A
+// CTA takes `per` runs of 256 entries: the product over the last eight variables from a
+// table of its own (itself products of two tables of 16), the one over the rest once per
+// run, and a product of the two per entry.  Bound by those chains (about 14 products at
+// 2^20 entries, eight at 2^14) and from 2^19 on by the products: 2^14 entries 27 -> 7 us,
+// 2^20 40 -> 29 (a copy of r, two table kernels and one of products before).
+constexpr int kEqMaxVars = 40;
+constexpr int kEqRunVars = 8;
+constexpr int kEqThreads = 256;
+constexpr int kEqMaxRuns = kEqThreads / 2;
+struct EqPoint {
+  uint32_t r[kEqMaxVars][8];
+};
+
+// The factors of variables first .. first + k - 1 for the k low bits of x.
+__device__ __forceinline__ Fr eq_product(const EqPoint& P, int first, int k, size_t x) {
+  Fr acc = fr_one_mont();
+#pragma unroll 1
+  for (int i = 0; i < k; i++) {
+    Fr f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) f.v[w] = P.r[first + i][w];
+    if (!((x >> (k - 1 - i)) & 1)) f = fr_sub(fr_one_mont(), f);
+    acc = i ? fr_mul(acc, f) : f;
   }
+  return acc;
 }
 
-// out[x] = hi[x >> nlo] * lo[x & (2^nlo - 1)] for x < num_entries.
-__global__ void eq_combine_kernel(const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo,
-                                  int nlo, size_t num_entries, uint64_t* __restrict__ out) {
-  for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < num_entries;
-       x += (size_t)gridDim.x * blockDim.x) {
-    fr_store(out, x, fr_mul(fr_load_ro(hi, x >> nlo), fr_load_ro(lo, x & ((size_t(1) << nlo) - 1))));
+__global__ void __launch_bounds__(kEqThreads) eq_hypercube_kernel(
+    const __grid_constant__ EqPoint P, int nr, size_t n, int per, uint64_t* __restrict__ out) {
+  __shared__ Fr high[kEqMaxRuns], part[32];
+  const int t = threadIdx.x, low = nr < kEqRunVars ? nr : kEqRunVars, kb = low / 2, ka = low - kb;
+  const size_t run0 = blockIdx.x * (size_t)per;
+  if (t < 32) {
+    const bool a = t < 16;
+    if ((t & 15) < 1 << (a ? ka : kb))
+      part[t] = eq_product(P, a ? nr - low : nr - kb, a ? ka : kb, (size_t)(t & 15));
+  } else if (t >= kEqThreads - kEqMaxRuns && t - (kEqThreads - kEqMaxRuns) < per) {
+    const int i = t - (kEqThreads - kEqMaxRuns);
+    high[i] = eq_product(P, 0, nr - low, run0 + i);
+  }
+  __syncthreads();
+  Fr mine = fr_zero();
+  if (t < 1 << low) mine = fr_mul(part[t >> kb], part[16 + (t & ((1 << kb) - 1))]);
+  for (int i = 0; i < per; i++) {
+    const size_t x = (run0 + i) * kEqThreads + t;
+    if (x < n) fr_store(out, x, fr_mul(high[i], mine));
   }
 }
 
@@ -301,29 +326,14 @@ int eq_hypercube_device(const uint64_t* r_host, size_t nr, size_t num_entries, u
   PK_REQUIRE(nr < 40 && num_entries <= (size_t(1) << nr), "num_entries %zu exceeds 2^%zu",
              num_entries, nr);
   PK_REQUIRE(out && aligned16(out), "out must be a 16-byte aligned device pointer");
-  if (nr == 0) {  // eq over no variables is the single entry 1
-    HostFr one = HostFr::one();
-    PK_CUDA(cudaMemcpyAsync(out, one.l, 32, cudaMemcpyHostToDevice, s));
-    PK_CUDA(cudaStreamSynchronize(s));
-    return PKG_OK;
-  }
-  int nhi = (int)(nr + 1) / 2, nlo = (int)nr - nhi;
-  Scratch scr;
-  size_t nh = size_t(1) << nhi, nl = size_t(1) << nlo;
-  int rc = scr.alloc(32 * (nr + nh + nl), s);
-  if (rc) return rc;
-  uint64_t* d_r = static_cast<uint64_t*>(scr.ptr);
-  uint64_t* d_hi = d_r + 4 * nr;
-  uint64_t* d_lo = d_hi + 4 * nh;
-  PK_CUDA(cudaMemcpyAsync(d_r, r_host, 32 * nr, cudaMemcpyHostToDevice, s));
-  eq_small_kernel<<<ew_grid(nh), 256, 0, s>>>(d_r, nhi, d_hi);
-  PK_CHECK_LAUNCH("eq_small_kernel");
-  eq_small_kernel<<<ew_grid(nl), 256, 0, s>>>(d_r + 4 * nhi, nlo, d_lo);
-  PK_CHECK_LAUNCH("eq_small_kernel");
-  eq_combine_kernel<<<ew_grid(num_entries), 256, 0, s>>>(d_hi, d_lo, nlo, num_entries, out);
-  PK_CHECK_LAUNCH("eq_combine_kernel");
-  // a pinned r must outlive the async copy: callers whose r stays valid
-  // until their next synchronisation pass sync = false
+  EqPoint P;
+  memset(&P, 0, sizeof P);
+  if (nr) memcpy(P.r, r_host, 32 * nr);
+  const size_t runs = (num_entries + kEqThreads - 1) / kEqThreads, ctas = 4 * (size_t)sm_count();
+  const int per = (int)std::min<size_t>(kEqMaxRuns, (runs + ctas - 1) / ctas);
+  eq_hypercube_kernel<<<(unsigned)((runs + per - 1) / per), kEqThreads, 0, s>>>(
+      P, (int)nr, num_entries, per, out);
+  PK_CHECK_LAUNCH("eq_hypercube_kernel");
   if (sync) PK_CUDA(cudaStreamSynchronize(s));
   return PKG_OK;
 }

@@ -56,3 +56,18 @@ def test_equality_tables(nv, npts):
     eq_accumulate(dw, nv, pts, cf)
     assert O.lib().pko_eq_accumulate(O.p64(w), nv, O.p64(pts), O.p64(cf), npts) == 0
     assert np.array_equal(dw.cpu().numpy().view(np.uint64), w)
+
+
+@pytest.mark.parametrize("nr,entries", [(0, 1), (3, 5), (8, 256), (9, 257), (9, 512), (14, 1 << 14),
+                                        (18, (1 << 18) - 1), (19, 1 << 19), (25, (1 << 25) - 300)])
+def test_equality_table_runs(nr, entries):
+    """Fewer variables than a run's eight, runs cut short, one and several runs a CTA, and
+    as many as a CTA takes (2^25 entries)."""
+    from provekit_b200.spartan import eq_hypercube
+    r = O.sample_fr(40 + nr, max(nr, 1))[:nr]
+    if nr:
+        r[-1] = np.array(to_limbs(P - 1), np.uint64)
+    exp = np.zeros((entries, 4), np.uint64)
+    assert O.lib().pko_eq_hypercube(O.p64(r) if nr else None, nr, entries, O.p64(exp)) == 0
+    got = eq_hypercube(r, entries).cpu().numpy().view(np.uint64)
+    assert np.array_equal(got, exp)
