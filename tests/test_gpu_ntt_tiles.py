@@ -70,3 +70,14 @@ def test_inverse_of_both_grids(log_n):
     a = values(1 << log_n, log_n, "edges")
     d = ntt_nr(dev(a), 1 << log_n, 1)
     assert np.array_equal(intt_rn(d).cpu().numpy().view(np.uint64), a)
+
+
+@pytest.mark.parametrize("log_n,columns,groups", [(8, 3, 1), (9, 7, 1), (10, 7, 2), (10, 5, 4),
+                                                  (13, 11, 1), (15, 12, 1), (17, 3, 1)])
+def test_columns_that_cut_the_last_pass(log_n, columns, groups):
+    """Odd column counts, whose last pass takes more stages than the passes before."""
+    n = 1 << log_n
+    a = values(n * columns, 5 + log_n, "edges")
+    got = ntt_nr(dev(a), n, groups).cpu().numpy().view(np.uint64)
+    assert O.ntt_nr(a, n, groups) == 0
+    assert np.array_equal(got, a)
