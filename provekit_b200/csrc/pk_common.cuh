@@ -56,9 +56,10 @@ int sm_count();
 // A launch whose CTAs may start while the stream's previous kernel still runs,
 // if that kernel says so (griddepcontrol.launch_dependents); they wait for its
 // end and its writes (griddepcontrol.wait) before they touch global memory.
-// The tiled kernels set up their shared and tensor memory meanwhile.  Such a
-// kernel reads what an earlier one may have written with plain loads only:
-// ld.global.nc is not ordered after the wait.
+// The tiled kernels set up their shared memory meanwhile, and take tensor memory
+// only after the wait (TileOf::begin in tc_reduce.cuh says why).  Such a kernel
+// reads what an earlier one may have written with plain loads only: ld.global.nc
+// is not ordered after the wait.
 //
 // Early only for grids of a few CTAs or of nearly as many as fit:
 // CTAs that start beside others gather on the SMs that have the most room, and

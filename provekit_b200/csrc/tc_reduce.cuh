@@ -234,12 +234,26 @@ struct TileOf {
   uint32_t phase;
   bool alone;      // a wait ran out: this thread reduces without the tensor cores
 
-  // Shared: image (16-byte aligned, as long as src), mbar, tmem.  The stream's
-  // next kernel may start from here on; this one continues past open() when
-  // the previous kernel's writes are there (launch_early in pk_common.cuh).
+  // Shared: image (16-byte aligned, as long as src), mbar, tmem.  open() is
+  // begin() and ready(); what touches neither tensor memory nor the other
+  // threads' data may stand between them, beside the allocation.
+  //
+  // The order of three steps keeps launch_early (pk_common.cuh) from closing a
+  // circle over tensor memory, whatever the kernels' registers allow beside
+  // each other and whoever's kernels they are:
+  //   wait for the previous kernel, then allocate: a CTA that waits for another
+  //     kernel holds no columns that this other kernel may still need;
+  //   allocate, then let the next kernel start: once its CTAs can take columns,
+  //     every CTA of this kernel has its own.
+  // A CTA that waits in the allocation therefore waits only for CTAs that hold
+  // everything they need.  Constants and barrier are set up before the wait,
+  // beside the previous kernel.  (Allocated before the wait as well, the encode of
+  // 12 x 5003 elements, whose second pass starts eight CTAs per SM at once, took
+  // 51.8 us instead of 55.0 and a small commitment 126.0 instead of 127.1; but a
+  // caller's kernel that triggers its dependents before it allocates could then
+  // wait for good.)
   template <class Shared, int kBlocks>
-  __device__ __forceinline__ void open(Shared& sh, const Image<kBlocks>& src) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  __device__ __forceinline__ void begin(Shared& sh, const Image<kBlocks>& src) {
     image = smem_addr(sh.image);
     mbar = smem_addr(&sh.mbar);
     phase = 0;
@@ -249,6 +263,8 @@ struct TileOf {
       sh.image[i] = __ldg(from + i);
     if (threadIdx.x == 0)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMA reads the constants
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x < 32) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                        smem_addr(&sh.tmem)),
@@ -256,14 +272,21 @@ struct TileOf {
                    : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMA reads the constants
+  }
+  template <class Shared>
+  __device__ __forceinline__ void ready(Shared& sh) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     tmem_after_sync();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     cols = __shfl_sync(0xffffffffu, sh.tmem, 0);
     warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     tmem = cols + (warp << 21);  // lane 32 * warp in bits 16..31
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+  template <class Shared, int kBlocks>
+  __device__ __forceinline__ void open(Shared& sh, const Image<kBlocks>& src) {
+    begin(sh, src);
+    ready(sh);
   }
 
   __device__ __forceinline__ void close() {
