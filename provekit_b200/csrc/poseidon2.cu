@@ -320,6 +320,7 @@ struct P2Tile : tc::TileOf<kP2Columns> {
       const Fr x2 = square(x);
       s[0] = product_internal(square(x2), x);
     }
+    tc::tmem_written();  // V's last writes, before they are read
 #pragma unroll
     for (int i = 1; i < 4; i++) tc::tmem_ld8(tmem + kV + 8 * (i - 1), s[i].v);
     full_rounds(s, 60);

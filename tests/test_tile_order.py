@@ -5,6 +5,8 @@ import glob
 import os
 import re
 
+import pytest
+
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "provekit_b200",
                     "csrc")
 
@@ -44,3 +46,45 @@ def test_columns_are_allocated_and_kernels_triggered_in_one_place():
     all_code = "".join(code(os.path.basename(f)) for f in glob.glob(os.path.join(CSRC, "*.cu*")))
     for step in ("tcgen05.alloc.", "griddepcontrol.launch_dependents", "griddepcontrol.wait"):
         assert all_code.count(step) == 1, step
+
+
+def calls(text):
+    """Names of the calls in text by where they end: arguments come before the call."""
+    found = []
+    for m in re.finditer(r"\b(\w+)\s*(?:<\w+>)?\s*\(", text):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[at], 0)
+            at += 1
+        found.append((at, m.group(1)))
+    return [name for _, name in sorted(found)]
+
+
+def accesses(text, function):
+    """Tensor memory's stores, waits for them and loads in the order of the source,
+    calls of the text's own functions followed."""
+    names = set(re.findall(r"\b(\w+)\s*\([^;{}()]*\)\s*(?:const\s*)?\{", text))
+    out = []
+    for name in calls(body(text, function)):
+        if name.startswith("tmem_st"):
+            out.append("store")
+        elif name == "tmem_written":
+            out.append("wait")
+        elif name.startswith("tmem_ld"):
+            out.append("load")
+        elif name in names - {"if", "for", "while", function}:
+            out += accesses(text, name)
+    return out
+
+
+@pytest.mark.parametrize("source,function", [("poseidon2.cu", "permute"),
+                                             ("sky_tc.cuh", "compress"), ("sky_tc.cuh", "permute")])
+def test_stores_are_complete_before_the_next_load(source, function):
+    """tcgen05.st is asynchronous: a tcgen05.ld after it without tcgen05.wait::st in
+    between may read what was there before."""
+    order = accesses(code(source) + code("tc_reduce.cuh"), function)
+    assert {"store", "wait", "load"} <= set(order)
+    pending = False
+    for step in order:
+        assert not (step == "load" and pending)
+        pending = step == "store" or (pending and step != "wait")
