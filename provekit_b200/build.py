@@ -28,38 +28,39 @@ def deps():
         os.path.join(ROOT, "include", "provekit_b200.h")]
 
 
-def up_to_date() -> bool:
-    if not os.path.exists(LIB):
+def up_to_date(lib: str = LIB) -> bool:
+    if not os.path.exists(lib):
         return False
-    t = os.path.getmtime(LIB)
+    t = os.path.getmtime(lib)
     return all(os.path.getmtime(d) <= t for d in deps())
 
 
-def _compile(src: str, obj: str, verbose: bool) -> None:
-    cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-c",
+def _compile(src: str, obj: str, verbose: bool, defines=()) -> None:
+    cmd = [NVCC, *ARCH, *defines, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-c",
            "-I", os.path.join(ROOT, "include"), "-o", obj, src]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
     subprocess.run(cmd, check=True)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
+def build(force: bool = False, verbose: bool = False, lib: str = LIB, defines=()) -> str:
     """Compile every translation unit to an object in parallel (each is
     self-contained: no device code crosses files), then link the shared
-    library."""
+    library.  lib, defines: another build (nvcc -D flags) in a place of its own,
+    as the tests make."""
     import concurrent.futures as cf
 
-    if not force and up_to_date():
-        return LIB
-    objdir = os.path.join(HERE, "_build")
+    if not force and up_to_date(lib):
+        return lib
+    objdir = os.path.join(HERE, "_build") if lib == LIB else lib[:-3] + "_build"
     os.makedirs(objdir, exist_ok=True)
     srcs = sources()
     objs = [os.path.join(objdir, os.path.basename(c)[:-3] + ".o") for c in srcs]
     with cf.ThreadPoolExecutor(max_workers=max(1, min(len(srcs), os.cpu_count() or 4))) as ex:
-        for f in [ex.submit(_compile, c, o, verbose) for c, o in zip(srcs, objs)]:
+        for f in [ex.submit(_compile, c, o, verbose, defines) for c, o in zip(srcs, objs)]:
             f.result()
-    subprocess.run([NVCC, *ARCH, "-shared", "-o", LIB, *objs, "-lcudart"], check=True)
-    return LIB
+    subprocess.run([NVCC, *ARCH, "-shared", "-o", lib, *objs, "-lcudart"], check=True)
+    return lib
 
 
 if __name__ == "__main__":

@@ -54,7 +54,7 @@ using P2Image = tc::Image<kP2Blocks>;
 __constant__ uint64_t kP2Rc[64][4][4];
 __device__ P2Image kP2Image;
 __constant__ uint64_t kP2DiagPlus1[3][4];  // Montgomery d1 + 1 .. d3 + 1, and ..
-__constant__ uint64_t kP2D0Plus1[4];       // .. d0 + 1, for a thread that is alone
+__constant__ uint64_t kP2D0Plus1[4];       // .. d0 + 1, for a warp that is alone
 
 static std::mutex g_p2_mu;
 static std::vector<char> g_p2_ready;
@@ -272,19 +272,17 @@ struct P2Tile : tc::TileOf<kP2Columns> {
     });
     join();
     Fr y2 = sum(0), y3 = sum(32);
-    if (__any_sync(0xffffffffu, alone)) {
+    if (alone) {
       Fr s[4];
 #pragma unroll
       for (int i = 1; i < 4; i++) tc::tmem_ld8(tmem + kV + 8 * (i - 1), s[i].v);
-      if (alone) {
-        p2_int_alone(a, b, s);
-        y0 = s[0];
-        y1 = s[1];
-        y2 = s[2];
-        y3 = s[3];
-      }
-      __syncwarp();
+      p2_int_alone(a, b, s);
+      y0 = s[0];
+      y1 = s[1];
+      y2 = s[2];
+      y3 = s[3];
     }
+    __syncwarp();
     tc::tmem_st8(tmem + kV, y1.v);
     tc::tmem_st8(tmem + kV + 8, y2.v);
     tc::tmem_st8(tmem + kV + 16, y3.v);

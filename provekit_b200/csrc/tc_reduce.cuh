@@ -222,6 +222,14 @@ __device__ __forceinline__ bool elect_lane() {
   return e != 0;
 }
 
+// Turns of a wait for an MMA (which takes well under one).
+constexpr int kWaitTries = 1 << 16;
+// Whether this thread takes a wait for one that ran out: an expression, which a
+// test's build of the library sets so that some or all warps go on alone.
+#ifndef PK_TILE_GIVES_UP
+#define PK_TILE_GIVES_UP false
+#endif
+
 // The CTA's tensor memory, constants and barrier.  All kThreads threads call
 // every member, together.
 template <uint32_t kColumns>
@@ -232,7 +240,10 @@ struct TileOf {
   uint32_t image;  // shared address of the constants
   uint32_t mbar;   // shared address of the MMA completion barrier
   uint32_t phase;
-  bool alone;      // a wait ran out: this thread reduces without the tensor cores
+  // A wait ran out: this warp reduces without the tensor cores from then on (the
+  // same in all lanes).  Warp 0, which issues the MMAs, then issues no more of
+  // them; the waits of the others run out after it, each once.
+  bool alone;
 
   // Shared: image (16-byte aligned, as long as src), mbar, tmem.  open() is
   // begin() and ready(); what touches neither tensor memory nor the other
@@ -290,7 +301,7 @@ struct TileOf {
   }
 
   __device__ __forceinline__ void close() {
-    if (alone) wait(phase ^ 1);  // the last MMA may still be running
+    if (warp == 0 && alone) wait(phase ^ 1);  // its last MMA may still be running
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     tmem_after_sync();
@@ -302,7 +313,7 @@ struct TileOf {
   // The MMA of the phase with this parity has completed; false when the wait
   // ran out.
   __device__ __forceinline__ bool wait(uint32_t parity) const {
-    for (int i = 0; i < (1 << 16); i++) {
+    for (int i = 0; i < kWaitTries; i++) {
       uint32_t done;
       asm volatile(
           "{\n\t"
@@ -323,7 +334,7 @@ struct TileOf {
   __device__ __forceinline__ void start(Issue&& issue) {
     tmem_written();
     cta_sync();
-    if (warp == 0 && elect_lane()) {
+    if (warp == 0 && !alone && elect_lane()) {
       tmem_after_sync();
       issue();
       asm volatile(
@@ -336,11 +347,14 @@ struct TileOf {
                                         bool accumulate) const {
     mma(cols + d, cols + a, image, image_block, accumulate);
   }
-  // The MMAs of start() are done, or the thread is alone from here on.
+  // The MMAs of start() are done, or the warp is alone from here on.  Warp 0
+  // starts its next MMA only after this one, so at most one is in flight and
+  // phase names it.
   __device__ __forceinline__ void join() {
-    if (!alone && !wait(phase)) alone = true;
-    phase ^= 1;
-    __syncwarp();
+    if (!alone) {
+      alone = __any_sync(0xffffffffu, !wait(phase) || PK_TILE_GIVES_UP);
+      phase ^= 1;
+    }
     tmem_after_sync();
   }
 };
@@ -351,10 +365,10 @@ struct Tile : TileOf<64> {
   __device__ __forceinline__ void block(int kblock, int image_block) const {
     TileOf<64>::block(0, 32 + 8 * kblock, image_block, kblock > 0);
   }
-  // D's columns; meaningless where the thread is alone.
+  // D's columns; meaningless where the warp is alone.
   __device__ __forceinline__ void finish(uint32_t* c) {
     join();
-    tmem_ld32(tmem, c);  // warp-wide: also where a thread is alone
+    tmem_ld32(tmem, c);
   }
 };
 
@@ -475,7 +489,7 @@ struct ProductShared {
 
 // Montgomery products through a Tile opened with kProductImage: start() after
 // the operands are known, finish() for a b 2^-256 mod p below 1.1 p
-// (meaningless where the thread is alone); any 256-bit a, b.
+// (meaningless where the warp is alone); any 256-bit a, b.
 struct ProductTile : Tile {
   __device__ __forceinline__ void start(const Fr& a, const Fr& b) {
     put_product(tmem + 32, a, b);
