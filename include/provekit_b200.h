@@ -386,13 +386,13 @@ int pkg_batch_job_info(pkg_batch *batch, size_t job, pkg_batch_job *out);
 /* NTT plan: passes of at most kmax stages (radix 2^kmax), 2^log_elems_per_cta
  * elements staged per CTA.  Re-planning drops a captured graph. */
 int pkg_batch_set_params(pkg_batch *batch, int kmax, int log_elems_per_cta);
-/* Butterflies per thread per stage, 2^log_bpt (0..2): kept in the plan and
+/* Deprecated: butterflies per thread per stage, 2^log_bpt (0..2), is kept and
  * reported, without effect on how the passes run (their CTAs have 128 threads,
- * so E staged elements take E / 256 turns a stage).  No counterpart in the
- * reference (its NTT is a CPU crate). */
+ * so E staged elements take E / 256 turns a stage); the plan and a captured
+ * graph stay.  No counterpart in the reference (its NTT is a CPU crate). */
 int pkg_batch_set_butterflies_per_thread(pkg_batch *batch, int log_bpt);
-/* The plan's current (kmax, log2 elements per CTA, log2 butterflies per
- * thread), e.g. after pkg_batch_tune.  No counterpart in the reference. */
+/* The plan's current (kmax, log2 elements per CTA), e.g. after pkg_batch_tune,
+ * and the value of pkg_batch_set_butterflies_per_thread.  No counterpart in the reference. */
 int pkg_batch_get_params(pkg_batch *batch, int *kmax, int *log_elems_per_cta,
                          int *log_butterflies_per_thread);
 /* Autotuner: times every (kmax in 4..11, elements per CTA) on this batch and

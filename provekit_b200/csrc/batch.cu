@@ -6,11 +6,10 @@
 // Every phase is ONE launch over all jobs: a small device table maps each CTA
 // (or each element) to its job, so 256 jobs cost the same number of launches
 // as one.  NTT passes take their radix (K stages) and CTA shape at run time
-// per job; the autotuner (pkg_batch_tune) sweeps the largest radix 2^4..2^11,
-// the elements per CTA and the butterflies each thread runs per stage (1, 2
-// or 4: the CTA size for a given tile).  The sumcheck's Fiat-Shamir transcript and the
-// round-polynomial bookkeeping run on the device (one thread per job), so a
-// whole batch has no host round trip and is captured once and replayed.
+// per job; the autotuner (pkg_batch_tune) sweeps the largest radix 2^4..2^11
+// and the elements per CTA.  The sumcheck's Fiat-Shamir transcript and the
+// round-polynomial bookkeeping run on the device (a warp per job, four jobs per
+// CTA), so a whole batch has no host round trip and is captured once and replayed.
 //
 // Results are bit-identical to running each job alone through pkg_ntt_nr,
 // pkg_whir_commit and pkg_spartan_sumcheck.
@@ -973,8 +972,8 @@ extern "C" int pkg_batch_set_params(pkg_batch* b, int kmax, int log_elems_per_ct
 extern "C" int pkg_batch_set_butterflies_per_thread(pkg_batch* b, int log_bpt) {
   PK_REQUIRE(b, "null batch");
   PK_REQUIRE(log_bpt >= 0 && log_bpt <= 2, "butterflies per thread 2^%d out of [1, 4]", log_bpt);
-  b->log_bpt = log_bpt;
-  return batch_replan(b);
+  b->log_bpt = log_bpt;  // the plan does not depend on it: tables and captured graph stay
+  return PKG_OK;
 }
 
 extern "C" int pkg_batch_get_params(pkg_batch* b, int* kmax, int* log_elems_per_cta,
