@@ -93,6 +93,16 @@ inline int log2_exact(size_t n) {
   return k;
 }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+// Whether the host can read p: not null, and no device memory.
+inline bool host_readable(const void* p) {
+  if (!p) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    (void)cudaGetLastError();  // no device: whatever it is, it is the host's
+    return true;
+  }
+  return at.type != cudaMemoryTypeDevice;
+}
 inline cudaStream_t as_stream(pkg_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
 

@@ -606,6 +606,7 @@ extern "C" int pkg_spartan_round(uint64_t* a, uint64_t* b, uint64_t* c, uint64_t
 
 extern "C" int pkg_eq_hypercube(const uint64_t* r, size_t nr, size_t num_entries, uint64_t* out,
                                 pkg_stream_t stream) {
+  PK_REQUIRE(num_entries == 0 || nr == 0 || host_readable(r), "r must be a host pointer");
   return eq_hypercube_device(r, nr, num_entries, out, as_stream(stream), true);
 }
 

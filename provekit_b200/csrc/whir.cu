@@ -649,5 +649,7 @@ extern "C" int pkg_eq_accumulate(uint64_t* w, size_t nv, const uint64_t* points,
   PK_REQUIRE(nv < 40, "too many variables (%zu)", nv);
   if (npts == 0) return PKG_OK;
   PK_REQUIRE(w && points && coeffs && aligned16(w), "null or unaligned pointer");
+  PK_REQUIRE((nv == 0 || host_readable(points)) && host_readable(coeffs),
+             "points and coeffs must be host pointers");
   return eq_accumulate_device(w, nv, points, coeffs, npts, as_stream(stream), true);
 }
