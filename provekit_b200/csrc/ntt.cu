@@ -141,9 +141,9 @@ int roots_reserve(size_t order, const uint64_t** out) {
 // reductions on the tensor cores (tc_reduce.cuh): 72 64-bit multiply-adds per
 // product instead of 128.  Values stay below 5 p between stages and passes.
 // Bound by the multiplier and by latency between its phases: 2^24 points take
-// 2.89 ms (the multiplier 62 % busy, DRAM 13 %) against 3.56 ms with the whole
-// product on the integer pipe; with CTAs that stay for several tiles 3.30 ms,
-// since they do not finish together.
+// 2.86 ms (the multiplier 65-69 % busy, DRAM 13-18 %), with the whole product on
+// the integer pipe 3.56 ms, with CTAs that stay for several tiles 3.30 ms, since
+// they do not finish together.
 // ---------------------------------------------------------------------------
 // Where a transform's first pass reads its input.
 enum : int { kFromData = 0, kFromEncode = 1, kFromReversed = 2 };
@@ -164,8 +164,8 @@ __device__ __forceinline__ Fr encode_load(const NttSource& s, uint64_t g) {
 // (40.5 against 43.2 us) but cost 5 % at 18 stages over 16 columns of 2^20.
 constexpr int kPassStages = 8;
 // Elements per CTA, log2: two batches of 128 butterflies a stage, or one below
-// 2^21 elements, where the batch's latency counts: 2^19 points 103 us with one
-// and 114 with two, 2^20 185 and 190, 2^22 744 and 699.  Four: 763.
+// 2^21 elements, where the batch's latency counts: 2^19 points 94 us with one
+// and 105 with two, 2^20 179 and 183, 2^21 352 and 341, 2^22 737 and 692.  Four: 757.
 constexpr int kTileElems = 9, kSmallTileElems = 8;
 constexpr uint64_t kSmallBelow = uint64_t(1) << 21;
 
@@ -208,7 +208,7 @@ struct PassShape {
 //
 // kAhead, for grids that leave two CTAs per SM or fewer: a stage's twiddle is loaded
 // during the stage before, with the registers that the missing CTAs leave (2^10 points
-// 12.9 -> 11.9 us, 2^16 26.5 -> 25.0); larger grids hide the load behind other CTAs, and eight
+// 12.3 -> 11.1 us, 2^16 26.7 -> 24.7); larger grids hide the load behind other CTAs, and eight
 // of them have no registers for it (2^24 2.85 -> 2.92 ms).
 constexpr int kAheadCtas = 2;
 template <int kSrc, bool kModeB, bool kAhead>
@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(tc::kThreads, kAhead ? kAheadCtas : tc::kMaxCt
   const int E = T << K;
   const uint64_t U = shape.U;
   tc::ProductTile tile;
-  // kAhead: the loads run beside the allocation (2^16 points 26.5 -> 24.6 us); with
-  // 64 registers that makes the stages slower (2^24 2.86 -> 2.92 ms)
+  // kAhead: the loads run beside the allocation (inverse of 2^16 points 26.5 -> 24.6 us);
+  // with 64 registers that makes the stages slower (2^24 2.86 -> 2.92 ms)
   if (kAhead)
     tile.begin(sh, tc::kProductImage);
   else

@@ -61,13 +61,14 @@ int sm_count();
 // reads what an earlier one may have written with plain loads only: ld.global.nc
 // is not ordered after the wait.
 //
-// Early only for grids of a few CTAs or of nearly as many as fit:
-// CTAs that start beside others gather on the SMs that have the most room, and
-// between those sizes that leaves the kernel unevenly spread, already with 64
-// CTAs on the 20 SMs that 128 leave free.  2^10 points (2 x
-// 8 CTAs) 18.5 -> 12.7 us, 2^18 (3 x 1024) 61.7 -> 53.0, a commitment's small
-// tree 129 -> 118; but 2^16 points (2 x 256) 26.7 -> 43.4 and 2^16 leaves of 8
-// (512) 101 -> 132, and a tree over 2^14 leaves (128, 64, 1) 149 -> 172.
+// Early for grids of a few CTAs or of nearly as many as fit (six of the eight per
+// SM that the large tiled kernels have; the others' grids stay below that): 2^10
+// points (2 x 4 CTAs) 16.5 -> 11.4 us, 2^18 (3 x 1024) 63.0 -> 54.3, a tree over
+// 2^12 leaves of 8 129 -> 118.  Between those sizes one stream would gain too
+// (an inverse of 2^16 points, 2 x 256 CTAs, 24.6 -> 19.7), but CTAs that wait
+// take room from the kernels of other streams: four threads proving 2^17
+// constraints make 727 proofs/s so and 672 with every launch early, eight
+// proving 2^14 2680 and 2500.
 template <class... Params, class... Args>
 cudaError_t launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
                          cudaStream_t stream, Args&&... args) {

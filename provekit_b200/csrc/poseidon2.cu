@@ -30,7 +30,7 @@ namespace pk {
 //     64..95          a square's or product's words, or four elements
 //     96..119         s[1], s[2], s[3]
 // Per partial round 184 64-bit multiply-adds instead of 840: 200003 hashes of 3
-// elements take 0.69 ms against 1.64 ms with one thread's products on the
+// elements take 0.68 ms against 1.64 ms with one thread's products on the
 // integer pipe.  Bound by the multiplier and by latency between the phases.
 constexpr uint32_t kA = 64, kV = 96, kP2Columns = 128;
 constexpr int kP2Ctas = 4;

@@ -4,9 +4,9 @@
 // interleaved_encode = (1) transpose the messages into the interleaved
 // [row][message] layout, (2) append the masks, (3) pick the coset size, (4)
 // replicate the first coset num_cosets times, (5) ntt_nr with the first
-// log2(num_cosets) stages skipped.  Steps 1, 2 and 4 are one gather kernel
-// that writes every codeword slot exactly once; step 5 is the NTT pass
-// pipeline of ntt.cu.
+// log2(num_cosets) stages skipped.  Steps 1, 2 and 4 are the loads of the
+// transform's first pass (encode_load in ntt.cu); one gather kernel that writes
+// every codeword slot once does them where no stage is left.
 #include <algorithm>
 #include <cstring>
 #include <mutex>

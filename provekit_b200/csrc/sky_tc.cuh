@@ -7,9 +7,9 @@
 // whose A byte (tensor memory column 62) is 1.
 //
 // Bound by the multiplier: 44 64-bit multiply-adds of four issue cycles per
-// square round against 100.  Measured on B200: 2^20 leaves of 16 Fr in 2.21 ms
-// (7.1 G compressions/s) against 4.10 ms with sky_compress.  A lone CTA takes
-// 6.2 us per compression against 8.0.  Merging E and O first and adding T's
+// square round against 100.  Measured on B200: 2^20 leaves of 16 Fr in 2.17 ms
+// (7.2 G compressions/s) against 4.10 ms with sky_compress.  A lone CTA takes
+// 6.1 us per compression against 8.0.  Merging E and O first and adding T's
 // high half on the ALU (one K block) was 10 % slower; two K blocks more for T's
 // high half and r instead of additions changed nothing.
 #pragma once

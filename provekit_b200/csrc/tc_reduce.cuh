@@ -8,8 +8,8 @@
 // constants (N = 32).  tcgen05.mma kind::i8 (u8 x u8 -> s32) does it exactly:
 // a column of 64 bytes with full residues is below 2^22, the other bytes add
 // theirs as they are.  What is left on the integer pipe is the product itself,
-// assembling 32 columns into 9 words (34 ALU operations), and one quotient
-// step back to 8 words (8 of the reduction's 64 64-bit multiply-adds).
+// adding the 32 columns up to two 8-word numbers and a top word (assemble), and
+// one quotient step over these (8 of the reduction's 64 64-bit multiply-adds).
 //
 // The sum is linear, so the product's two accumulators (even and odd word
 // offsets, see fr.cuh) are never added: both go in as they are, the odd one

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) eq_tables_kernel(const uint64_t* __restri
 
 // w[b] += sum_j hi_j[b >> nlo] lo_j[b & (2^nlo - 1)], the products of an entry
 // summed unreduced (fr_lazy.cuh).  2^split threads share an entry's points, so that
-// a short table still fills the chip; those of one entry lie 256 / 2^split apart,
+// a short table still fills the chip; those of one entry lie 128 / 2^split apart,
 // and a warp's loads stay in line.  Bound by the multiplier (256 cycles per warp
 // and point): 2^18 entries of 118 points 446 us with binary64 sums, 283 now; 2^14 of
 // 40 32 -> 12, 2^21 of two (a product each before) 115 -> 82.
