@@ -96,11 +96,11 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
   const PassDesc& d = descs[find_desc(begins, ndesc, blockIdx.x)];
   const int K = (int)d.K, T = (int)d.T, log_t = (int)d.log_t, log_u = (int)d.log_u;
   const int E = T << K;
-  const bool mode_b = d.mode_b != 0;
+  const int mode = d.mode_b ? kModeB : kModeA;
   const uint64_t U = d.U;
   const uint64_t l0 = (uint64_t)(blockIdx.x - d.cta_begin) * T;
   uint64_t high_a = 0, u0 = 0;
-  if (!mode_b) {
+  if (mode == kModeA) {
     high_a = l0 / U;
     u0 = l0 - high_a * U;
   }
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    pass_index(mode_b, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    pass_index(mode, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     const uint4* in;
     if (d.src_kind == 0) {
       in = reinterpret_cast<const uint4*>(data + 4 * g);
@@ -122,12 +122,12 @@ __global__ void __launch_bounds__(tc::kThreads, tc::kMaxCtas)
     sm[E + sidx] = in[1];  // high 16 bytes: plane 1
   }
   __syncthreads();
-  tile_stages<false>(tile, sm, mode_b, K, T, log_t, log_u, l0, high_a, d.first != 0, roots);
+  tile_stages<false>(tile, sm, mode, K, T, log_t, log_u, U, l0, high_a, d.first != 0, roots);
   const bool last = d.last != 0;
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    pass_index(mode_b, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    pass_index(mode, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     Fr v = tile_load(sm, E, sidx);
     if (last) v = fr_reduce_once(tc::reduce_any(v));
     fr_store(data, g, v);

@@ -133,7 +133,9 @@ int roots_reserve(size_t order, const uint64_t** out) {
 // [0, U), U = 2^B * M, and line element j is at (high*2^K + j)*U + u.
 // A CTA owns T consecutive lines.  Mode A (T divides U): the lines share
 // `high` and are contiguous per j.  Mode B (U divides T, U a power of two):
-// the CTA's lines cover a contiguous memory range.
+// the CTA's lines cover a contiguous memory range.  Mode C (U no power of two):
+// each line finds its own `high`, for passes in which mode A's T, at most the
+// power-of-two part of U, would leave a tile fewer butterflies than threads.
 // Stage s of the pass (global stage t+s) pairs j0 = grp*2h + pos with
 // j0 + h (h = 2^(K-1-s)) and uses twiddle roots[(high << s) | grp].
 //
@@ -202,7 +204,7 @@ struct PassShape {
   int inverse;     // last pass of an inverse over 2^inverse points, or 0
 };
 
-// kModeB selects mode B at compile time.  In mode A every line of the CTA
+// kMode selects the mode at compile time.  In mode A every line of the CTA
 // shares `high`, so stage s reads only the 2^s twiddles roots[(high << s) |
 // grp], which stay in L1.
 //
@@ -211,7 +213,7 @@ struct PassShape {
 // 12.3 -> 11.1 us, 2^16 26.7 -> 24.7); larger grids hide the load behind other CTAs, and eight
 // of them have no registers for it (2^24 2.85 -> 2.92 ms).
 constexpr int kAheadCtas = 2;
-template <int kSrc, bool kModeB, bool kAhead>
+template <int kSrc, int kMode, bool kAhead>
 __global__ void __launch_bounds__(tc::kThreads, kAhead ? kAheadCtas : tc::kMaxCtas)
     ntt_pass_kernel(uint64_t* data, uint64_t* out, const uint64_t* __restrict__ roots,
                     const PassShape shape, const NttSource src) {
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(tc::kThreads, kAhead ? kAheadCtas : tc::kMaxCt
     tile.open(sh, tc::kProductImage);
   const uint64_t l0 = (uint64_t)blockIdx.x * T;
   uint64_t high_a = 0, u0 = 0;
-  if (!kModeB) {
+  if (kMode == kModeA) {
     high_a = l0 / U;
     u0 = l0 - high_a * U;
   }
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__(tc::kThreads, kAhead ? kAheadCtas : tc::kMaxCt
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    pass_index(kModeB, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    pass_index(kMode, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     if (kSrc != kFromData) {
       // reversed: the inverse's first permutation, v[bitrev((n - g) mod n)]
       const Fr v = kSrc == kFromEncode
@@ -255,12 +257,12 @@ __global__ void __launch_bounds__(tc::kThreads, kAhead ? kAheadCtas : tc::kMaxCt
     tile.ready(sh);  // a barrier for the loads too
   else
     __syncthreads();
-  tile_stages<kAhead>(tile, sm, kModeB, K, T, log_t, log_u, l0, high_a, shape.first, roots);
+  tile_stages<kAhead>(tile, sm, kMode, K, T, log_t, log_u, U, l0, high_a, shape.first, roots);
   // ---- store ----
   for (int e = threadIdx.x; e < E; e += tc::kThreads) {
     uint64_t g;
     int sidx;
-    pass_index(kModeB, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
+    pass_index(kMode, e, K, T, log_t, log_u, U, l0, high_a, u0, &g, &sidx);
     Fr v = tile_load(sm, E, sidx);
     if (shape.inverse) v = halve(v, shape.inverse);
     if (shape.last) v = fr_reduce_once(tc::reduce_any(v));
@@ -270,10 +272,15 @@ __global__ void __launch_bounds__(tc::kThreads, kAhead ? kAheadCtas : tc::kMaxCt
 }
 
 using PassKernel = void (*)(uint64_t*, uint64_t*, const uint64_t*, PassShape, NttSource);
+template <int kSrc, int kMode>
+static PassKernel pass_kernel(bool ahead) {
+  return ahead ? ntt_pass_kernel<kSrc, kMode, true> : ntt_pass_kernel<kSrc, kMode, false>;
+}
 template <int kSrc>
-static PassKernel pass_kernel(bool mode_b, bool ahead) {
-  if (ahead) return mode_b ? ntt_pass_kernel<kSrc, true, true> : ntt_pass_kernel<kSrc, false, true>;
-  return mode_b ? ntt_pass_kernel<kSrc, true, false> : ntt_pass_kernel<kSrc, false, false>;
+static PassKernel pass_kernel(int mode, bool ahead) {
+  if (mode == kModeA) return pass_kernel<kSrc, kModeA>(ahead);
+  if (kSrc == kFromReversed || mode == kModeB) return pass_kernel<kSrc, kModeB>(ahead);
+  return pass_kernel<kSrc == kFromReversed ? kFromData : kSrc, kModeC>(ahead);  // one column: no mode C
 }
 
 static inline uint64_t pow2_part(uint64_t x) { return x & (~x + 1); }
@@ -305,11 +312,18 @@ static int run_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end
     const uint64_t num_lines = (uint64_t(1) << t) * U;
     uint64_t T = uint64_t(1) << (K >= log_elems ? 0 : log_elems - K);
     if (T > num_lines) T = pow2_part(num_lines);
-    const bool mode_b = is_pow2(U) && U < T;
-    if (!mode_b) T = std::min(T, pow2_part(U));
+    int mode = is_pow2(U) && U < T ? kModeB : kModeA;
+    if (mode == kModeA && pow2_part(U) < T) {
+      // the last stages of 33 columns of 2^12 points, one and two of them: 360 and 210 us
+      // in mode A (2 and 4 elements a CTA), 8.7 and 10.4 in mode C; seven: 22.1 and 18.6
+      if (t > 0 && (pow2_part(U) << K) < 2 * tc::kThreads && num_lines >> 32 == 0)
+        mode = kModeC, T = std::min(T, pow2_part(num_lines));
+      else
+        T = pow2_part(U);
+    }
     PassShape shape;
     shape.U = U;
-    shape.log_u = mode_b ? log2_exact(U) : 0;
+    shape.log_u = mode == kModeB ? log2_exact(U) : 0;
     shape.T = (int)T;
     shape.log_t = log2_exact(T);
     shape.K = K;
@@ -327,9 +341,9 @@ static int run_stages(uint64_t* data, size_t N, size_t M, int t_begin, int t_end
     }
     uint64_t* const out = inverse && shape.last ? inverse : data;
     const bool ahead = grid <= kAheadCtas * (unsigned)sm_count();
-    const PassKernel fn = kind == kFromData     ? pass_kernel<kFromData>(mode_b, ahead)
-                          : kind == kFromEncode ? pass_kernel<kFromEncode>(mode_b, ahead)
-                                                : pass_kernel<kFromReversed>(mode_b, ahead);
+    const PassKernel fn = kind == kFromData     ? pass_kernel<kFromData>(mode, ahead)
+                          : kind == kFromEncode ? pass_kernel<kFromEncode>(mode, ahead)
+                                                : pass_kernel<kFromReversed>(mode, ahead);
     PK_CUDA(launch_early(fn, grid, tc::kThreads, smem, stream, data, out, roots, shape, s));
     PK_CHECK_LAUNCH("ntt_pass_kernel");
     t += K;

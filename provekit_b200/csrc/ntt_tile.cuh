@@ -21,13 +21,26 @@ __device__ __forceinline__ void tile_store(uint4* sm, int E, int i, const Fr& x)
 // The product where the tensor cores' wait ran out (w < p, x < 5 p).
 static __device__ __noinline__ Fr product_alone(const Fr w, const Fr x) { return fr_mul(w, x); }
 
+// How the T lines of a tile lie (see ntt.cu).
+enum : int { kModeA = 0, kModeB = 1, kModeC = 2 };
+
+// `high` of line l in mode C (fewer than 2^32 lines).
+__device__ __forceinline__ uint64_t line_high(uint64_t l, uint64_t U) {
+  return (uint32_t)l / (uint32_t)U;
+}
+
 // Index of tile element e in the data and in shared memory.
-__device__ __forceinline__ void pass_index(bool mode_b, int e, int K, int T, int log_t, int log_u, uint64_t U,
-                                           uint64_t l0, uint64_t high, uint64_t u0, uint64_t* g,
-                                           int* sidx) {
-  if (!mode_b) {
+__device__ __forceinline__ void pass_index(int mode, int e, int K, int T, int log_t, int log_u,
+                                           uint64_t U, uint64_t l0, uint64_t high, uint64_t u0,
+                                           uint64_t* g, int* sidx) {
+  if (mode == kModeA) {
     const int j = e >> log_t, ll = e & (T - 1);
     *g = ((high << K) + j) * U + u0 + ll;
+    *sidx = e;
+  } else if (mode == kModeC) {
+    const int j = e >> log_t;
+    const uint64_t l = l0 + (e & (T - 1)), h = line_high(l, U);
+    *g = ((h << K) + j) * U + (l - h * U);
     *sidx = e;
   } else {
     const int j = (e >> log_u) & ((1 << K) - 1);
@@ -93,8 +106,8 @@ __device__ __forceinline__ void loose_butterfly(const Fr& x0, const Fr& m, Fr& y
 // is stage 0 of the transform, whose twiddles are all 1.  kAhead: the next twiddle is
 // loaded beside the matrix product (ntt.cu says where).
 template <bool kAhead>
-__device__ __forceinline__ void tile_stages(tc::ProductTile& tile, uint4* sm, bool mode_b, int K,
-                                            int T, int log_t, int log_u, uint64_t l0,
+__device__ __forceinline__ void tile_stages(tc::ProductTile& tile, uint4* sm, int mode, int K,
+                                            int T, int log_t, int log_u, uint64_t U, uint64_t l0,
                                             uint64_t high_a, bool first,
                                             const uint64_t* __restrict__ roots) {
   const int E = T << K, half = E >> 1;
@@ -103,7 +116,9 @@ __device__ __forceinline__ void tile_stages(tc::ProductTile& tile, uint4* sm, bo
   const auto twiddle = [&](int s, int b0) {
     const int b = b0 + (int)threadIdx.x;
     const int bb = b < half ? b : 0;
-    const uint64_t high = mode_b ? (l0 + (bb & (T - 1))) >> log_u : high_a;
+    const uint64_t l = l0 + (bb & (T - 1));
+    const uint64_t high =
+        mode == kModeB ? l >> log_u : (mode == kModeC ? line_high(l, U) : high_a);
     return fr_load_ro(roots, (high << s) | (uint64_t)((bb >> log_t) >> (K - 1 - s)));
   };
   if (kAhead && !first) ahead = twiddle(0, 0);
@@ -132,7 +147,9 @@ __device__ __forceinline__ void tile_stages(tc::ProductTile& tile, uint4* sm, bo
         if (kAhead) {
           w = ahead;
         } else {
-          const uint64_t high = mode_b ? (l0 + ll) >> log_u : high_a;
+          const uint64_t l = l0 + ll;
+          const uint64_t high =
+              mode == kModeB ? l >> log_u : (mode == kModeC ? line_high(l, U) : high_a);
           w = fr_load_ro(roots, (high << s) | (uint64_t)grp);
         }
         tile.start(w, x1);
