@@ -62,16 +62,25 @@ static void fold_weights(const uint64_t* alpha, unsigned k, FrParams<1 << kMaxFo
   for (size_t j = 0; j < w.size(); j++) put_param(W, (int)j, w[j]);
 }
 
-// out[i] = sum_j w_j c[j L + i]  (w_0 = 1)
+// out[i] = sum_j w_j c[j L + i]  (w_0 = 1).  A product alone (m = 2) is reduced at
+// once: 2^21 coefficients 30.8 us, with the unreduced sum 35.5 (rows are the same
+// either way, and their larger folds lose registers by it).
 __global__ void whir_fold_coeffs_kernel(const uint64_t* __restrict__ c, size_t L, int m,
                                         const __grid_constant__ FrParams<1 << kMaxFoldK> W,
                                         uint64_t* __restrict__ out) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < L;
        i += (size_t)gridDim.x * blockDim.x) {
-    lazy::Acc acc;
-    acc.zero();
-    for (int j = 1; j < m; j++) acc.mac(param_fr(W, j), fr_load_ro(c, j * L + i));
-    fr_store(out, i, fr_add(fr_load_ro(c, i), acc.finish()));
+    const Fr head = fr_load_ro(c, i);
+    Fr tail;
+    if (m == 2) {
+      tail = fr_mul(param_fr(W, 1), fr_load_ro(c, L + i));
+    } else {
+      lazy::Acc acc;
+      acc.zero();
+      for (int j = 1; j < m; j++) acc.mac(param_fr(W, j), fr_load_ro(c, j * L + i));
+      tail = acc.finish();
+    }
+    fr_store(out, i, fr_add(head, tail));
   }
 }
 
