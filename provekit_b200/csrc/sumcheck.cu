@@ -326,9 +326,15 @@ int eq_hypercube_device(const uint64_t* r_host, size_t nr, size_t num_entries, u
   PK_REQUIRE(nr < 40 && num_entries <= (size_t(1) << nr), "num_entries %zu exceeds 2^%zu",
              num_entries, nr);
   PK_REQUIRE(out && aligned16(out), "out must be a 16-byte aligned device pointer");
+  if (nr == 0) {  // the single entry 1: a copy takes 15 us with its wait, a launch 18
+    const HostFr one = HostFr::one();
+    PK_CUDA(cudaMemcpyAsync(out, one.l, 32, cudaMemcpyHostToDevice, s));
+    if (sync) PK_CUDA(cudaStreamSynchronize(s));
+    return PKG_OK;
+  }
   EqPoint P;
   memset(&P, 0, sizeof P);
-  if (nr) memcpy(P.r, r_host, 32 * nr);
+  memcpy(P.r, r_host, 32 * nr);
   const size_t runs = (num_entries + kEqThreads - 1) / kEqThreads, ctas = 4 * (size_t)sm_count();
   const int per = (int)std::min<size_t>(kEqMaxRuns, (runs + ctas - 1) / ctas);
   eq_hypercube_kernel<<<(unsigned)((runs + per - 1) / per), kEqThreads, 0, s>>>(
