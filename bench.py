@@ -51,10 +51,10 @@ WIDE_PER_POSEIDON2 = (8 * 4 + 56) * (2 * WIDE_PER_SQR + WIDE_PER_MUL) + 56 * 3 *
 # dram__bytes_read.sum + dram__bytes_write.sum of one fold_tc_kernel launch from an ncu
 # capture of this shape (the fold kernel's profile summary under profiles/), keyed by
 # (log2 coeffs, folding factor, log inv rate).
-LEAF_TRAFFIC_BYTES = {(20, 4, 2): 134.298e6 + 6.458e6}
+LEAF_TRAFFIC_BYTES = {(20, 4, 2): 135.039e6 + 5.989e6}
 # the same for the whole proof's witness commitment (whir-ZK: 2^20 leaves of 16 Fr, the
 # witness and blinding polynomials of m = 21 at rate 1/4).
-LEAF_TRAFFIC_PROVE_BYTES = 536.947e6 + 31.544e6
+LEAF_TRAFFIC_PROVE_BYTES = 540.728e6 + 36.093e6
 
 
 def wide_rate(L):

@@ -118,6 +118,8 @@ extern "C" int pkg_intt_rn_noalloc(uint64_t* values, size_t len, pkg_stream_t st
   PK_CHECK_LAUNCH("noalloc_roots_kernel");
   noalloc_gather_in<<<blocks, 256, 0, s>>>(values, tmp, len, log_n);
   PK_CHECK_LAUNCH("noalloc_gather_in");
+  // The passes may start early and read the table with ld.global.nc; noalloc_gather_in,
+  // which lets nothing start before its end, stands between them and the table's kernel.
   rc = ntt_stages(tmp, len, 1, 0, log_n, roots, s);
   if (rc) return rc;
   HostFr ninv = HostFr::inv(HostFr::from_u64(len));

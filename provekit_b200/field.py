@@ -15,7 +15,7 @@ OPS = {("mul", "fp64"): 0, ("sqr", "fp64"): 1, ("from_mont", "fp64"): 2,
 def fr_op(op: str, a: torch.Tensor, b: torch.Tensor = None, pipe: str = "fp64", out=None,
           stream=None) -> torch.Tensor:
     """out[i] = op(a[i], b[i]); op in {"mul", "sqr", "from_mont"}, pipe in
-    {"fp64", "int"}.  Inputs are (n, 4) int64 device tensors of Fr limbs."""
+    {"fp64", "int"} (the integer one is the faster and the kernels' own).  Inputs are (n, 4) int64 device tensors of Fr limbs."""
     code = OPS[(op, pipe)]
     fr_tensor(a, "a")
     if op == "mul":
