@@ -84,7 +84,9 @@ cudaError_t launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_
   config.stream = stream;
   config.attrs = &attr;
   config.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, Params(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();  // the next launch's check is not to see it
+  return e;
 }
 
 inline bool is_pow2(size_t n) { return n && !(n & (n - 1)); }
